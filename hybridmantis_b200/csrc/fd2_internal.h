@@ -40,6 +40,7 @@ struct TransportArgs {
     int64_t event_base;          // global index of event 0 (RNG counters)
     uint32_t round_keys[20];     // Philox key schedule of the seed
     const uint32_t *run_tag;     // device counter: runs since submission
+    int pull_shift;              // a warp's refill takes (chunks left) >> pull_shift, 1 to 32 (set by launch_transport)
     int chunk;
     int refill;
     int fresnel_batch;           // parked lanes before the Fresnel pass runs

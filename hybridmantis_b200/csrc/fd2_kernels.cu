@@ -372,7 +372,6 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
     unsigned int *s_cnt = reinterpret_cast<unsigned int *>(smem + L.cnt);
     float *s_dist = reinterpret_cast<float *>(smem + L.dist);
     unsigned int *s_win = reinterpret_cast<unsigned int *>(smem + L.win);
-    (void)nwarps;
 
     if (kMulti)
         for (int i = threadIdx.x; i < a.n_geom; i += blockDim.x) s_geom[i] = a.geoms[i];
@@ -384,7 +383,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
     Slot *ring = s_ring + wid * kRing;
     // never read past the chunk buffer, whatever the scan produced
     const unsigned long long total_chunks = min(*a.n_chunks, (unsigned long long)a.chunk_capacity);
-    int ring_len = 0, slot = 0, refills = 0;
+    int ring_len = 0, slot = 0;
     uint32_t used = 0;
     bool exhausted = false, alive = false, parked = false;
     bool xretry = false;  // the lane's crosstalk normal is retried this round
@@ -414,22 +413,35 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
         if (needy && !exhausted && ((unsigned)__popc(needy) >= refill_min || needy == kFull)) {
             while (needy) {
                 if (slot >= ring_len) {
+                    // A refill takes a share of what is left: 32 chunks while
+                    // every warp can still take that many twice, then fewer,
+                    // down to one, so that a small run spreads over the warps
+                    // (always taking 32 chunks gave a 25-x-ray run to 66 of
+                    // 4,736 warps) and a large one ends evenly.
+                    // The abort flag lies in host memory: one warp of the
+                    // grid polls it and the others see the device's status
+                    // word.  Every warp reading it at its first refill queued
+                    // 4,736 reads on PCIe, 4.2 ms of every launch.
                     unsigned long long base = 0;
-                    int stop = 0;
+                    int take = 0;
                     if (lane == 0) {
-                        stop = (a.abort_flag && (refills & 15) == 0 && *a.abort_flag) ? 1 : 0;
-                        if (!stop) base = atomicAdd(a.queue_head, (unsigned long long)kRing);
+                        if (a.abort_flag && blockIdx.x == 0 && wid == 0 && *a.abort_flag)
+                            atomicOr(a.status, kStatusAborted);
+                        const unsigned long long head = *(const volatile unsigned long long *)a.queue_head;
+                        if (!(*(const volatile int *)a.status & kStatusAborted)) {
+                            const unsigned long long left = total_chunks > head ? total_chunks - head : 0ull;
+                            take = (int)min(max(left >> a.pull_shift, 1ull), (unsigned long long)kRing);
+                            base = atomicAdd(a.queue_head, (unsigned long long)take);
+                        }
                     }
-                    ++refills;
-                    stop = __shfl_sync(kFull, stop, 0);
+                    take = __shfl_sync(kFull, take, 0);
                     base = __shfl_sync(kFull, base, 0);
-                    if (stop) {
-                        if (lane == 0) atomicOr(a.status, kStatusAborted);
+                    if (take == 0) {
                         exhausted = true;
                         break;
                     }
                     const unsigned long long idx = base + lane;
-                    const bool ok = idx < total_chunks;
+                    const bool ok = lane < take && idx < total_chunks;
                     __syncwarp();  // every lane is done reading the old ring
                     if (ok) {
                         const uint2 c = a.chunks[idx];
@@ -777,10 +789,15 @@ size_t transport_smem_bytes(const TransportConfig &cfg, int n_geom)
     return SmemLayout(cfg.block, n_geom, cfg.window).total;
 }
 
-cudaError_t launch_transport(cudaStream_t s, const TransportConfig &cfg, int sm_count, const TransportArgs &a)
+cudaError_t launch_transport(cudaStream_t s, const TransportConfig &cfg, int sm_count, const TransportArgs &args)
 {
+    TransportArgs a = args;
     const size_t smem = transport_smem_bytes(cfg, a.n_geom);
     const unsigned grid = (unsigned)(sm_count * cfg.ctas_per_sm);
+    // a refill takes 1 / 2^pull_shift of the chunks left: at most half of a
+    // warp's even share
+    for (a.pull_shift = 1; (1ll << a.pull_shift) < 2ll * grid * (cfg.block / 32); ++a.pull_shift) {
+    }
     const bool multi = a.n_geom > 1;
     const int per_sm = cfg.block > 256 ? 1 : std::min(std::max(cfg.ctas_per_sm, 2), 4);
     if (a.g0.grid) {
