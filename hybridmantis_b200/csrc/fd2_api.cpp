@@ -371,28 +371,17 @@ void fit_window(fd2_ctx *c)
     }
 }
 
-// Launch shape unless the options give one, measured on a B200 (config-1
-// events, 20,000 x-rays): one geometry 256 threads x 4 CTAs per SM (32 warps
-// at 64 registers; 6.7e8 photons/s against 5.8e8 for 320 x 2), chunks of 16
-// photons; several geometries 256 x 3 (8.5e8 against 7.9e8 for 256 x 4,
-// whose variant spills); the column lattice 320 x 2 (2.2e8 against 2.0e8 for
-// 256 x 2 or x 3); label mode with one geometry (the surrogate's audit) as
-// one geometry, with several 256 x 2.
+// Launch shape unless the options give one, measured on a B200: one geometry
+// 256 threads x 4 CTAs per SM (32 warps at 64 registers; 20,000 config-1
+// x-rays 51.6 ms against 55.6 for 256 x 3), chunks of 16 photons; several
+// geometries 256 x 3 (configuration 2, 500 x-rays: 73.0 ms against 90.6 for
+// 256 x 2; 256 x 4 the same); the column lattice 256 x 3 (10,001 config-1
+// x-rays 77.2 ms against 82.5 for 320 x 2); label mode with one geometry
+// (the surrogate's audit) as one geometry, with several 256 x 3.
 static void default_launch(const fd2_ctx *c, int n_geom, fd2::TransportConfig *cfg)
 {
     int block = 256, ctas = 4, chunk = 16;
-    if (c->opt.radial_bins > 0) {
-        // label mode: one geometry (the surrogate's audit) as a production
-        // run; several (training labels) 256 x 2
-        if (n_geom > 1) {
-            ctas = 2;
-            chunk = 32;
-        }
-    } else if (c->opt.column_grid) {
-        block = 320;
-        ctas = 2;
-        chunk = 32;
-    } else if (n_geom > 1) {
+    if (c->opt.column_grid || n_geom > 1) {
         ctas = 3;
         chunk = 32;
     }
@@ -454,7 +443,9 @@ std::string tune_key(const fd2_ctx *c)
 {
     double mean = c->n_events ? c->mu_total / (double)c->n_events : 0.0;
     char b[256];
-    std::snprintf(b, sizeof b, "%s|ev%d|ph%d|g%d|m%d", c->device_name.c_str(), (int)std::log2((double)c->n_events + 1),
+    // "q": tuned with the warps' queue of waiting photons; an entry of the
+    // kernel before it holds a Fresnel batch that is slow with this one
+    std::snprintf(b, sizeof b, "%s|q|ev%d|ph%d|g%d|m%d", c->device_name.c_str(), (int)std::log2((double)c->n_events + 1),
                   (int)std::log2(mean + 1), (int)c->geoms.size(), c->opt.count_mode);
     return b;
 }
@@ -643,11 +634,13 @@ fd2_status fd2_create(const fd2_params *p, const fd2_options *opt, fd2_ctx **out
     if ((st = alloc_tallies(c)) != FD2_OK) return bail(st);
     fd2::TransportConfig cfg;
     default_launch(c, 1, &cfg);
-    cfg.refill = c->opt.refill > 0 ? c->opt.refill : 4;
-    // parked lanes before the warp's Fresnel pass (8), or with a column lattice
-    // gap lanes before the warp's gap segments (12: square 1.755 / hexagonal
-    // 1.333e8 photons/s on config 1, against 1.743 / 1.297 at 8)
-    cfg.fresnel = c->opt.fresnel_batch > 0 ? c->opt.fresnel_batch : (c->opt.column_grid ? 12 : 8);
+    // idle lanes that trigger a refill (20,000 config-1 x-rays: 2 / 4 / 6 / 8
+    // lanes 53.4 / 51.9 / 51.7 / 52.1 ms; the lattice 78.3 / 77.3 / 77.2 / 77.9)
+    cfg.refill = c->opt.refill > 0 ? c->opt.refill : 6;
+    // photons waiting for the Fresnel part (with a lattice: in the gap) before
+    // the warp runs it for them: a full warp's (16 / 24 / 32 photons: 56.7 /
+    // 53.3 / 51.9 ms, hexagonal lattice 114 ms at 24, 104 at 32)
+    cfg.fresnel = c->opt.fresnel_batch > 0 ? c->opt.fresnel_batch : 32;
     if ((st = set_config(c, cfg)) != FD2_OK) return bail(st);
     *out = c;
     return FD2_OK;
@@ -1246,8 +1239,8 @@ fd2_status fd2_autotune(fd2_ctx *c, int32_t budget_runs)
     // refill and Fresnel batch one knob at a time, twice over
     const std::vector<std::pair<int, int>> shapes = {{256, 4}, {128, 8}, {256, 3}, {320, 2}, {256, 2}, {512, 1}};
     const std::vector<int> chunks = {8, 16, 32, 64, 128};
-    const std::vector<int> refills = {1, 2, 4, 8, 16};
-    const std::vector<int> fresnels = {1, 4, 8, 12, 16};
+    const std::vector<int> refills = {2, 4, 6, 8, 16};
+    const std::vector<int> fresnels = {8, 16, 24, 28, 32};
     auto try_cfg = [&](const fd2::TransportConfig &k) {
         // the CTA's shared memory must fit ctas_per_sm times (set_config
         // shrinks the PRF window to fit; without it, skip)

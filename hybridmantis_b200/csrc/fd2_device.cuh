@@ -86,9 +86,21 @@ struct RngKey {
 
 // ---------------------------------------------------------------- walker
 
+// a b + c d with c d rounded and a b fused, and a b + c d + e f with c d
+// rounded and the others fused.  Written out because which product of a sum
+// the compiler fuses depends on the code around it: the transport's kernel
+// variants must round a walk alike (a column billiard turns a last-bit
+// difference into another history), so that label runs, geometry scans and
+// single-geometry runs of the same photons keep giving the same tallies.
+__device__ __forceinline__ float sum2(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }
+__device__ __forceinline__ float sum3(float a, float b, float c, float d, float e, float f)
+{
+    return __fmaf_rn(e, f, sum2(a, b, c, d));
+}
+
 __device__ __forceinline__ void renorm(float &x, float &y, float &z)
 {
-    const float nrm = sqrtf(x * x + y * y + z * z);
+    const float nrm = sqrtf(sum3(x, x, y, y, z, z));
     if (nrm < 1.0f - kEps || nrm > 1.0f + kEps) {
         const float inv = 1.0f / nrm;
         x *= inv; y *= inv; z *= inv;
@@ -102,14 +114,14 @@ __device__ __forceinline__ float fresnel(float c, float ct, float eta)
     const float a = eta * c, b = eta * ct;
     const float rs = __fdividef(a - ct, a + ct);
     const float rp = __fdividef(c - b, c + b);
-    return 0.5f * (rs * rs + rp * rp);
+    return 0.5f * sum2(rs, rs, rp, rp);
 }
 
 // Larger root of a t^2 + b t + c = 0 (the far wall of the column), without
 // cancellation; 999 where the reference's formula yields NaN.
 __device__ __forceinline__ float wall_root(float qa, float qb, float qc)
 {
-    float disc = qb * qb - 4.0f * qa * qc;
+    float disc = sum2(-(4.0f * qa), qc, qb, qb);
     if (fabsf(disc) < 2.44140625e-4f * (qb * qb)) {
         // near-cancelling discriminant: products of floats are exact in FP64
         disc = (float)((double)qb * (double)qb - 4.0 * (double)qa * (double)qc);
@@ -205,7 +217,7 @@ struct Walker {
         // |q|^2 = (1 - u1^2) + (2 u1 - 1)^2 = 3 u1^2 - 4 u1 + 2 for u1 in (0, 1)
         const float bq = beta * rsqrtf(fmaf(u1, fmaf(3.0f, u1, -4.0f), 2.0f));
         const float rx = fmaf(bq, qx, nx), ry = fmaf(bq, qy, ny), rz = fmaf(bq, qz, nz);
-        const float ir = rsqrtf(rx * rx + ry * ry + rz * rz);
+        const float ir = rsqrtf(sum3(rx, rx, ry, ry, rz, rz));
         nx = rx * ir; ny = ry * ir; nz = rz * ir;
     }
 
@@ -225,7 +237,7 @@ struct Walker {
         const float qx = rr * c, qy = rr * s;
         const float iq = rsqrtf(fmaf(u1, fmaf(3.0f, u1, -4.0f), 2.0f));  // 1 / |q|, as in roughen
         const float vx = fmaf(iq, qx, ix), vy = fmaf(iq, qy, iy);
-        const float inv = rsqrtf(vx * vx + vy * vy);
+        const float inv = rsqrtf(sum2(vx, vx, vy, vy));
         nx = vx * inv;
         ny = vy * inv;
         nz = 0.0f;
@@ -254,9 +266,9 @@ struct Walker {
     __device__ __forceinline__ int flight(const G &g)
     {
         const float ddx = px - xc, ddy = py - yc;
-        const float qa = dx * dx + dy * dy;
-        const float qb = 2.0f * (ddx * dx + ddy * dy);
-        const float qc = ddx * ddx + ddy * ddy - g.R * g.R;
+        const float qa = sum2(dy, dy, dx, dx);
+        const float qb = 2.0f * sum2(ddy, dy, ddx, dx);
+        const float qc = __fmaf_rn(-g.R, g.R, sum2(ddy, ddy, ddx, ddx));
         const float dcyl = wall_root(qa, qb, qc);
         float d = dcyl;
         if (dz != 0.0f) {
@@ -274,14 +286,14 @@ struct Walker {
         py = fmaf(d, dy, py);
         if (outside_detector(g)) return kLost;
         const float thr = g.R - 1e-5f;
-        float r = sqrtf((px - xc) * (px - xc) + (py - yc) * (py - yc));
+        float r = sqrtf(sum2(px - xc, px - xc, py - yc, py - yc));
         float step = 0.5f;
         int moved = 0, halved = 0;
         while (r > thr && moved < 10 && halved < 10) {
             const float sx = px, sy = py;
             px = fmaf(-step, dx, px);
             py = fmaf(-step, dy, py);
-            const float rn = sqrtf((px - xc) * (px - xc) + (py - yc) * (py - yc));
+            const float rn = sqrtf(sum2(px - xc, px - xc, py - yc, py - yc));
             if (rn > r) {
                 px = sx; py = sy;
                 step *= 0.5f;
@@ -326,7 +338,7 @@ struct Walker {
         for (;;) {
             flat_rough(ix, iy, iz);
             if (always_rough || g.beta > 0.0f) roughen(g.beta);
-            if (!(ix * nx + iy * ny + iz * nz < kCos157)) return kAlive;
+            if (!(sum3(iy, ny, ix, nx, iz, nz) < kCos157)) return kAlive;
             if (tries < 100) {
                 ++tries;
                 continue;
@@ -517,7 +529,7 @@ struct Walker {
         const float ix = -dx, iy = -dy, iz = -dz;
         flat_rough(ix, iy, iz);
         if (g.beta > 0.0f) roughen(g.beta);
-        if (!(ix * nx + iy * ny + iz * nz < kCos157)) {
+        if (!(sum3(iy, ny, ix, nx, iz, nz) < kCos157)) {
             xc = fmaf(-g.R, nx, px);
             yc = fmaf(-g.R, ny, py);
             return kAlive;
@@ -545,7 +557,7 @@ struct Walker {
             if (stage == kNewSurface) {
                 if (!outside) {
                     const float ax = xc - px, ay = yc - py;
-                    const float im = rsqrtf(ax * ax + ay * ay);
+                    const float im = rsqrtf(sum2(ay, ay, ax, ax));
                     nx = ax * im; ny = ay * im; nz = 0.0f;
                     if (g.beta > 0.0f) roughen(g.beta);
                 } else {
@@ -569,7 +581,7 @@ struct Walker {
                 stage = kIncidence;
             }
             if (stage == kIncidence) {
-                const float c1 = -(dx * nx + dy * ny + dz * nz);
+                const float c1 = -sum3(dy, ny, dx, nx, dz, nz);
                 if (c1 > 1.0f || c1 < 0.0f) {
                     if (outside) {
                         const int f = new_column_normal(g, -dx, -dy, -dz, tries_normal, false);
@@ -608,7 +620,7 @@ struct Walker {
                     dy = fmaf(2.0f * c1, ny, dy);
                     dz = fmaf(2.0f * c1, nz, dz);
                     renorm(dx, dy, dz);
-                    if (kx * dx + ky * dy + kz * dz < kCos157) {
+                    if (sum3(ky, dy, kx, dx, kz, dz) < kCos157) {
                         if (++reperturbs < 4) {
                             stage = kRestore;
                             continue;
@@ -629,9 +641,9 @@ struct Walker {
                     // refraction with the reference's formula
                     const float ratio = si > 0.0f ? __fdividef(st, si) : 0.0f;
                     const float tx = fmaf(c1, nx, dx), ty = fmaf(c1, ny, dy), tz = fmaf(c1, nz, dz);
-                    dx = -ct * nx - ratio * tx;
-                    dy = -ct * ny - ratio * ty;
-                    dz = -ct * nz - ratio * tz;
+                    dx = sum2(-ct, nx, -ratio, tx);
+                    dy = sum2(-ct, ny, -ratio, ty);
+                    dz = sum2(-ct, nz, -ratio, tz);
                     renorm(dx, dy, dz);
                     if (outside) break;  // entered the next column: done
                     stage = kLeave;

@@ -323,20 +323,32 @@ struct Slot {
     uint32_t geom;
 };
 constexpr int kRing = 32;
+// Photons a warp holds beside its lanes' (in shared memory), and the 16-byte
+// words of one: position, direction, column centre, path length, absorption
+// budget, boundary count, tag (event slot and geometry), random state.
+constexpr int kPark = 32;
+constexpr int kParkWords = 4;
+// Waiting photons that start a pass once the queue and the ready photons are
+// used up: waiting for more would only idle lanes then.
+constexpr int kTailBatch = 8;
 
 // Shared-memory layout of the transport kernel (dynamic).
 struct SmemLayout {
-    size_t geom, ring, cnt, dist, win, total;
+    size_t geom, park, event, ring, cnt, dist, win, total;
     __host__ __device__ SmemLayout(int block, int n_geom, int window)
     {
         size_t o = 0;
         geom = o;
         o += sizeof(DevGeom) * (size_t)n_geom;
         o = (o + 15) & ~(size_t)15;
+        park = o;
+        o += sizeof(float4) * (size_t)(block / 32) * kParkWords * kPark;
+        event = o;
+        o += sizeof(float4) * (size_t)(block / 32) * (32 + kPark);
         ring = o;
         o += sizeof(Slot) * (size_t)(block / 32) * kRing;
         cnt = o;
-        o += sizeof(unsigned) * (size_t)n_geom * kCounterStride;
+        o += sizeof(unsigned) * (size_t)(n_geom == 1 ? kCounterStride : 0);  // kAgg: one geometry
         dist = o;
         o += sizeof(float) * (size_t)n_geom;
         o = (o + 15) & ~(size_t)15;
@@ -347,10 +359,20 @@ struct SmemLayout {
 };
 
 // Persistent transport.  Each warp keeps a ring of up to 32 chunk slots in
-// shared memory, filled with one coalesced load per lane; each lane owns one
-// photon at a time and takes a new one from the ring as soon as (or, with
-// refill > 1, once enough lanes of the warp are) idle, so lanes never wait
-// for the longest walk in the warp.  Tallies: by default every ended photon
+// shared memory, filled with one coalesced load per lane; each lane runs one
+// photon at a time and takes another as soon as (or, with refill > 1, once
+// enough lanes of the warp are) idle, so lanes never wait for the longest walk
+// in the warp.  What bounds the kernel is instruction issue, so what counts is
+// how many lanes of a warp share each instruction.  Photons that wait for the
+// rarer, longer part of the walk (the Fresnel part at a wall; with a column
+// lattice the flight through the gap) leave their lane for the warp's shared
+// memory (up to 32, 64 bytes each) and the lane goes on with another photon;
+// once `fresnel_batch` wait, they are exchanged into the lanes and that part
+// runs for all of them, the photons they displaced waiting as ready ones.
+// Photons that waited in their lane for 8 others had the Fresnel part run at
+// 9.1 lanes for a third of the warps' time and steps at 25 lanes; 20,000
+// config-1 x-rays 59.2 -> 51.6 ms, with a square / hexagonal lattice 109 / 151
+// -> 77 / 97 ms (one B200).  Tallies: by default every ended photon
 // adds to the global fates, per-primary counts and PRF with one L2
 // reduction of its lane; with kAgg (tally_mode 1) they are aggregated across
 // the warp before touching memory and the PRF core of geometry 0 is tallied
@@ -375,42 +397,115 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
 
     if (kMulti)
         for (int i = threadIdx.x; i < a.n_geom; i += blockDim.x) s_geom[i] = a.geoms[i];
-    for (int i = threadIdx.x; i < a.n_geom * kCounterStride; i += blockDim.x) s_cnt[i] = 0;
+    if (kAgg)
+        for (int i = threadIdx.x; i < kCounterStride; i += blockDim.x) s_cnt[i] = 0;
     for (int i = threadIdx.x; i < a.n_geom; i += blockDim.x) s_dist[i] = 0.0f;
     for (int i = threadIdx.x; i < win * win; i += blockDim.x) s_win[i] = 0;
     __syncthreads();
 
     Slot *ring = s_ring + wid * kRing;
+    float4 *park = reinterpret_cast<float4 *>(smem + L.park) + wid * kParkWords * kPark;
+    float4 *event = reinterpret_cast<float4 *>(smem + L.event) + wid * (32 + kPark);
     // never read past the chunk buffer, whatever the scan produced
     const unsigned long long total_chunks = min(*a.n_chunks, (unsigned long long)a.chunk_capacity);
     int ring_len = 0, slot = 0;
     uint32_t used = 0;
-    bool exhausted = false, alive = false, parked = false;
+    bool exhausted = false, alive = false;
     bool xretry = false;  // the lane's crosstalk normal is retried this round
     int xtries = 0;
-    const unsigned refill_min = (unsigned)a.refill;
-    const unsigned fresnel_min = (unsigned)max(a.fresnel_batch, 1);
+    const int refill_min = max(a.refill, 1);
+    const int batch = min(max(a.fresnel_batch, 1), kPark);
     // Philox round keys and run counter, shared by the CTA
     __shared__ uint32_t s_rk[20];
     __shared__ uint32_t s_run;
     if (threadIdx.x < 20) s_rk[threadIdx.x] = a.round_keys[threadIdx.x];
     if (threadIdx.x == 0) s_run = *a.run_tag;
 
-    __syncthreads();
     Walker w;
-    const RngKey key{s_rk, s_run};
-    int geom = 0;
-    // the lane's current event record (x, y, z, history index bits): read at
-    // a trapped restart, a detection and in label mode, so it need not stay
-    // in registers through the walk; and the lane's path-length sum
-    __shared__ float4 s_lane[kMaxThreads];
+    // The lane's tag: the shared-memory slot of its photon's event record
+    // (x, y, z, history index bits; read at a trapped restart, a detection and
+    // in label mode) in bits 0-7, the geometry above.  The warp's 64 slots are
+    // always a permutation over its lanes and parked photons.
+    uint32_t tag = lane;
+    reinterpret_cast<uint32_t *>(&park[2 * kPark + lane])[3] = 32u + lane;
+    // and the lane's path-length sum
     __shared__ float s_ldist[kMaxThreads];
     s_ldist[threadIdx.x] = 0.0f;
+    w.in_gap = false;
+    bool &parked = w.in_gap;
+    // Waiting photons [0, n_wait) and ready ones [n_wait, n_wait + n_ready) of
+    // the warp's parked photons (never more than kPark - 1 together: a photon
+    // is added only while fewer than `batch` wait and none is ready).
+    int n_wait = 0, n_ready = 0;
+    __syncthreads();
+    const RngKey key{s_rk, s_run};
 
     for (;;) {
+        // ---- which pass: a step of the lanes' photons, or the waiting ones
+        const unsigned live = __ballot_sync(kFull, alive);
+        const unsigned held = __ballot_sync(kFull, alive && parked);
+        const unsigned busy = live & ~held;
+        const int n_held = __popc(held), waiting = n_wait + n_held;
+        const bool supply = n_ready > 0 || !exhausted;
+        bool flush = waiting >= (supply ? batch : min(batch, kTailBatch)) || (waiting > 0 && !busy && !supply);
+        int at = -1;  // the parked photon this lane exchanges its own with
+        if (flush) {
+            // waiting photons into the lanes that hold none: first the empty
+            // lanes (when no photon is ready for them), then lanes whose
+            // photon can wait as a ready one
+            const unsigned none = n_ready == 0 ? ~live : 0u;
+            const unsigned other = busy & ~__ballot_sync(kFull, xretry);
+            const int n_none = __popc(none), take = min(n_wait, n_none + __popc(other));
+            const bool empty = (none >> lane) & 1u;
+            const int rank = empty ? __popc(none & lanemask_lt()) : n_none + __popc(other & lanemask_lt());
+            if ((((none | other) >> lane) & 1u) && rank < take) at = n_wait - 1 - rank;
+            n_wait -= take;
+            n_ready += take - min(take, n_none);
+            flush = n_held + take > 0;  // no lane can run one: step the others first
+        }
+        if (!flush && supply && (32 - __popc(busy) >= (exhausted ? 1 : refill_min) || !busy)) {
+            // lanes with a waiting photon park it, for a ready one if there
+            // is one; empty lanes take ready ones
+            const int left = max(n_ready - n_held, 0), n_empty = 32 - __popc(live);
+            if ((held >> lane) & 1u) {
+                const int rank = __popc(held & lanemask_lt());
+                at = n_wait + rank;
+                alive = rank < n_ready;
+            } else if (!alive) {
+                const int rank = __popc(~live & lanemask_lt());
+                if (rank < left) {
+                    at = n_wait + n_ready - 1 - rank;
+                    alive = true;
+                }
+            }
+            n_wait += n_held;
+            n_ready = left - min(left, n_empty);
+        }
+        if (__ballot_sync(kFull, at >= 0)) {
+            __syncwarp();
+            if (at >= 0) {
+                float4 *q = park + at, t = q[0];
+                q[0] = make_float4(w.px, w.py, w.pz, w.dx);
+                w.px = t.x, w.py = t.y, w.pz = t.z, w.dx = t.w;
+                t = q[kPark];
+                q[kPark] = make_float4(w.dy, w.dz, w.xc, w.yc);
+                w.dy = t.x, w.dz = t.y, w.xc = t.z, w.yc = t.w;
+                t = q[2 * kPark];
+                q[2 * kPark] = make_float4(w.dist, w.budget, __uint_as_float(w.rebound), __uint_as_float(tag));
+                w.dist = t.x, w.budget = t.y, w.rebound = __float_as_uint(t.z), tag = __float_as_uint(t.w);
+                t = q[3 * kPark];
+                q[3 * kPark] = make_float4(__uint_as_float(w.s0), __uint_as_float(w.s1), __uint_as_float(w.s2),
+                                           __uint_as_float(w.s3));
+                w.s0 = __float_as_uint(t.x), w.s1 = __float_as_uint(t.y);
+                w.s2 = __float_as_uint(t.z), w.s3 = __float_as_uint(t.w);
+                parked = flush;
+                if (flush) alive = true;
+            }
+            __syncwarp();
+        }
         // ---- hand out photons to idle lanes
         unsigned needy = __ballot_sync(kFull, !alive);
-        if (needy && !exhausted && ((unsigned)__popc(needy) >= refill_min || needy == kFull)) {
+        if (!flush && !exhausted && needy && (__popc(needy) >= refill_min || needy == kFull)) {
             while (needy) {
                 if (slot >= ring_len) {
                     // A refill takes a share of what is left: 32 chunks while
@@ -475,9 +570,10 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                 if (mine) {
                     const Slot &s = ring[slot];
                     const uint32_t k = s.first + used + rank;
-                    s_lane[threadIdx.x] = s.pos;
-                    geom = (int)s.geom;
+                    tag = (tag & 0xffu) | (s.geom << 8);
+                    event[tag & 0xffu] = s.pos;
                     w.start(s.pos.x, s.pos.y, s.pos.z, k, (uint32_t)(a.event_base + s.event), k == 0, key);
+                    parked = false;
                     if constexpr (kGrid) w.grid_place(a.g0);
                     alive = true;
                 }
@@ -486,52 +582,37 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
             }
         }
         if (__ballot_sync(kFull, alive) == 0) {
-            if (exhausted) break;
+            if (exhausted && n_wait + n_ready == 0) break;
             continue;
         }
 
-        // ---- one transport step per live lane; a lane whose photon meets a
-        // column wall without crosstalk parks it there, and the warp runs the
-        // Fresnel part for the parked lanes together once `fresnel_batch` of
-        // them wait (or nothing else runs)
+        // ---- one transport step per live lane, or the waiting photons' pass
         int fate = kAlive;
+        const int geom = (int)(tag >> 8);
         if constexpr (kGrid) {
-            // explicit column lattice: one segment per round per live lane;
-            // a lane in the gap waits until `fresnel_batch` lanes of the warp
-            // are in the gap (or no lane is in a column), so the gap's
-            // cell-by-cell search runs with more lanes at once.  Waiting only
-            // delays a photon's segments: its history is unchanged.
-            const unsigned gap = __ballot_sync(kFull, alive && w.in_gap);
-            const unsigned col = __ballot_sync(kFull, alive && !w.in_gap);
-            const bool go = alive && (!w.in_gap || (unsigned)__popc(gap) >= fresnel_min || col == 0);
-            if (go) fate = w.grid_segment(a.g0);
+            // explicit column lattice: one segment per pass, of the photons in
+            // a column or of those in the gap
+            if (alive && parked == flush) fate = w.grid_segment(a.g0);
+        } else if (flush) {
+            if (alive && parked) {
+                fate = kMulti ? w.surface_fresnel(s_geom[geom]) : w.surface_fresnel(a.g0);
+                parked = false;
+            }
         } else {
             if (alive && !parked && !xretry) {
-                fate = kMulti ? w.step(s_geom[geom], s_lane[threadIdx.x]) : w.step(a.g0, s_lane[threadIdx.x]);
+                fate = kMulti ? w.step(s_geom[geom], event[tag & 0xffu]) : w.step(a.g0, event[tag & 0xffu]);
                 if (fate == kNeedsFresnel) {
                     parked = true;
                     fate = kAlive;
                 }
             }
-            if (alive && !parked) {
-                // crosstalk: one attempt at the next column's normal per round, so
-                // a rejected attempt is retried beside the other lanes' first ones
-                if (xretry || fate == kNeedsNormal) {
-                    fate = kMulti ? w.crosstalk_normal(s_geom[geom], xtries) : w.crosstalk_normal(a.g0, xtries);
-                    xretry = fate == kRetryNormal;
-                    if (xretry) fate = kAlive;
-                    else xtries = 0;
-                }
-            }
-            const unsigned waiting = __ballot_sync(kFull, parked);
-            if (waiting) {
-                const unsigned busy = __ballot_sync(kFull, alive && !parked && fate == kAlive);
-                if ((unsigned)__popc(waiting) >= fresnel_min || busy == 0) {
-                    if (parked) {
-                        fate = kMulti ? w.surface_fresnel(s_geom[geom]) : w.surface_fresnel(a.g0);
-                        parked = false;
-                    }
-                }
+            // crosstalk: one attempt at the next column's normal per round, so
+            // a rejected attempt is retried beside the other lanes' first ones
+            if (xretry || fate == kNeedsNormal) {
+                fate = kMulti ? w.crosstalk_normal(s_geom[geom], xtries) : w.crosstalk_normal(a.g0, xtries);
+                xretry = fate == kRetryNormal;
+                if (xretry) fate = kAlive;
+                else xtries = 0;
             }
         }
 
@@ -551,10 +632,11 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                 if (kMulti) atomicAdd(&s_dist[geom], w.dist);
                 else s_ldist[threadIdx.x] += w.dist;  // lane-private: no atomic
                 alive = false;
+                parked = false;
             }
             const unsigned det = __ballot_sync(kFull, fate == kDetect);
             if (fate == kDetect) {
-                const float4 ev = s_lane[threadIdx.x];
+                const float4 ev = event[tag & 0xffu];
                 const int prim = __float_as_int(ev.w);
                 if (!kAgg) {
                     if ((unsigned)prim < (unsigned)a.n_prim) atomicAdd(&a.per_primary[prim], 1);
@@ -590,8 +672,9 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
 
     // ---- flush the CTA's private tallies
     __syncthreads();
-    for (int i = threadIdx.x; i < a.n_geom * kCounterStride; i += blockDim.x)
-        if (s_cnt[i]) atomicAdd(&a.counters[i], (unsigned long long)s_cnt[i]);
+    if (kAgg)
+        for (int i = threadIdx.x; i < kCounterStride; i += blockDim.x)
+            if (s_cnt[i]) atomicAdd(&a.counters[i], (unsigned long long)s_cnt[i]);
     if (!kMulti) {
         // the lanes' path-length sums: summed per warp in double, then added to the CTA's
         double d = (double)s_ldist[threadIdx.x];
@@ -752,7 +835,7 @@ cudaError_t launch_fill_chunks(cudaStream_t s, int64_t n, int chunk, const int32
     X(false, 256, 2, false, true, false) X(false, 320, 2, false, true, false)              \
     X(false, 256, 3, false, false, false) X(false, 256, 4, false, false, false)            \
     X(true, 512, 1, false, false, false) X(true, 256, 2, false, false, false)              \
-    X(true, 256, 3, false, false, false) X(true, 256, 2, true, false, false)               \
+    X(true, 256, 3, false, false, false) X(true, 256, 3, true, false, false)               \
     X(true, 256, 4, false, false, false) X(false, 256, 3, false, true, false)              \
     X(false, 512, 1, false, false, true) X(false, 256, 2, false, false, true)              \
     X(false, 320, 2, false, false, true) X(false, 256, 3, false, false, true)              \
@@ -793,12 +876,17 @@ cudaError_t launch_transport(cudaStream_t s, const TransportConfig &cfg, int sm_
 {
     TransportArgs a = args;
     const size_t smem = transport_smem_bytes(cfg, a.n_geom);
-    const unsigned grid = (unsigned)(sm_count * cfg.ctas_per_sm);
+    const bool multi = a.n_geom > 1;
+    // label mode, 256 threads: one geometry (the surrogate's audit) as the
+    // production kernel, four CTAs per SM, else (training labels) three (80
+    // registers without a spill; 64 geometries x 100 points x 4,000 photons:
+    // 22.9 ms, 28.5 ms with two)
+    const int per_sm_label = !multi && cfg.ctas_per_sm >= 4 ? 4 : 3;
+    const unsigned grid = (unsigned)(sm_count * (a.radial ? per_sm_label : cfg.ctas_per_sm));
     // a refill takes 1 / 2^pull_shift of the chunks left: at most half of a
     // warp's even share
     for (a.pull_shift = 1; (1ll << a.pull_shift) < 2ll * grid * (cfg.block / 32); ++a.pull_shift) {
     }
-    const bool multi = a.n_geom > 1;
     const int per_sm = cfg.block > 256 ? 1 : std::min(std::max(cfg.ctas_per_sm, 2), 4);
     if (a.g0.grid) {
         // explicit column lattice: single geometry, 256 or 320 threads
@@ -808,14 +896,9 @@ cudaError_t launch_transport(cudaStream_t s, const TransportConfig &cfg, int sm_
         else if (cfg.block <= 256) transport_kernel<false, 256, 2, false, true><<<grid, cfg.block, smem, s>>>(a);
         else return cudaErrorInvalidConfiguration;
     } else if (a.radial) {
-        // label mode, 256 threads: one geometry (the surrogate's audit) as the
-        // production kernel, four CTAs per SM; several geometries (training
-        // labels) two CTAs per SM
         if (cfg.block > 256) return cudaErrorInvalidConfiguration;
-        if (!multi && cfg.ctas_per_sm >= 4)
-            transport_kernel<false, 256, 4, true><<<(unsigned)(sm_count * 4), cfg.block, smem, s>>>(a);
-        else
-            transport_kernel<true, 256, 2, true><<<(unsigned)(sm_count * 2), cfg.block, smem, s>>>(a);
+        if (per_sm_label == 4) transport_kernel<false, 256, 4, true><<<grid, cfg.block, smem, s>>>(a);
+        else transport_kernel<true, 256, 3, true><<<grid, cfg.block, smem, s>>>(a);
     } else if (!multi && cfg.aggregate) {
         // warp-aggregated, shared-memory privatised tallies (tally_mode 1)
         if (cfg.block == 320) transport_kernel<false, 320, 2, false, false, true><<<grid, cfg.block, smem, s>>>(a);
