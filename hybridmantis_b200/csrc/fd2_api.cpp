@@ -373,7 +373,8 @@ void fit_window(fd2_ctx *c)
 
 // Launch shape unless the options give one, measured on a B200: one geometry
 // 256 threads x 4 CTAs per SM (32 warps at 64 registers; 20,000 config-1
-// x-rays 51.6 ms against 55.6 for 256 x 3), chunks of 16 photons; several
+// x-rays 51.6 ms against 54.1 for 224 x 4 and 55.6 for 256 x 3, before the
+// steps below a full exchange were looped), chunks of 16 photons; several
 // geometries 256 x 3 (configuration 2, 500 x-rays: 73.0 ms against 90.6 for
 // 256 x 2; 256 x 4 the same); the column lattice 256 x 3 (10,001 config-1
 // x-rays 77.2 ms against 82.5 for 320 x 2); label mode with one geometry
@@ -634,9 +635,9 @@ fd2_status fd2_create(const fd2_params *p, const fd2_options *opt, fd2_ctx **out
     if ((st = alloc_tallies(c)) != FD2_OK) return bail(st);
     fd2::TransportConfig cfg;
     default_launch(c, 1, &cfg);
-    // idle lanes that trigger a refill (20,000 config-1 x-rays: 2 / 4 / 6 / 8
-    // lanes 53.4 / 51.9 / 51.7 / 52.1 ms; the lattice 78.3 / 77.3 / 77.2 / 77.9)
-    cfg.refill = c->opt.refill > 0 ? c->opt.refill : 6;
+    // idle lanes that trigger a refill (20,000 config-1 x-rays: 4 / 6 / 8 / 10
+    // lanes 47.8 / 46.5 / 46.0 / 46.2 ms; the lattice 71.6 / 70.3 / 70.3 / 71.0)
+    cfg.refill = c->opt.refill > 0 ? c->opt.refill : 8;
     // photons waiting for the Fresnel part (with a lattice: in the gap) before
     // the warp runs it for them: a full warp's (16 / 24 / 32 photons: 56.7 /
     // 53.3 / 51.9 ms, hexagonal lattice 114 ms at 24, 104 at 32)
@@ -1239,7 +1240,7 @@ fd2_status fd2_autotune(fd2_ctx *c, int32_t budget_runs)
     // refill and Fresnel batch one knob at a time, twice over
     const std::vector<std::pair<int, int>> shapes = {{256, 4}, {128, 8}, {256, 3}, {320, 2}, {256, 2}, {512, 1}};
     const std::vector<int> chunks = {8, 16, 32, 64, 128};
-    const std::vector<int> refills = {2, 4, 6, 8, 16};
+    const std::vector<int> refills = {4, 6, 8, 10, 16};
     const std::vector<int> fresnels = {8, 16, 24, 28, 32};
     auto try_cfg = [&](const fd2::TransportConfig &k) {
         // the CTA's shared memory must fit ctas_per_sm times (set_config

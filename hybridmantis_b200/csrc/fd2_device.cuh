@@ -126,13 +126,26 @@ __device__ __forceinline__ float wall_root(float qa, float qb, float qc)
         // near-cancelling discriminant: products of floats are exact in FP64
         disc = (float)((double)qb * (double)qb - 4.0 * (double)qa * (double)qc);
     }
-    if (!(qa > 0.0f) || !(disc >= 0.0f)) return 999.0f;
+    // one division for both signs of qb, chosen by selects: the lanes of a
+    // warp have both
     const float s = sqrtf(disc);
-    if (qb >= 0.0f) {
-        const float den = qb + s;
-        return den != 0.0f ? (-2.0f * qc) / den : 0.0f;
+    const bool far = qb >= 0.0f;
+    const float den = far ? qb + s : 2.0f * qa;
+    float t = (far ? -2.0f * qc : s - qb) / den;
+    t = far && den == 0.0f ? 0.0f : t;
+    return !(qa > 0.0f) || !(disc >= 0.0f) ? 999.0f : t;
+}
+
+// The PRF pixel of a photon detected at (x, y); -1 outside the PRF's bounds.
+template <class G>
+__device__ __forceinline__ void detection_pixel(const G &g, float x, float y, int &ii, int &jj)
+{
+    ii = -1;
+    jj = -1;
+    if (x <= g.ub_x && y <= g.ub_y && x >= g.lb_x && y >= g.lb_y) {
+        ii = (int)floorf(__fdiv_rn(x - g.lb_x, g.pixel));
+        jj = (int)floorf(__fdiv_rn(y - g.lb_y, g.pixel));
     }
-    return (s - qb) / (2.0f * qa);
 }
 
 struct Walker {
@@ -144,7 +157,6 @@ struct Walker {
     float dist;         // path length
     float budget;       // absorption lengths left before bulk absorption
     uint32_t rebound;   // boundary interactions
-    int ii, jj;         // detection pixel (-1: outside the PRF bounds)
     // The photon's random stream: xoshiro128+ state (never all zero; a
     // Philox block is all zero with probability 2^-128, and start() then
     // sets one bit).  The float uses the top 23 bits of each output, the
@@ -181,7 +193,6 @@ struct Walker {
         nx = 0.0f; ny = 0.0f; nz = 0.0f;
         dist = 0.0f;
         rebound = 0;
-        ii = -1; jj = -1;
         emit(first);
         budget = -__logf(u());  // Exp(1)
     }
@@ -261,7 +272,8 @@ struct Walker {
     }
 
     // Wall or z plane ahead, then the reference's pull-back into the column
-    // (dist_to_surface), then bulk absorption (isotropic).
+    // (dist_to_surface), then bulk absorption (isotropic).  Selects instead of
+    // early exits: few lanes of a warp leave at any one of them.
     template <class G>
     __device__ __forceinline__ int flight(const G &g)
     {
@@ -270,26 +282,20 @@ struct Walker {
         const float qb = 2.0f * sum2(ddy, dy, ddx, dx);
         const float qc = __fmaf_rn(-g.R, g.R, sum2(ddy, ddy, ddx, ddx));
         const float dcyl = wall_root(qa, qb, qc);
-        float d = dcyl;
-        if (dz != 0.0f) {
-            const float zp = dz > 0.0f ? g.half : -g.half;
-            const bool straight = fabsf(dx) < kEps && fabsf(dy) < kEps && fabsf(fabsf(dz) - 1.0f) < kEps;
-            const float dplane = (zp - pz) / dz;
-            if (!straight && dplane >= dcyl) {
-                pz = fmaf(d, dz, pz);
-            } else {
-                d = dplane;
-                pz = zp;
-            }
-        }
+        const float zp = dz > 0.0f ? g.half : -g.half;
+        const bool straight = fabsf(dx) < kEps && fabsf(dy) < kEps && fabsf(fabsf(dz) - 1.0f) < kEps;
+        const float dplane = (zp - pz) / dz;
+        const bool plane = dz != 0.0f && (straight || !(dplane >= dcyl));
+        const float d = plane ? dplane : dcyl;
+        pz = plane ? zp : fmaf(d, dz, pz);
         px = fmaf(d, dx, px);
         py = fmaf(d, dy, py);
-        if (outside_detector(g)) return kLost;
+        const bool lost = outside_detector(g);
         const float thr = g.R - 1e-5f;
         float r = sqrtf(sum2(px - xc, px - xc, py - yc, py - yc));
         float step = 0.5f;
         int moved = 0, halved = 0;
-        while (r > thr && moved < 10 && halved < 10) {
+        while (r > thr && !lost && moved < 10 && halved < 10) {
             const float sx = px, sy = py;
             px = fmaf(-step, dx, px);
             py = fmaf(-step, dy, py);
@@ -303,30 +309,18 @@ struct Walker {
                 ++moved;
             }
         }
-        if (r > thr) return kOutOfCol;
-        if (outside_detector(g)) return kLost;
-        dist += d;
+        int fate = lost ? kLost : r > thr ? kOutOfCol : outside_detector(g) ? kLost : kAlive;
+        dist += fate == kAlive ? d : 0.0f;
         if (g.neg_inv_mu != 0.0f) {
             // bulk absorption: one Exp(1) budget of absorption lengths per
             // photon, spent flight by flight; by the exponential's lack of
             // memory the same law as the reference's fresh draw per flight
             // (absorbed when d >= -ln(u) / mu)
             const float da = d * g.mu;
-            if (da >= budget && d >= 0.0f) return kAbsBulk;
+            fate = fate == kAlive && da >= budget && d >= 0.0f ? kAbsBulk : fate;
             budget -= da;
         }
-        return kAlive;
-    }
-
-    template <class G>
-    __device__ __forceinline__ void set_pixel(const G &g)
-    {
-        ii = -1;
-        jj = -1;
-        if (px <= g.ub_x && py <= g.ub_y && px >= g.lb_x && py >= g.lb_y) {
-            ii = (int)floorf(__fdiv_rn(px - g.lb_x, g.pixel));
-            jj = (int)floorf(__fdiv_rn(py - g.lb_y, g.pixel));
-        }
+        return fate;
     }
 
     // Orientation of the next column: a random normal within 1.57 rad of
@@ -407,7 +401,6 @@ struct Walker {
             } else if (st == kSensor) {
                 // sensor between columns: reflect with sensorRefl, else detect
                 if (!(g.sensor_refl > 0.0f && u() < g.sensor_refl)) {
-                    set_pixel(g);
                     return kDetect;
                 }
                 dz = -dz;
@@ -488,32 +481,34 @@ struct Walker {
         }
     }
 
-    // Interaction with a surface (boundary_analysis), first part: the top
-    // surface and columnar crosstalk.  Returns a fate, kAlive, or
-    // kNeedsFresnel when the photon meets the column wall without crosstalk;
-    // the Fresnel part (surface_fresnel) can then run later, from the photon
-    // state alone.
+    // Top reflector above the columns: absorb, or diffuse reflection down.
+    template <class G>
+    __device__ __forceinline__ int top_reflector(const G &g)
+    {
+        if (g.top_absfrac > 0.0f && u() < g.top_absfrac) return kAbsTop;
+        dz = -fabsf(2.0f * u() - 1.0f);
+        const float rr = sqrtf(fmaxf(0.0f, 1.0f - dz * dz));
+        float s, c;
+        __sincosf(kPi * (2.0f * u() - 1.0f), &s, &c);
+        dx = rr * c;
+        dy = rr * s;
+        return kAlive;
+    }
+
+    // Interaction with a column wall (boundary_analysis), first part: whether
+    // the photon crosses into the adjacent column (kNeedsNormal) or meets the
+    // wall (kNeedsFresnel); the rest (crosstalk_normal, surface_wait) can run
+    // later, from the photon state alone.
     template <class G>
     __device__ __forceinline__ int surface_entry(const G &g)
     {
-        if (at_top(g)) {
-            if (g.top_absfrac > 0.0f && u() < g.top_absfrac) return kAbsTop;
-            dz = -fabsf(2.0f * u() - 1.0f);
-            const float rr = sqrtf(fmaxf(0.0f, 1.0f - dz * dz));
-            float s, c;
-            __sincosf(kPi * (2.0f * u() - 1.0f), &s, &c);
-            dx = rr * c;
-            dy = rr * s;
-            return kAlive;
-        }
         // columnar crosstalk: certain in the top 20 %, linear to 0.5 at mid
         // depth, back to 1 at the sensor
-        float cct = 0.0f;
-        if (pz <= g.half && pz >= g.cct_band_lo) cct = 1.0f;
-        else if (pz < g.cct_band_lo && pz >= 0.0f) cct = fmaf(pz, g.cct_k_hi, 0.5f);
-        else if (pz < 0.0f && pz >= -g.half) cct = fmaf(pz + g.half, g.cct_k_lo, 1.0f);
-        if (!(u() < cct)) return kNeedsFresnel;
-        return kNeedsNormal;
+        const float above = fmaf(pz, g.cct_k_hi, 0.5f), below = fmaf(pz + g.half, g.cct_k_lo, 1.0f);
+        float cct = pz < 0.0f && pz >= -g.half ? below : 0.0f;
+        cct = pz < g.cct_band_lo && pz >= 0.0f ? above : cct;
+        cct = pz <= g.half && pz >= g.cct_band_lo ? 1.0f : cct;
+        return u() < cct ? kNeedsNormal : kNeedsFresnel;
     }
 
     // Crosstalk into the adjacent column (transmit with crosstalk): one
@@ -539,6 +534,14 @@ struct Walker {
             return kRetryNormal;
         }
         return kTheta1;
+    }
+
+    // What a waiting photon waits for: the top reflector or the wall.
+    template <class G>
+    __device__ __forceinline__ int surface_wait(const G &g)
+    {
+        if (at_top(g)) return top_reflector(g);
+        return surface_fresnel(g);
     }
 
     // Second part: Fresnel reflection / refraction on the rough wall, with
@@ -691,7 +694,7 @@ struct Walker {
             for (int q = 0; q < 5; ++q) {
                 float cx, cy;
                 hex_candidate(g, i, j, q, cx, cy);
-                const float d2 = (px - cx) * (px - cx) + (py - cy) * (py - cy);
+                const float d2 = sum2(px - cx, px - cx, py - cy, py - cy);
                 if (d2 < bd) { bd = d2; bx = cx; by = cy; }
             }
             xc = bx;
@@ -702,7 +705,7 @@ struct Walker {
         xc = (floorf(px / g.pitch) + 0.5f) * g.pitch;
         yc = (floorf(py / g.pitch) + 0.5f) * g.pitch;
         const float rx = px - xc, ry = py - yc;
-        in_gap = rx * rx + ry * ry >= g.R * g.R;
+        in_gap = sum2(rx, rx, ry, ry) >= g.R * g.R;
     }
 
     // Hexagonal lattice: the rows are strips of height h; in row j the
@@ -729,18 +732,8 @@ struct Walker {
     template <class G>
     __device__ __forceinline__ int grid_plane(const G &g, bool top)
     {
-        if (top) {
-            if (g.top_absfrac > 0.0f && u() < g.top_absfrac) return kAbsTop;
-            dz = -fabsf(2.0f * u() - 1.0f);
-            const float rr = sqrtf(fmaxf(0.0f, 1.0f - dz * dz));
-            float s, c;
-            __sincosf(kPi * (2.0f * u() - 1.0f), &s, &c);
-            dx = rr * c;
-            dy = rr * s;
-            return kAlive;
-        }
+        if (top) return top_reflector(g);
         if (!(g.sensor_refl > 0.0f && u() < g.sensor_refl)) {
-            set_pixel(g);
             return kDetect;
         }
         dz = -dz;
@@ -755,7 +748,7 @@ struct Walker {
     __device__ __forceinline__ int grid_wall(const G &g, float cx, float cy, bool inside)
     {
         float ox = px - cx, oy = py - cy;
-        const float inv = rsqrtf(ox * ox + oy * oy);
+        const float inv = rsqrtf(sum2(oy, oy, ox, ox));
         ox *= inv;
         oy *= inv;
         const float sgn = inside ? -1.0f : 1.0f;  // normal toward the incident medium
@@ -763,12 +756,12 @@ struct Walker {
         for (int t = 0; t < 8; ++t) {
             nx = sgn * ox; ny = sgn * oy; nz = 0.0f;
             if (g.beta > 0.0f) roughen(g.beta);
-            c1 = -(dx * nx + dy * ny + dz * nz);
+            c1 = -sum3(dy, ny, dx, nx, dz, nz);
             if (c1 > 0.0f) break;
         }
         if (!(c1 > 0.0f)) {
             nx = sgn * ox; ny = sgn * oy; nz = 0.0f;
-            c1 = fmaxf(-(dx * nx + dy * ny), 0.0f);
+            c1 = fmaxf(-sum2(dx, nx, dy, ny), 0.0f);
         }
         const float eta = inside ? g.eta_in : g.eta_out;  // n_incident / n_transmitted
         const float st2 = eta * eta * fmaxf(0.0f, 1.0f - c1 * c1);
@@ -807,11 +800,11 @@ struct Walker {
         const float dplane = dz != 0.0f ? (zp - pz) / dz : 3.0e38f;
         if (!in_gap) {
             const float ddx = px - xc, ddy = py - yc;
-            const float qa = dx * dx + dy * dy;
-            const float qb = 2.0f * (ddx * dx + ddy * dy);
+            const float qa = sum2(dy, dy, dx, dx);
+            const float qb = 2.0f * sum2(ddy, dy, ddx, dx);
             // a photon on the wall (rounded just outside it) is on the wall:
             // the far root then always exists
-            const float qc = fminf(ddx * ddx + ddy * ddy - g.R * g.R, 0.0f);
+            const float qc = fminf(__fmaf_rn(-g.R, g.R, sum2(ddy, ddy, ddx, ddx)), 0.0f);
             const float dw = wall_root(qa, qb, qc);
             const bool plane = dplane <= dw;
             const float d = fmaxf(plane ? dplane : dw, 0.0f);
@@ -847,7 +840,7 @@ struct Walker {
             const float h = p * 0.8660254037844386f;
             int j = (int)floorf(py / h);
             int i = (int)floorf((px - ((j & 1) ? 0.5f * p : 0.0f)) / p);
-            const float qa = dx * dx + dy * dy;
+            const float qa = sum2(dy, dy, dx, dx);
             float tin = 0.0f;
             for (int k = 0; k < kMaxGridCells; ++k) {
                 const float o = (j & 1) ? 0.5f * p : 0.0f;
@@ -864,7 +857,7 @@ struct Walker {
                     const float qb = 2.0f * (fx * dx + fy * dy);
                     const float qc = fx * fx + fy * fy - g.R * g.R;
                     if (qa > 0.0f && qb < 0.0f) {
-                        const float disc = qb * qb - 4.0f * qa * qc;
+                        const float disc = sum2(qb, qb, -(4.0f * qa), qc);
                         if (disc >= 0.0f) {
                             const float t1 = (2.0f * qc) / (-qb + sqrtf(disc));
                             if (t1 > 1e-4f && t1 >= tin - 1e-4f && t1 <= tout + 1e-4f && t1 < tb) {
@@ -912,14 +905,14 @@ struct Walker {
         float tmy = dy != 0.0f ? (((float)(dy > 0.0f ? j + 1 : j)) * p - py) / dy : 3.0e38f;
         const float tdx = dx != 0.0f ? p / fabsf(dx) : 3.0e38f;
         const float tdy = dy != 0.0f ? p / fabsf(dy) : 3.0e38f;
-        const float qa = dx * dx + dy * dy;
+        const float qa = sum2(dy, dy, dx, dx);
         for (int k = 0; k < kMaxGridCells; ++k) {
             const float cx = ((float)i + 0.5f) * p, cy = ((float)j + 0.5f) * p;
             const float fx = px - cx, fy = py - cy;
-            const float qb = 2.0f * (fx * dx + fy * dy);
-            const float qc = fx * fx + fy * fy - g.R * g.R;
+            const float qb = 2.0f * sum2(fx, dx, fy, dy);
+            const float qc = __fmaf_rn(-g.R, g.R, sum2(fx, fx, fy, fy));
             if (qa > 0.0f && qb < 0.0f) {
-                const float disc = qb * qb - 4.0f * qa * qc;
+                const float disc = sum2(qb, qb, -(4.0f * qa), qc);
                 if (disc >= 0.0f) {
                     const float t1 = (2.0f * qc) / (-qb + sqrtf(disc));  // the entry root
                     if (t1 > 1e-4f && t1 < tend) {
@@ -971,27 +964,26 @@ struct Walker {
 
     // One transport step (the body of the reference's step function algo):
     // flight, sensor, trapped-photon restart (from `event`, the x, y, z of
-    // the photon's event), or a surface interaction up to the Fresnel part.  Returns the photon's fate, kAlive while it is in
-    // flight, or kNeedsFresnel (run surface_fresnel next).
+    // the photon's event), or a surface interaction up to the part that waits.
+    // Returns the photon's fate, kAlive while it is in flight, kNeedsNormal
+    // (run crosstalk_normal next) or kNeedsFresnel (surface_wait next).  A
+    // photon reflected by the sensor inside a column flies on in its next step,
+    // beside the warp's others; `reflected` then keeps it from meeting the
+    // sensor again where it stands.
     template <class G>
-    __device__ __forceinline__ int step(const G &g, const float4 &event)
+    __device__ __forceinline__ int step(const G &g, const float4 &event, bool &reflected)
     {
-        // one flight, and a second after a specular reflection on the sensor
-        // inside a column (a loop, so that the kernel holds one flight)
-        bool reflected = false;
-#pragma unroll 1
-        for (;;) {
-            const int f = flight(g);
-            if (f != kAlive) return f;
-            if (reflected || !(fabsf(pz + g.half) < kEps)) break;
+        const int f = flight(g);
+        if (f != kAlive) return f;
+        const bool sensor = !reflected && fabsf(pz + g.half) < kEps;
+        reflected = false;
+        if (sensor) {
             // sensor plane inside a column (detection)
-            if (!(g.sensor_refl > 0.0f && u() < g.sensor_refl)) {
-                set_pixel(g);
-                return kDetect;
-            }
+            if (!(g.sensor_refl > 0.0f && u() < g.sensor_refl)) return kDetect;
             dz = -dz;  // specular reflection on the flat sensor
             renorm(dx, dy, dz);
             reflected = true;
+            return kAlive;
         }
         if (fabsf(dz) < kEps) {
             // trapped travelling horizontally: restart from the event position,
@@ -1001,6 +993,7 @@ struct Walker {
             return kAlive;
         }
         if (++rebound > kMaxBoundaryCalls) return kCapped;
+        if (at_top(g)) return kNeedsFresnel;
         return surface_entry(g);
     }
 };

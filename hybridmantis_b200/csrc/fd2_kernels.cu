@@ -328,27 +328,35 @@ constexpr int kRing = 32;
 // budget, boundary count, tag (event slot and geometry), random state.
 constexpr int kPark = 32;
 constexpr int kParkWords = 4;
+// Ended photons a warp holds: fewer than 32 wait, and up to 32 end in a pass.
+constexpr int kEnded = 64;
 // Waiting photons that start a pass once the queue and the ready photons are
 // used up: waiting for more would only idle lanes then.
 constexpr int kTailBatch = 8;
 
-// Shared-memory layout of the transport kernel (dynamic).
+// A warp's shared memory: its parked and ended photons, its photons' event
+// records, and its ring of chunks.
+struct WarpMem {
+    float4 park[kParkWords * kPark];
+    float4 event[32 + kPark];
+    float4 ended[kEnded];
+    Slot ring[kRing];
+    int slot, len;   // the ring's current slot and its filled slots
+    uint32_t used;   // photons of the current slot handed out
+    uint32_t pad;
+};
+
+// Shared-memory layout of the transport kernel (dynamic): the warps' blocks,
+// at constant offsets of the warp's base so that one register addresses them.
 struct SmemLayout {
-    size_t geom, park, event, ring, cnt, dist, win, total;
+    size_t geom, cnt, dist, win, total;
     __host__ __device__ SmemLayout(int block, int n_geom, int window)
     {
-        size_t o = 0;
+        size_t o = sizeof(WarpMem) * (size_t)(block / 32);
         geom = o;
-        o += sizeof(DevGeom) * (size_t)n_geom;
-        o = (o + 15) & ~(size_t)15;
-        park = o;
-        o += sizeof(float4) * (size_t)(block / 32) * kParkWords * kPark;
-        event = o;
-        o += sizeof(float4) * (size_t)(block / 32) * (32 + kPark);
-        ring = o;
-        o += sizeof(Slot) * (size_t)(block / 32) * kRing;
+        o += n_geom > 1 ? sizeof(DevGeom) * (size_t)n_geom : 0;
         cnt = o;
-        o += sizeof(unsigned) * (size_t)(n_geom == 1 ? kCounterStride : 0);  // kAgg: one geometry
+        o += n_geom > 1 ? 0 : sizeof(unsigned) * kCounterStride;  // kAgg: one geometry
         dist = o;
         o += sizeof(float) * (size_t)n_geom;
         o = (o + 15) & ~(size_t)15;
@@ -357,6 +365,54 @@ struct SmemLayout {
         total = o;
     }
 };
+
+// Tallies of ended photons, one per lane of `lanes` (e: the place, relative to
+// the event in label mode; history index; fate and geometry): fate and
+// per-history counts with one reduction per distinct address of the warp, the
+// PRF pixel with one of its lane.
+template <bool kMulti, bool kRadial, bool kAgg>
+__device__ __forceinline__ void tally_ended(const TransportArgs &a, const DevGeom *s_geom, unsigned *s_cnt,
+                                            unsigned *s_win, const float4 &e, unsigned lanes)
+{
+    const int lane = threadIdx.x & 31;
+    const int code = __float_as_int(e.w), fate = code & 0xff, geom = kMulti ? code >> 8 : 0;
+    const int prim = __float_as_int(e.z);
+    const DevGeom &g = kMulti ? s_geom[geom] : a.g0;
+    const unsigned key = (unsigned)(geom * kCounterStride + fate);
+    unsigned peers = __match_any_sync(lanes, key);
+    if (lane == __ffs(peers) - 1) {
+        if (kAgg) atomicAdd(&s_cnt[key], (unsigned)__popc(peers));
+        else atomicAdd(&a.counters[key], (unsigned long long)__popc(peers));
+    }
+    const unsigned det = __ballot_sync(lanes, fate == kDetect);
+    if (fate != kDetect) return;
+    const bool counted = (unsigned)prim < (unsigned)a.n_prim;
+    peers = __match_any_sync(det, prim);
+    if (lane == __ffs(peers) - 1 && counted) atomicAdd(&a.per_primary[prim], __popc(peers));
+    if (kRadial) {
+        // quadratic edges: bin = floor(bins sqrt(r / r_max))
+        const float rr = sqrtf(e.x * e.x + e.y * e.y) * a.radial_inv_max;
+        const int b = rr < 1.0f ? min((int)(sqrtf(rr) * (float)a.radial_bins), a.radial_bins - 1) : a.radial_bins;
+        if (counted && b >= 0) atomicAdd(&a.radial[(long long)prim * (a.radial_bins + 1) + b], 1u);
+        return;
+    }
+    int ii, jj;
+    detection_pixel(g, e.x, e.y, ii, jj);
+    const bool in = ii >= 0 && jj >= 0 && ii < g.xdim && jj < g.ydim;
+    const unsigned seen = __ballot_sync(det, in);
+    if (!in) return;
+    // geometry by geometry where the warp's photons have several
+    peers = kMulti ? __match_any_sync(seen, geom) : seen;
+    if (lane == __ffs(peers) - 1) {
+        if (kAgg) atomicAdd(&s_cnt[kNumFates], (unsigned)__popc(peers));
+        else atomicAdd(&a.counters[geom * kCounterStride + kNumFates], (unsigned long long)__popc(peers));
+    }
+    const int win = a.window, wx = ii - a.win_x0, wy = jj - a.win_y0;
+    if (kAgg && win > 0 && (unsigned)wx < (unsigned)win && (unsigned)wy < (unsigned)win)
+        atomicAdd(&s_win[wx * win + wy], 1u);
+    else
+        atomicAdd(&a.prf[g.prf_offset + (long long)ii * g.ydim + jj], 1ull);
+}
 
 // Persistent transport.  Each warp keeps a ring of up to 32 chunk slots in
 // shared memory, filled with one coalesced load per lane; each lane runs one
@@ -385,12 +441,10 @@ template <bool kMulti, int kMaxThreads, int kMinBlocks, bool kRadial = false, bo
 __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(const __grid_constant__ TransportArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int nwarps = blockDim.x >> 5;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int win = a.window;
     const SmemLayout L(blockDim.x, a.n_geom, win);
     DevGeom *s_geom = reinterpret_cast<DevGeom *>(smem + L.geom);
-    Slot *s_ring = reinterpret_cast<Slot *>(smem + L.ring);
     unsigned int *s_cnt = reinterpret_cast<unsigned int *>(smem + L.cnt);
     float *s_dist = reinterpret_cast<float *>(smem + L.dist);
     unsigned int *s_win = reinterpret_cast<unsigned int *>(smem + L.win);
@@ -403,18 +457,19 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
     for (int i = threadIdx.x; i < win * win; i += blockDim.x) s_win[i] = 0;
     __syncthreads();
 
-    Slot *ring = s_ring + wid * kRing;
-    float4 *park = reinterpret_cast<float4 *>(smem + L.park) + wid * kParkWords * kPark;
-    float4 *event = reinterpret_cast<float4 *>(smem + L.event) + wid * (32 + kPark);
-    // never read past the chunk buffer, whatever the scan produced
-    const unsigned long long total_chunks = min(*a.n_chunks, (unsigned long long)a.chunk_capacity);
-    int ring_len = 0, slot = 0;
-    uint32_t used = 0;
-    bool exhausted = false, alive = false;
-    bool xretry = false;  // the lane's crosstalk normal is retried this round
+    WarpMem &m = reinterpret_cast<WarpMem *>(smem)[wid];
+    if (lane == 0) {
+        m.slot = m.len = 0;
+        m.used = 0;
+    }
+    bool exhausted = false;
+    // The lane: without a photon, running one, or holding one that waits; the
+    // fate of one that has ended and is not yet recorded; a crosstalk normal
+    // that is retried in the next step
+    enum { kEmpty, kRun, kWait };
+    int state = kEmpty, fate = kAlive;
+    bool xretry = false;
     int xtries = 0;
-    const int refill_min = max(a.refill, 1);
-    const int batch = min(max(a.fresnel_batch, 1), kPark);
     // Philox round keys and run counter, shared by the CTA
     __shared__ uint32_t s_rk[20];
     __shared__ uint32_t s_run;
@@ -423,68 +478,98 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
 
     Walker w;
     // The lane's tag: the shared-memory slot of its photon's event record
-    // (x, y, z, history index bits; read at a trapped restart, a detection and
-    // in label mode) in bits 0-7, the geometry above.  The warp's 64 slots are
-    // always a permutation over its lanes and parked photons.
+    // (x, y, z, history index bits; read at a trapped restart and at the
+    // photon's end) in bits 0-7, the geometry in bits 8-15, bit 16 a photon
+    // just reflected by the sensor.  The warp's 64 slots are always a
+    // permutation over its lanes and parked photons.
+    constexpr uint32_t kSlot = 0xffu, kReflected = 1u << 16;
     uint32_t tag = lane;
-    reinterpret_cast<uint32_t *>(&park[2 * kPark + lane])[3] = 32u + lane;
+    reinterpret_cast<uint32_t *>(&m.park[2 * kPark + lane])[3] = 32u + lane;
     // and the lane's path-length sum
     __shared__ float s_ldist[kMaxThreads];
     s_ldist[threadIdx.x] = 0.0f;
-    w.in_gap = false;
-    bool &parked = w.in_gap;
     // Waiting photons [0, n_wait) and ready ones [n_wait, n_wait + n_ready) of
     // the warp's parked photons (never more than kPark - 1 together: a photon
     // is added only while fewer than `batch` wait and none is ready).
     int n_wait = 0, n_ready = 0;
+    int n_ended = 0;  // ended photons not yet tallied
     __syncthreads();
     const RngKey key{s_rk, s_run};
 
     for (;;) {
-        // ---- which pass: a step of the lanes' photons, or the waiting ones
-        const unsigned live = __ballot_sync(kFull, alive);
-        const unsigned held = __ballot_sync(kFull, alive && parked);
-        const unsigned busy = live & ~held;
+        // ---- photons that ended: kept in shared memory (place, history,
+        // fate and geometry) until a warp's worth is tallied together.  One to
+        // two photons end in a step, and their pixel's two divisions and their
+        // reductions cost the warp as many instructions as 32 photons' do.
+        const unsigned over = __ballot_sync(kFull, fate != kAlive);
+        if (over) {
+            if (fate != kAlive) {
+                const float4 ev = m.event[tag & kSlot];
+                m.ended[n_ended + __popc(over & lanemask_lt())] =
+                    make_float4(kRadial ? w.px - ev.x : w.px, kRadial ? w.py - ev.y : w.py, ev.w,
+                                __int_as_float((int)(tag & 0xff00u) | fate));
+                if (kMulti) atomicAdd(&s_dist[(tag >> 8) & 0xffu], w.dist);
+                else s_ldist[threadIdx.x] += w.dist;  // lane-private: no atomic
+                fate = kAlive;
+            }
+            n_ended += __popc(over);
+        }
+        // ---- which pass: steps of the lanes' photons, or the waiting ones
+        unsigned run = __ballot_sync(kFull, state == kRun);
+        const unsigned held = __ballot_sync(kFull, state == kWait);
         const int n_held = __popc(held), waiting = n_wait + n_held;
-        const bool supply = n_ready > 0 || !exhausted;
-        bool flush = waiting >= (supply ? batch : min(batch, kTailBatch)) || (waiting > 0 && !busy && !supply);
-        int at = -1;  // the parked photon this lane exchanges its own with
+        bool supply = n_ready > 0 || !exhausted;
+        bool flush = waiting >= (supply ? a.fresnel_batch : min(a.fresnel_batch, kTailBatch)) ||
+                     (waiting > 0 && !run && !supply);
+        const bool finished = !run && waiting == 0 && !supply;
+        while (n_ended >= 32 || (finished && n_ended > 0)) {
+            const int n = min(n_ended, 32);
+            n_ended -= n;
+            __syncwarp();
+            if (lane < n)
+                tally_ended<kMulti, kRadial, kAgg>(a, s_geom, s_cnt, s_win, m.ended[n_ended + lane],
+                                                   kFull >> (32 - n));
+            __syncwarp();
+        }
+        if (finished) break;
+        int at = -1;     // the parked photon this lane exchanges its own with
+        int moved = 0;   // lanes that do
+        bool deal = false;
         if (flush) {
             // waiting photons into the lanes that hold none: first the empty
             // lanes (when no photon is ready for them), then lanes whose
             // photon can wait as a ready one
-            const unsigned none = n_ready == 0 ? ~live : 0u;
-            const unsigned other = busy & ~__ballot_sync(kFull, xretry);
-            const int n_none = __popc(none), take = min(n_wait, n_none + __popc(other));
+            const unsigned none = n_ready == 0 ? ~(run | held) : 0u;
+            const unsigned other = run & ~__ballot_sync(kFull, xretry);
+            const int n_none = __popc(none);
+            moved = min(n_wait, n_none + __popc(other));
             const bool empty = (none >> lane) & 1u;
             const int rank = empty ? __popc(none & lanemask_lt()) : n_none + __popc(other & lanemask_lt());
-            if ((((none | other) >> lane) & 1u) && rank < take) at = n_wait - 1 - rank;
-            n_wait -= take;
-            n_ready += take - min(take, n_none);
-            flush = n_held + take > 0;  // no lane can run one: step the others first
+            if ((((none | other) >> lane) & 1u) && rank < moved) at = n_wait - 1 - rank;
+            n_wait -= moved;
+            n_ready += moved - min(moved, n_none);
+            flush = n_held + moved > 0;  // no lane can run one: step the others first
         }
-        if (!flush && supply && (32 - __popc(busy) >= (exhausted ? 1 : refill_min) || !busy)) {
+        if (!flush && supply && (32 - __popc(run) >= (exhausted ? 1 : a.refill) || !run)) {
             // lanes with a waiting photon park it, for a ready one if there
-            // is one; empty lanes take ready ones
-            const int left = max(n_ready - n_held, 0), n_empty = 32 - __popc(live);
-            if ((held >> lane) & 1u) {
-                const int rank = __popc(held & lanemask_lt());
-                at = n_wait + rank;
-                alive = rank < n_ready;
-            } else if (!alive) {
-                const int rank = __popc(~live & lanemask_lt());
-                if (rank < left) {
-                    at = n_wait + n_ready - 1 - rank;
-                    alive = true;
-                }
+            // is one; empty lanes take ready ones; the rest get new photons
+            const unsigned none = ~(run | held);
+            const int left = max(n_ready - n_held, 0), taken = min(left, __popc(none));
+            if (state != kRun) {
+                const int rank = __popc((state == kWait ? held : none) & lanemask_lt());
+                const bool park = state == kWait, got = rank < (park ? n_ready : left);
+                if (park || got) at = park ? n_wait + rank : n_wait + n_ready - 1 - rank;
+                state = got ? kRun : kEmpty;
             }
+            moved = n_held + taken;
             n_wait += n_held;
-            n_ready = left - min(left, n_empty);
+            n_ready = left - taken;
+            deal = !exhausted;
         }
-        if (__ballot_sync(kFull, at >= 0)) {
+        if (moved) {
             __syncwarp();
             if (at >= 0) {
-                float4 *q = park + at, t = q[0];
+                float4 *q = m.park + at, t = q[0];
                 q[0] = make_float4(w.px, w.py, w.pz, w.dx);
                 w.px = t.x, w.py = t.y, w.pz = t.z, w.dx = t.w;
                 t = q[kPark];
@@ -498,16 +583,31 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                                            __uint_as_float(w.s3));
                 w.s0 = __float_as_uint(t.x), w.s1 = __float_as_uint(t.y);
                 w.s2 = __float_as_uint(t.z), w.s3 = __float_as_uint(t.w);
-                parked = flush;
-                if (flush) alive = true;
+                if (flush) state = kWait;
+                if (kGrid) w.in_gap = flush;
             }
             __syncwarp();
         }
+        if (flush) {
+            // ---- the waiting photons' pass
+            if (state == kWait) {
+                if constexpr (kGrid) {
+                    fate = w.grid_segment(a.g0);
+                    state = fate != kAlive ? kEmpty : w.in_gap ? kWait : kRun;
+                } else {
+                    fate = kMulti ? w.surface_wait(s_geom[(tag >> 8) & 0xffu]) : w.surface_wait(a.g0);
+                    state = fate != kAlive ? kEmpty : kRun;
+                }
+            }
+            continue;
+        }
         // ---- hand out photons to idle lanes
-        unsigned needy = __ballot_sync(kFull, !alive);
-        if (!flush && !exhausted && needy && (__popc(needy) >= refill_min || needy == kFull)) {
+        unsigned needy = __ballot_sync(kFull, state == kEmpty);
+        if (deal && needy && (__popc(needy) >= a.refill || needy == kFull)) {
+            int slot = m.slot, len = m.len;
+            uint32_t used = m.used;
             while (needy) {
-                if (slot >= ring_len) {
+                if (slot >= len) {
                     // A refill takes a share of what is left: 32 chunks while
                     // every warp can still take that many twice, then fewer,
                     // down to one, so that a small run spreads over the warps
@@ -524,9 +624,12 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                             atomicOr(a.status, kStatusAborted);
                         const unsigned long long head = *(const volatile unsigned long long *)a.queue_head;
                         if (!(*(const volatile int *)a.status & kStatusAborted)) {
-                            const unsigned long long left = total_chunks > head ? total_chunks - head : 0ull;
+                            const unsigned long long total = min(*a.n_chunks, (unsigned long long)a.chunk_capacity);
+                            const unsigned long long left = total > head ? total - head : 0ull;
                             take = (int)min(max(left >> a.pull_shift, 1ull), (unsigned long long)kRing);
                             base = atomicAdd(a.queue_head, (unsigned long long)take);
+                            // never read past the chunk buffer, whatever the scan produced
+                            if (base + take > total) take = base < total ? (int)(total - base) : 0;
                         }
                     }
                     take = __shfl_sync(kFull, take, 0);
@@ -536,7 +639,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                         break;
                     }
                     const unsigned long long idx = base + lane;
-                    const bool ok = lane < take && idx < total_chunks;
+                    const bool ok = lane < take;
                     __syncwarp();  // every lane is done reading the old ring
                     if (ok) {
                         const uint2 c = a.chunks[idx];
@@ -547,18 +650,14 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                         const int32_t n = a.ev_n[c.x];
                         s.count = (uint32_t)min(a.chunk, n - (int32_t)c.y);
                         s.geom = (kMulti && a.ev_geom) ? a.ev_geom[c.x] : 0;
-                        ring[lane] = s;
+                        m.ring[lane] = s;
                     }
-                    ring_len = __popc(__ballot_sync(kFull, ok));
+                    len = take;
                     __syncwarp();
                     slot = 0;
                     used = 0;
-                    if (ring_len == 0) {
-                        exhausted = true;
-                        break;
-                    }
                 }
-                const uint32_t count = ring[slot].count;
+                const uint32_t count = m.ring[slot].count;
                 if (used >= count) {
                     ++slot;
                     used = 0;
@@ -568,106 +667,64 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                 const unsigned rank = __popc(needy & lanemask_lt());
                 const bool mine = ((needy >> lane) & 1u) && rank < take;
                 if (mine) {
-                    const Slot &s = ring[slot];
+                    const Slot &s = m.ring[slot];
                     const uint32_t k = s.first + used + rank;
-                    tag = (tag & 0xffu) | (s.geom << 8);
-                    event[tag & 0xffu] = s.pos;
+                    tag = (tag & kSlot) | (s.geom << 8);
+                    m.event[tag & kSlot] = s.pos;
                     w.start(s.pos.x, s.pos.y, s.pos.z, k, (uint32_t)(a.event_base + s.event), k == 0, key);
-                    parked = false;
-                    if constexpr (kGrid) w.grid_place(a.g0);
-                    alive = true;
+                    state = kRun;
+                    if constexpr (kGrid) {
+                        w.grid_place(a.g0);
+                        state = w.in_gap ? kWait : kRun;
+                    }
                 }
                 needy &= ~__ballot_sync(kFull, mine);
                 used += take;
             }
-        }
-        if (__ballot_sync(kFull, alive) == 0) {
-            if (exhausted && n_wait + n_ready == 0) break;
-            continue;
-        }
-
-        // ---- one transport step per live lane, or the waiting photons' pass
-        int fate = kAlive;
-        const int geom = (int)(tag >> 8);
-        if constexpr (kGrid) {
-            // explicit column lattice: one segment per pass, of the photons in
-            // a column or of those in the gap
-            if (alive && parked == flush) fate = w.grid_segment(a.g0);
-        } else if (flush) {
-            if (alive && parked) {
-                fate = kMulti ? w.surface_fresnel(s_geom[geom]) : w.surface_fresnel(a.g0);
-                parked = false;
+            if (lane == 0) {
+                m.slot = slot;
+                m.len = len;
+                m.used = used;
             }
-        } else {
-            if (alive && !parked && !xretry) {
-                fate = kMulti ? w.step(s_geom[geom], event[tag & 0xffu]) : w.step(a.g0, event[tag & 0xffu]);
-                if (fate == kNeedsFresnel) {
-                    parked = true;
-                    fate = kAlive;
-                }
-            }
-            // crosstalk: one attempt at the next column's normal per round, so
-            // a rejected attempt is retried beside the other lanes' first ones
-            if (xretry || fate == kNeedsNormal) {
-                fate = kMulti ? w.crosstalk_normal(s_geom[geom], xtries) : w.crosstalk_normal(a.g0, xtries);
-                xretry = fate == kRetryNormal;
-                if (xretry) fate = kAlive;
-                else xtries = 0;
-            }
+            __syncwarp();
+            supply = n_ready > 0 || !exhausted;
         }
-
-        // ---- tallies of the photons that ended: one global reduction per lane
-        // (the default), or (kAgg) aggregated across the warp and privatised in
-        // shared memory
-        const unsigned ended = __ballot_sync(kFull, fate != kAlive);
-        if (ended) {
-            if (fate != kAlive) {
-                const unsigned key = (unsigned)(geom * kCounterStride + fate);
-                if (!kAgg) {
-                    atomicAdd(&a.counters[key], 1ull);
+        // ---- steps of the lanes' photons until enough lanes are idle to make
+        // the exchange worth its instructions; with nothing to fill them, until
+        // one more is
+        run = __ballot_sync(kFull, state == kRun);
+        if (!run) continue;
+        const int stay = supply ? 33 - a.refill : __popc(run);
+        do {
+            if (state == kRun) {
+                if constexpr (kGrid) {
+                    // explicit column lattice: one segment, of a photon in a column
+                    fate = w.grid_segment(a.g0);
+                    state = fate != kAlive ? kEmpty : w.in_gap ? kWait : kRun;
                 } else {
-                    const unsigned peers = __match_any_sync(ended, key);
-                    if (lane == __ffs(peers) - 1) atomicAdd(&s_cnt[key], (unsigned)__popc(peers));
-                }
-                if (kMulti) atomicAdd(&s_dist[geom], w.dist);
-                else s_ldist[threadIdx.x] += w.dist;  // lane-private: no atomic
-                alive = false;
-                parked = false;
-            }
-            const unsigned det = __ballot_sync(kFull, fate == kDetect);
-            if (fate == kDetect) {
-                const float4 ev = event[tag & 0xffu];
-                const int prim = __float_as_int(ev.w);
-                if (!kAgg) {
-                    if ((unsigned)prim < (unsigned)a.n_prim) atomicAdd(&a.per_primary[prim], 1);
-                } else {
-                    const unsigned peers = __match_any_sync(det, prim);
-                    if (lane == __ffs(peers) - 1 && (unsigned)prim < (unsigned)a.n_prim)
-                        atomicAdd(&a.per_primary[prim], __popc(peers));
-                }
-                const int xdim = kMulti ? s_geom[geom].xdim : a.g0.xdim;
-                const int ydim = kMulti ? s_geom[geom].ydim : a.g0.ydim;
-                if (kRadial) {
-                    const float rx = w.px - ev.x, ry = w.py - ev.y;
-                    // quadratic edges: bin = floor(bins sqrt(r / r_max))
-                    const float rr = sqrtf(rx * rx + ry * ry) * a.radial_inv_max;
-                    const int b = rr < 1.0f ? min((int)(sqrtf(rr) * (float)a.radial_bins), a.radial_bins - 1)
-                                            : a.radial_bins;
-                    if ((unsigned)prim < (unsigned)a.n_prim && b >= 0)
-                        atomicAdd(&a.radial[(long long)prim * (a.radial_bins + 1) + b], 1u);
-                } else if (w.ii >= 0 && w.jj >= 0 && w.ii < xdim && w.jj < ydim) {
-                    if (!kAgg) atomicAdd(&a.counters[geom * kCounterStride + kNumFates], 1ull);
-                    else atomicAdd(&s_cnt[geom * kCounterStride + kNumFates], 1u);
-                    const int wx = w.ii - a.win_x0, wy = w.jj - a.win_y0;
-                    if (kAgg && geom == 0 && win > 0 && (unsigned)wx < (unsigned)win && (unsigned)wy < (unsigned)win) {
-                        atomicAdd(&s_win[wx * win + wy], 1u);
-                    } else {
-                        const long long off = kMulti ? s_geom[geom].prf_offset : a.g0.prf_offset;
-                        atomicAdd(&a.prf[off + (long long)w.ii * ydim + w.jj], 1ull);
+                    int f = kNeedsNormal;
+                    if (!xretry) {
+                        bool reflected = (tag & kReflected) != 0u;
+                        f = kMulti ? w.step(s_geom[(tag >> 8) & 0xffu], m.event[tag & kSlot], reflected)
+                                   : w.step(a.g0, m.event[tag & kSlot], reflected);
+                        tag = (tag & ~kReflected) | (reflected ? kReflected : 0u);
                     }
+                    // crosstalk: one attempt at the next column's normal per
+                    // step, so a rejected attempt is retried beside the other
+                    // lanes' first ones
+                    if (f == kNeedsNormal) {
+                        f = kMulti ? w.crosstalk_normal(s_geom[(tag >> 8) & 0xffu], xtries)
+                                   : w.crosstalk_normal(a.g0, xtries);
+                        xretry = f == kRetryNormal;
+                        xtries = xretry ? xtries : 0;
+                    }
+                    const bool flies = f == kAlive || f == kRetryNormal;
+                    state = flies ? kRun : f == kNeedsFresnel ? kWait : kEmpty;
+                    fate = flies || f == kNeedsFresnel ? kAlive : f;
                 }
             }
-        }
+            run = __ballot_sync(kFull, state == kRun);
+        } while (__popc(run) >= stay);
     }
 
     // ---- flush the CTA's private tallies
@@ -883,6 +940,8 @@ cudaError_t launch_transport(cudaStream_t s, const TransportConfig &cfg, int sm_
     // 22.9 ms, 28.5 ms with two)
     const int per_sm_label = !multi && cfg.ctas_per_sm >= 4 ? 4 : 3;
     const unsigned grid = (unsigned)(sm_count * (a.radial ? per_sm_label : cfg.ctas_per_sm));
+    a.refill = std::min(std::max(a.refill, 1), 32);
+    a.fresnel_batch = std::min(std::max(a.fresnel_batch, 1), kPark);
     // a refill takes 1 / 2^pull_shift of the chunks left: at most half of a
     // warp's even share
     for (a.pull_shift = 1; (1ll << a.pull_shift) < 2ll * grid * (cfg.block / 32); ++a.pull_shift) {
