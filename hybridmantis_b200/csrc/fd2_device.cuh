@@ -64,7 +64,8 @@ __device__ __forceinline__ uint4 philox4x32_10_rk(uint4 c, const uint32_t *rk)
 // (1 + k 2^-23) - (1 - 2^-24), exact in float.
 __device__ __forceinline__ float u01(uint32_t r)
 {
-    return __uint_as_float(0x3F800000u | (r >> 9)) - 0.99999994039535522461f;
+    // one funnel shift: 0x7F above the top 23 bits is 0x3F800000 | (r >> 9)
+    return __uint_as_float(__funnelshift_r(r, 0x7Fu, 9)) - 0.99999994039535522461f;
 }
 
 // Internal step result: the photon waits at a column wall for the Fresnel
@@ -73,6 +74,7 @@ constexpr int kNeedsFresnel = 100;
 // Internal step results of the crosstalk path: the photon crosses into the
 // adjacent column and needs that column's normal (crosstalk_normal), or its
 // attempt was rejected and is retried in the next round.
+constexpr int kNeedsHop = 103;  // the photon has left the column and hops to the next
 constexpr int kNeedsNormal = 101;
 constexpr int kRetryNormal = 102;
 
@@ -154,7 +156,7 @@ struct Walker {
     float dx, dy, dz;   // direction
     float nx, ny, nz;   // current surface normal
     float xc, yc;       // centre of the current column
-    float dist;         // path length
+    float dist;         // path length of the lane's photons since it was last summed
     float budget;       // absorption lengths left before bulk absorption
     uint32_t rebound;   // boundary interactions
     // The photon's random stream: xoshiro128+ state (never all zero; a
@@ -191,7 +193,6 @@ struct Walker {
         px = ex; py = ey; pz = ez;
         xc = ex; yc = ey;
         nx = 0.0f; ny = 0.0f; nz = 0.0f;
-        dist = 0.0f;
         rebound = 0;
         emit(first);
         budget = -__logf(u());  // Exp(1)
@@ -536,25 +537,33 @@ struct Walker {
         return kTheta1;
     }
 
-    // What a waiting photon waits for: the top reflector or the wall.
-    template <class G>
-    __device__ __forceinline__ int surface_wait(const G &g)
-    {
-        if (at_top(g)) return top_reflector(g);
-        return surface_fresnel(g);
-    }
+    // Retry counts of a wall interaction, kept in a word of the photon while
+    // it waits for a hop: tries at an incidence angle and at a next normal (at
+    // most 100 each), perturbations (3) and smooth attempts (25).
+    static constexpr int kTheta = 9, kPerturb = 16, kSmooth = 18, kNormalTry = 23;
+    static constexpr uint32_t kCounts = (0x7fu << kTheta) | (3u << kPerturb) | (0x1fu << kSmooth) | (0x7fu << kNormalTry);
 
-    // Second part: Fresnel reflection / refraction on the rough wall, with
-    // hops between columns until the photon is back inside a column.
+    // What a waiting photon waits for: the top reflector, or Fresnel reflection
+    // / refraction on the rough wall (boundary_analysis, second part).  A
+    // photon that refracts out of its column waits again, for its hop
+    // (kNeedsHop); with `hop` it continues there, until it is back inside a
+    // column or meets the next column's wall from outside and hops again.  One
+    // in five wall interactions leaves the column: run to their end beside the
+    // others, the hops took half of the pass at 2 to 3 lanes.  `counts` keeps
+    // the retry counts between the two.
     template <class G>
-    __device__ __forceinline__ int surface_fresnel(const G &g)
+    __device__ __forceinline__ int surface_wait(const G &g, bool hop, uint32_t &counts)
     {
-        bool outside = false;
-        int tries_theta = 0, tries_normal = 0, reperturbs = 0, smooth = 0;
+        if (!hop && at_top(g)) return top_reflector(g);
+        if (hop && ++rebound > kMaxBoundaryCalls) return kCapped;  // bounds the passes of one interaction
+        bool outside = hop;
+        int tries_theta = (counts >> kTheta) & 0x7f, tries_normal = (counts >> kNormalTry) & 0x7f;
+        int reperturbs = (counts >> kPerturb) & 3, smooth = (counts >> kSmooth) & 0x1f;
+        counts &= ~kCounts;
         float pr = __int_as_float(0x7fc00000);  // 0/0 until a rule sets it
         float st = 0.0f, ct = 1.0f;            // sin, cos of the last refraction angle
         float kx = 0, ky = 0, kz = 0, kdx = 0, kdy = 0, kdz = 0;
-        enum { kLeave, kNewSurface, kRestore, kIncidence } stage = kNewSurface;
+        enum { kLeave, kNewSurface, kRestore, kIncidence } stage = hop ? kLeave : kNewSurface;
         int fate = kAlive;
         for (int loop = 0; loop < kMaxSurfaceLoops; ++loop) {
             if (stage == kNewSurface) {
@@ -595,6 +604,13 @@ struct Walker {
                     }
                     if (tries_theta < 100) {
                         ++tries_theta;
+                        if (!outside) {
+                            // from within the column nothing else is carried
+                            // over: tried again in the next pass
+                            counts |= (uint32_t)tries_theta << kTheta | (uint32_t)reperturbs << kPerturb |
+                                      (uint32_t)smooth << kSmooth;
+                            return kNeedsFresnel;
+                        }
                         stage = kNewSurface;
                         continue;
                     }
@@ -650,6 +666,13 @@ struct Walker {
                     renorm(dx, dy, dz);
                     if (outside) break;  // entered the next column: done
                     stage = kLeave;
+                }
+                // the low-contrast rule looks back at the last refraction:
+                // such photons go on at once
+                if (!g.stale_out) {
+                    counts |= (uint32_t)tries_theta << kTheta | (uint32_t)tries_normal << kNormalTry |
+                              (uint32_t)reperturbs << kPerturb | (uint32_t)smooth << kSmooth;
+                    return kNeedsHop;
                 }
             }
             // kLeave: hop between columns
@@ -963,7 +986,7 @@ struct Walker {
     }
 
     // One transport step (the body of the reference's step function algo):
-    // flight, sensor, trapped-photon restart (from `event`, the x, y, z of
+    // flight, sensor, trapped-photon restart (from `*event`, the x, y, z of
     // the photon's event), or a surface interaction up to the part that waits.
     // Returns the photon's fate, kAlive while it is in flight, kNeedsNormal
     // (run crosstalk_normal next) or kNeedsFresnel (surface_wait next).  A
@@ -971,7 +994,7 @@ struct Walker {
     // beside the warp's others; `reflected` then keeps it from meeting the
     // sensor again where it stands.
     template <class G>
-    __device__ __forceinline__ int step(const G &g, const float4 &event, bool &reflected)
+    __device__ __forceinline__ int step(const G &g, const float4 *event, bool &reflected)
     {
         const int f = flight(g);
         if (f != kAlive) return f;
@@ -988,7 +1011,8 @@ struct Walker {
         if (fabsf(dz) < kEps) {
             // trapped travelling horizontally: restart from the event position,
             // keeping the current column (the reference does not reset it)
-            px = event.x; py = event.y; pz = event.z;
+            const float4 e = *event;
+            px = e.x; py = e.y; pz = e.z;
             emit(false);
             return kAlive;
         }

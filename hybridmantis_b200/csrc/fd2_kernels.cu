@@ -323,22 +323,23 @@ struct Slot {
     uint32_t geom;
 };
 constexpr int kRing = 32;
-// Photons a warp holds beside its lanes' (in shared memory), and the 16-byte
-// words of one: position, direction, column centre, path length, absorption
-// budget, boundary count, tag (event slot and geometry), random state.
+// Photons a warp holds beside its lanes' (in shared memory), of each kind, and
+// the 16-byte words of one: position, direction, column centre, absorption
+// budget, boundary count, tag, event, random state.
 constexpr int kPark = 32;
 constexpr int kParkWords = 4;
+constexpr int kParkKind = kPark * kParkWords;  // words from one kind's photons to the other's
 // Ended photons a warp holds: fewer than 32 wait, and up to 32 end in a pass.
 constexpr int kEnded = 64;
 // Waiting photons that start a pass once the queue and the ready photons are
 // used up: waiting for more would only idle lanes then.
 constexpr int kTailBatch = 8;
 
-// A warp's shared memory: its parked and ended photons, its photons' event
-// records, and its ring of chunks.
+// A warp's shared memory: its parked photons (those that wait at a wall, and
+// those that wait for a hop), its ended photons and its ring of chunks.
 struct WarpMem {
-    float4 park[kParkWords * kPark];
-    float4 event[32 + kPark];
+    float4 park[2 * kParkKind];
+    float park_dist[2 * kPark];  // path lengths, where they are summed by geometry
     float4 ended[kEnded];
     Slot ring[kRing];
     int slot, len;   // the ring's current slot and its filled slots
@@ -366,8 +367,8 @@ struct SmemLayout {
     }
 };
 
-// Tallies of ended photons, one per lane of `lanes` (e: the place, relative to
-// the event in label mode; history index; fate and geometry): fate and
+// Tallies of ended photons, one per lane of `lanes` (e: the place; event index;
+// fate and geometry): fate and
 // per-history counts with one reduction per distinct address of the warp, the
 // PRF pixel with one of its lane.
 template <bool kMulti, bool kRadial, bool kAgg>
@@ -376,7 +377,8 @@ __device__ __forceinline__ void tally_ended(const TransportArgs &a, const DevGeo
 {
     const int lane = threadIdx.x & 31;
     const int code = __float_as_int(e.w), fate = code & 0xff, geom = kMulti ? code >> 8 : 0;
-    const int prim = __float_as_int(e.z);
+    const float4 ev = a.ev_pos[__float_as_uint(e.z)];
+    const int prim = __float_as_int(ev.w);
     const DevGeom &g = kMulti ? s_geom[geom] : a.g0;
     const unsigned key = (unsigned)(geom * kCounterStride + fate);
     unsigned peers = __match_any_sync(lanes, key);
@@ -391,7 +393,8 @@ __device__ __forceinline__ void tally_ended(const TransportArgs &a, const DevGeo
     if (lane == __ffs(peers) - 1 && counted) atomicAdd(&a.per_primary[prim], __popc(peers));
     if (kRadial) {
         // quadratic edges: bin = floor(bins sqrt(r / r_max))
-        const float rr = sqrtf(e.x * e.x + e.y * e.y) * a.radial_inv_max;
+        const float rx = e.x - ev.x, ry = e.y - ev.y;
+        const float rr = sqrtf(rx * rx + ry * ry) * a.radial_inv_max;
         const int b = rr < 1.0f ? min((int)(sqrtf(rr) * (float)a.radial_bins), a.radial_bins - 1) : a.radial_bins;
         if (counted && b >= 0) atomicAdd(&a.radial[(long long)prim * (a.radial_bins + 1) + b], 1u);
         return;
@@ -420,19 +423,21 @@ __device__ __forceinline__ void tally_ended(const TransportArgs &a, const DevGeo
 // enough lanes of the warp are) idle, so lanes never wait for the longest walk
 // in the warp.  What bounds the kernel is instruction issue, so what counts is
 // how many lanes of a warp share each instruction.  Photons that wait for the
-// rarer, longer part of the walk (the Fresnel part at a wall; with a column
-// lattice the flight through the gap) leave their lane for the warp's shared
-// memory (up to 32, 64 bytes each) and the lane goes on with another photon;
-// once `fresnel_batch` wait, they are exchanged into the lanes and that part
-// runs for all of them, the photons they displaced waiting as ready ones.
-// Photons that waited in their lane for 8 others had the Fresnel part run at
-// 9.1 lanes for a third of the warps' time and steps at 25 lanes; 20,000
-// config-1 x-rays 59.2 -> 51.6 ms, with a square / hexagonal lattice 109 / 151
-// -> 77 / 97 ms (one B200).  Tallies: by default every ended photon
-// adds to the global fates, per-primary counts and PRF with one L2
-// reduction of its lane; with kAgg (tally_mode 1) they are aggregated across
-// the warp before touching memory and the PRF core of geometry 0 is tallied
-// in a shared-memory window (identical tallies, slower on a B200).  kMulti: the
+// rarer, longer parts of the walk (the Fresnel part at a wall, the hop between
+// columns after it; with a column lattice the flight through the gap) leave
+// their lane for the warp's shared memory (up to 32 of either kind, 64 bytes
+// each) and the lane goes on with another photon; once `fresnel_batch` wait,
+// they are exchanged into the lanes and that part runs for all of them, the
+// photons they displaced waiting as ready ones.  Photons that waited in their
+// lane for 8 others had the Fresnel part run at 9.1 lanes for a third of the
+// warps' time, its hops at 2 to 3, and steps at 25.  20,000 config-1 x-rays
+// (one B200): 59.2 ms before, 51.6 with the wall's photons parked, 46.0 with
+// ended photons tallied together and steps looped, 44.2 with the hops parked;
+// square / hexagonal lattice 109 / 151 -> 71 / 91 ms.  Per photon 1,252 -> 995
+// warp instructions, issue slots 87 % busy, 22.7 of 32 lanes.  Tallies:
+// ended photons are tallied 32 at a time (tally_ended) with L2 reductions;
+// with kAgg (tally_mode 1) the fates and the PRF core of geometry 0 are
+// tallied in shared memory first (identical tallies).  kMulti: the
 // geometry of each photon comes from the table in shared memory; otherwise
 // the single geometry is read from the kernel parameters.  kRadial (label
 // mode): a detected photon is binned by its distance from its event into
@@ -463,10 +468,11 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
         m.used = 0;
     }
     bool exhausted = false;
-    // The lane: without a photon, running one, or holding one that waits; the
+    // The lane: without a photon, running one, or holding one that waits (at a
+    // wall or for a hop); the
     // fate of one that has ended and is not yet recorded; a crosstalk normal
     // that is retried in the next step
-    enum { kEmpty, kRun, kWait };
+    enum { kEmpty, kRun, kWait, kHop };
     int state = kEmpty, fate = kAlive;
     bool xretry = false;
     int xtries = 0;
@@ -477,21 +483,20 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
     if (threadIdx.x == 0) s_run = *a.run_tag;
 
     Walker w;
-    // The lane's tag: the shared-memory slot of its photon's event record
-    // (x, y, z, history index bits; read at a trapped restart and at the
-    // photon's end) in bits 0-7, the geometry in bits 8-15, bit 16 a photon
-    // just reflected by the sensor.  The warp's 64 slots are always a
-    // permutation over its lanes and parked photons.
-    constexpr uint32_t kSlot = 0xffu, kReflected = 1u << 16;
-    uint32_t tag = lane;
-    reinterpret_cast<uint32_t *>(&m.park[2 * kPark + lane])[3] = 32u + lane;
-    // and the lane's path-length sum
+    // The photon's event, and its tag: the geometry in bits 0-7, bit 8 a photon
+    // just reflected by the sensor, above it the retry counts of a wall
+    // interaction (Walker::kCounts).
+    constexpr uint32_t kGeomBits = 0xffu, kReflected = 1u << 8;
+    uint32_t tag = 0, event = 0;
+    w.dist = 0.0f;
+    // the lane's path-length sum
     __shared__ float s_ldist[kMaxThreads];
     s_ldist[threadIdx.x] = 0.0f;
-    // Waiting photons [0, n_wait) and ready ones [n_wait, n_wait + n_ready) of
-    // the warp's parked photons (never more than kPark - 1 together: a photon
-    // is added only while fewer than `batch` wait and none is ready).
-    int n_wait = 0, n_ready = 0;
+    // Of either kind of parked photons, [0, n_wait) wait and
+    // [n_wait, n_wait + n_ready) are ready (never more than kPark - 1
+    // together: a photon is added only while fewer than `batch` wait and none
+    // is ready).
+    int n_wait = 0, n_ready = 0, n_hop = 0, n_hready = 0;
     int n_ended = 0;  // ended photons not yet tallied
     __syncthreads();
     const RngKey key{s_rk, s_run};
@@ -504,24 +509,26 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
         const unsigned over = __ballot_sync(kFull, fate != kAlive);
         if (over) {
             if (fate != kAlive) {
-                const float4 ev = m.event[tag & kSlot];
                 m.ended[n_ended + __popc(over & lanemask_lt())] =
-                    make_float4(kRadial ? w.px - ev.x : w.px, kRadial ? w.py - ev.y : w.py, ev.w,
-                                __int_as_float((int)(tag & 0xff00u) | fate));
-                if (kMulti) atomicAdd(&s_dist[(tag >> 8) & 0xffu], w.dist);
-                else s_ldist[threadIdx.x] += w.dist;  // lane-private: no atomic
+                    make_float4(w.px, w.py, __uint_as_float(event), __int_as_float((int)(tag & kGeomBits) << 8 | fate));
+                if (kMulti) {
+                    atomicAdd(&s_dist[tag & kGeomBits], w.dist);
+                } else {
+                    s_ldist[threadIdx.x] += w.dist;  // lane-private: no atomic
+                    w.dist = 0.0f;
+                }
                 fate = kAlive;
             }
             n_ended += __popc(over);
         }
         // ---- which pass: steps of the lanes' photons, or the waiting ones
-        unsigned run = __ballot_sync(kFull, state == kRun);
-        const unsigned held = __ballot_sync(kFull, state == kWait);
-        const int n_held = __popc(held), waiting = n_wait + n_held;
-        bool supply = n_ready > 0 || !exhausted;
-        bool flush = waiting >= (supply ? a.fresnel_batch : min(a.fresnel_batch, kTailBatch)) ||
-                     (waiting > 0 && !run && !supply);
-        const bool finished = !run && waiting == 0 && !supply;
+        const unsigned odd = __ballot_sync(kFull, (state & 1) != 0), upper = __ballot_sync(kFull, state >= kWait);
+        unsigned run = odd & ~upper;
+        const unsigned held = upper & ~odd, hops = kGrid ? 0u : upper & odd, none = ~(upper | odd);
+        const int n_held = __popc(held), n_hops = __popc(hops);
+        const int waiting = n_wait + n_held, hopping = n_hop + n_hops;
+        bool supply = n_ready + n_hready > 0 || !exhausted;
+        const bool finished = !run && waiting + hopping == 0 && !supply;
         while (n_ended >= 32 || (finished && n_ended > 0)) {
             const int n = min(n_ended, 32);
             n_ended -= n;
@@ -534,36 +541,61 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
         if (finished) break;
         int at = -1;     // the parked photon this lane exchanges its own with
         int moved = 0;   // lanes that do
-        bool deal = false;
-        if (flush) {
-            // waiting photons into the lanes that hold none: first the empty
-            // lanes (when no photon is ready for them), then lanes whose
-            // photon can wait as a ready one
-            const unsigned none = n_ready == 0 ? ~(run | held) : 0u;
+        bool flush = false, hop = false, deal = false;
+        const int batch = supply ? a.fresnel_batch : min(a.fresnel_batch, kTailBatch);
+        if (waiting >= batch || hopping >= batch || (!run && !supply)) {
+            // waiting photons into the lanes that hold none of their kind:
+            // first the empty lanes (when no photon is ready among them), then
+            // lanes whose photon can wait as a ready one.  Without a lane that
+            // can run one, the others step first.
             const unsigned other = run & ~__ballot_sync(kFull, xretry);
-            const int n_none = __popc(none);
-            moved = min(n_wait, n_none + __popc(other));
-            const bool empty = (none >> lane) & 1u;
-            const int rank = empty ? __popc(none & lanemask_lt()) : n_none + __popc(other & lanemask_lt());
-            if ((((none | other) >> lane) & 1u) && rank < moved) at = n_wait - 1 - rank;
-            n_wait -= moved;
-            n_ready += moved - min(moved, n_none);
-            flush = n_held + moved > 0;  // no lane can run one: step the others first
+            const int n_none = __popc(none), n_other = __popc(other);
+            hop = !kGrid && (hopping >= batch || waiting == 0) &&
+                  (n_hops > 0 || n_other > 0 || (n_hready == 0 && n_none > 0));
+            flush = hop || ((waiting >= batch || (!run && !supply)) &&
+                            (n_held > 0 || n_other > 0 || (n_ready == 0 && n_none > 0)));
+            if (flush) {
+                const int nw = hop ? n_hop : n_wait, nr = hop ? n_hready : n_ready;
+                const unsigned take = nr == 0 ? none : 0u;
+                const int n_take = __popc(take);
+                moved = min(nw, n_take + n_other);
+                const bool empty = (take >> lane) & 1u;
+                const int rank = empty ? __popc(take & lanemask_lt()) : n_take + __popc(other & lanemask_lt());
+                if ((((take | other) >> lane) & 1u) && rank < moved) at = (hop ? kParkKind : 0) + nw - 1 - rank;
+                const int ready = nr + moved - min(moved, n_take);
+                (hop ? n_hop : n_wait) = nw - moved;
+                (hop ? n_hready : n_ready) = ready;
+            }
         }
         if (!flush && supply && (32 - __popc(run) >= (exhausted ? 1 : a.refill) || !run)) {
-            // lanes with a waiting photon park it, for a ready one if there
-            // is one; empty lanes take ready ones; the rest get new photons
-            const unsigned none = ~(run | held);
-            const int left = max(n_ready - n_held, 0), taken = min(left, __popc(none));
+            // lanes with a waiting photon park it, for a ready one of its kind
+            // if there is one; empty lanes take ready ones; the rest get new
+            // photons
+            const int n_none = __popc(none);
+            const int left = max(n_ready - n_held, 0), hleft = max(n_hready - n_hops, 0);
+            const int taken = min(left, n_none), htaken = min(hleft, n_none - taken);
             if (state != kRun) {
-                const int rank = __popc((state == kWait ? held : none) & lanemask_lt());
-                const bool park = state == kWait, got = rank < (park ? n_ready : left);
-                if (park || got) at = park ? n_wait + rank : n_wait + n_ready - 1 - rank;
+                const unsigned same = state == kWait ? held : !kGrid && state == kHop ? hops : none;
+                const int rank = __popc(same & lanemask_lt());
+                bool got;
+                if (state == kWait) {
+                    at = n_wait + rank;
+                    got = rank < n_ready;
+                } else if (!kGrid && state == kHop) {
+                    at = kParkKind + n_hop + rank;
+                    got = rank < n_hready;
+                } else {
+                    got = rank < taken + htaken;
+                    if (got) at = rank < taken ? n_wait + n_ready - 1 - rank
+                                               : kParkKind + n_hop + n_hready - 1 - (rank - taken);
+                }
                 state = got ? kRun : kEmpty;
             }
-            moved = n_held + taken;
+            moved = n_held + n_hops + taken + htaken;
             n_wait += n_held;
+            n_hop += n_hops;
             n_ready = left - taken;
+            n_hready = hleft - htaken;
             deal = !exhausted;
         }
         if (moved) {
@@ -576,27 +608,38 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                 q[kPark] = make_float4(w.dy, w.dz, w.xc, w.yc);
                 w.dy = t.x, w.dz = t.y, w.xc = t.z, w.yc = t.w;
                 t = q[2 * kPark];
-                q[2 * kPark] = make_float4(w.dist, w.budget, __uint_as_float(w.rebound), __uint_as_float(tag));
-                w.dist = t.x, w.budget = t.y, w.rebound = __float_as_uint(t.z), tag = __float_as_uint(t.w);
+                q[2 * kPark] = make_float4(w.budget, __uint_as_float(w.rebound), __uint_as_float(tag),
+                                           __uint_as_float(event));
+                if (kMulti) {
+                    float &pd = m.park_dist[at < kParkKind ? at : at - kParkKind + kPark];
+                    const float d = pd;
+                    pd = w.dist;
+                    w.dist = d;
+                }
+                w.budget = t.x, w.rebound = __float_as_uint(t.y), tag = __float_as_uint(t.z);
+                event = __float_as_uint(t.w);
                 t = q[3 * kPark];
                 q[3 * kPark] = make_float4(__uint_as_float(w.s0), __uint_as_float(w.s1), __uint_as_float(w.s2),
                                            __uint_as_float(w.s3));
                 w.s0 = __float_as_uint(t.x), w.s1 = __float_as_uint(t.y);
                 w.s2 = __float_as_uint(t.z), w.s3 = __float_as_uint(t.w);
-                if (flush) state = kWait;
+                if (flush) state = !kGrid && hop ? kHop : kWait;
                 if (kGrid) w.in_gap = flush;
             }
             __syncwarp();
         }
         if (flush) {
             // ---- the waiting photons' pass
-            if (state == kWait) {
+            if (state == (!kGrid && hop ? kHop : kWait)) {
                 if constexpr (kGrid) {
                     fate = w.grid_segment(a.g0);
                     state = fate != kAlive ? kEmpty : w.in_gap ? kWait : kRun;
                 } else {
-                    fate = kMulti ? w.surface_wait(s_geom[(tag >> 8) & 0xffu]) : w.surface_wait(a.g0);
-                    state = fate != kAlive ? kEmpty : kRun;
+                    const int f = kMulti ? w.surface_wait(s_geom[tag & kGeomBits], hop, tag)
+                                         : w.surface_wait(a.g0, hop, tag);
+                    const bool waits = f == kNeedsHop || f == kNeedsFresnel;
+                    state = f == kAlive ? kRun : f == kNeedsHop ? kHop : waits ? kWait : kEmpty;
+                    fate = waits ? kAlive : f;
                 }
             }
             continue;
@@ -669,8 +712,9 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                 if (mine) {
                     const Slot &s = m.ring[slot];
                     const uint32_t k = s.first + used + rank;
-                    tag = (tag & kSlot) | (s.geom << 8);
-                    m.event[tag & kSlot] = s.pos;
+                    tag = s.geom;
+                    event = s.event;
+                    if (kMulti) w.dist = 0.0f;
                     w.start(s.pos.x, s.pos.y, s.pos.z, k, (uint32_t)(a.event_base + s.event), k == 0, key);
                     state = kRun;
                     if constexpr (kGrid) {
@@ -705,15 +749,15 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                     int f = kNeedsNormal;
                     if (!xretry) {
                         bool reflected = (tag & kReflected) != 0u;
-                        f = kMulti ? w.step(s_geom[(tag >> 8) & 0xffu], m.event[tag & kSlot], reflected)
-                                   : w.step(a.g0, m.event[tag & kSlot], reflected);
+                        f = kMulti ? w.step(s_geom[tag & kGeomBits], a.ev_pos + event, reflected)
+                                   : w.step(a.g0, a.ev_pos + event, reflected);
                         tag = (tag & ~kReflected) | (reflected ? kReflected : 0u);
                     }
                     // crosstalk: one attempt at the next column's normal per
                     // step, so a rejected attempt is retried beside the other
                     // lanes' first ones
                     if (f == kNeedsNormal) {
-                        f = kMulti ? w.crosstalk_normal(s_geom[(tag >> 8) & 0xffu], xtries)
+                        f = kMulti ? w.crosstalk_normal(s_geom[tag & kGeomBits], xtries)
                                    : w.crosstalk_normal(a.g0, xtries);
                         xretry = f == kRetryNormal;
                         xtries = xretry ? xtries : 0;
@@ -734,7 +778,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
             if (s_cnt[i]) atomicAdd(&a.counters[i], (unsigned long long)s_cnt[i]);
     if (!kMulti) {
         // the lanes' path-length sums: summed per warp in double, then added to the CTA's
-        double d = (double)s_ldist[threadIdx.x];
+        double d = (double)s_ldist[threadIdx.x] + (double)w.dist;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(kFull, d, o);
         if (lane == 0 && d != 0.0) atomicAdd(&a.distance[0], d);
