@@ -72,12 +72,18 @@ struct fd2_sg {
     unsigned long long *d_step = nullptr;
     double *d_acc = nullptr;
     float *d_lr = nullptr;  // Adam step size (read by the captured step)
-    float *ws = nullptr;  // split-K partials
+    float *ws = nullptr;  // split-K partials, ws_floats for each layer
     int64_t ws_floats = 0;
+    // the layers' weight gradients: a stream each, forked off the step's stream
+    // and joined at the end of the backward pass
+    cudaStream_t side[4] = {};
+    cudaEvent_t ev_main[4] = {}, ev_side[4] = {};
     // tcgen05 backward: transposed BF16 weights (W2^T, W3^T: H x H; W4^T:
     // H x 64) and batch-major operands transposed to [columns][rows padded
-    // to 256] (tA: the incoming gradient, tB: the layer's input)
+    // to 256] (tA: the incoming gradient, tB: the layer's input; t_stride
+    // elements for each layer)
     __nv_bfloat16 *pbT = nullptr, *tA = nullptr, *tB = nullptr;
+    int64_t t_stride = 0;
 
     // activations for up to cap_rows rows
     int cap_rows = 0;

@@ -57,87 +57,129 @@ __device__ __forceinline__ uint4 philox10(uint4 c, uint32_t k0, uint32_t k1)
     return c;
 }
 
-// Loss of one point and (optionally) d loss / d out.  y: normalised radial
-// label over bins + 1 categories (null = no radial term).  The radial term
-// is the cross-entropy -sum_j y_j log q_j of the ring mixture's category
-// probabilities q_j = sum_k w_k M_k(e_j, e_j+1) / S_k (fd2_sg_mix.cuh).
-__device__ float point_loss(const float *o, float t, const float *y, int bins, float r_max, float lambda,
-                            float *dout, float *det_loss, float *rad_loss)
+// One point's loss and the gradients of its outputs, in a warp: lanes 0..7
+// hold the gradients of component lane's weight, radius and width outputs.
+struct PointLoss {
+    float det, rad, total;
+    float gz, ga, gom, gls;
+};
+
+constexpr int kLossWarps = 4;
+constexpr int kSums = 3 * kComponents + 1;  // sums over the categories: A1, Amu, Asd of the components, and the loss
+
+// Loss of one point and its gradients, computed by the 32 lanes of a warp
+// together.  o: the network's outputs; y: normalised radial label over bins + 1
+// categories, used when has_rad (else the point has no radial term).  The
+// radial term is the cross-entropy -sum_j y_j log q_j of the ring mixture's
+// category probabilities q_j = sum_k w_k M_k(e_j, e_j+1) / S_k
+// (fd2_sg_mix.cuh).  A lane holds one edge of the categories, 31 categories a
+// pass, and goes through the components in order; the sums over the categories
+// run in category order, a lane per sum, from shared memory (v: kSums rows).
+__device__ __forceinline__ PointLoss point_loss(const float *o, float t, const float *y, bool has_rad, int bins,
+                                                float r_max, float lambda, float (*v)[33], float *cj)
 {
+    const int lane = threadIdx.x & 31, k = lane % kComponents;
+    PointLoss p;
     // detection
     const float z = o[0];
-    const float p = 1.0f / (1.0f + expf(-z));
+    const float pd = 1.0f / (1.0f + expf(-z));
     // log p = -softplus(-z), log(1 - p) = -softplus(z)
     const float sp_neg = fmaxf(-z, 0.0f) + log1pf(expf(-fabsf(z)));
     const float sp_pos = fmaxf(z, 0.0f) + log1pf(expf(-fabsf(z)));
     const float ld = t * sp_neg + (1.0f - t) * sp_pos;
-    if (dout) dout[0] = p - t;
-    *det_loss = ld;
-    *rad_loss = 0.0f;
-    if (!y) {
-        if (dout)
-            for (int i = 1; i < kOutputs; ++i) dout[i] = 0.0f;
-        return ld;
-    }
-    Mix m;
-    decode_mix(o, m);
-    // per component: A1 = sum_j c_j M_kj, Amu = sum_j c_j dM_kj/dmu, Asd = sum_j c_j dM_kj/dsd
-    float A1[kComponents], Amu[kComponents], Asd[kComponents];
-    Edge lo[kComponents];
+    p.gz = pd - t;
+    p.det = p.total = ld;
+    p.rad = p.ga = p.gom = p.gls = 0.0f;
+    if (!has_rad) return p;
+    // component k, the same in lanes k, 8 + k, ... (decode_mix)
+    const float a = o[1 + k], om = o[1 + kComponents + k], ls = o[1 + 2 * kComponents + k];
+    float amax = a;
 #pragma unroll
-    for (int k = 0; k < kComponents; ++k) {
-        A1[k] = 0.0f;
-        Amu[k] = 0.0f;
-        Asd[k] = 0.0f;
-        lo[k] = edge_at(0.0f, false, m.mu[k], m.sd[k]);
-    }
-    float lr = 0.0f;
-    for (int j = 0; j <= bins; ++j) {
-        const bool top = j >= bins;
-        const float e_hi = top ? 0.0f : radial_edge(j + 1, bins, r_max);
-        float M[kComponents], dM_mu[kComponents], dM_sd[kComponents];
-        Edge hi[kComponents];
+    for (int d = kComponents / 2; d > 0; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
+    const float ew = expf(a - amax);
+    float s = 0.0f;
+#pragma unroll
+    for (int c = 0; c < kComponents; ++c) s += __shfl_sync(0xffffffffu, ew, c);
+    const float w = ew / s;
+    const float mu = kMuScale * (fmaxf(om, 0.0f) + log1pf(expf(-fabsf(om))));  // softplus
+    const float dmu = kMuScale / (1.0f + expf(-om));                           // d mu / d output
+    const bool clamped = ls < kLogSdMin || ls > kLogSdMax;
+    const float sd = kSdScale * expf(fminf(fmaxf(ls, kLogSdMin), kLogSdMax));
+    const float t0 = -mu / sd;
+    const float c0 = normcdff(-t0), p0 = norm_pdf(t0);
+    const float S = fmaxf(mu * c0 + sd * p0, 1e-30f);
+    // lane c of the first kSums: A1 = sum_j c_j M_j, Amu = sum_j c_j dM_j/dmu,
+    // Asd = sum_j c_j dM_j/dsd of component c % 8, and the last the loss
+    float sum = 0.0f;
+    for (int j0 = 0; j0 <= bins; j0 += 31) {
+        const int j = j0 + lane;
+        Edge lo;
+        lo.inf = j > bins;
+        lo.e = lo.inf ? 0.0f : radial_edge(j, bins, r_max);
         float q = 0.0f;
-#pragma unroll
-        for (int k = 0; k < kComponents; ++k) {
-            hi[k] = edge_at(e_hi, top, m.mu[k], m.sd[k]);
-            M[k] = ring_mass(lo[k], hi[k], m.mu[k], m.sd[k], &dM_mu[k], &dM_sd[k]);
-            q += m.w[k] * M[k] / m.S[k];
-        }
-        const float yj = y[j];
-        if (yj > 0.0f) {
-            const float qe = q + 1e-12f;
-            lr -= yj * logf(qe);
-            const float c = yj / qe;
-#pragma unroll
-            for (int k = 0; k < kComponents; ++k) {
-                A1[k] += c * M[k];
-                Amu[k] += c * dM_mu[k];
-                Asd[k] += c * dM_sd[k];
+#pragma unroll 2
+        for (int c = 0; c < kComponents; ++c) {
+            const float wc = __shfl_sync(0xffffffffu, w, c), mc = __shfl_sync(0xffffffffu, mu, c);
+            const float sc = __shfl_sync(0xffffffffu, sd, c), Sc = __shfl_sync(0xffffffffu, S, c);
+            // of an edge's two tails only those that the intervals on its two
+            // sides read (ring_mass): the lower one before the ring's radius,
+            // the upper one past it, both at the first edge past it
+            lo.t = (lo.e - mc) / sc;
+            const bool past = lo.t >= 0.0f;
+            lo.cdf = lo.ccdf = normcdff(past ? -lo.t : lo.t);
+            const bool before = __shfl_up_sync(0xffffffffu, lo.t, 1) < 0.0f;
+            if (past && before) lo.cdf = normcdff(lo.t);
+            lo.pdf = norm_pdf(lo.t);
+            if (lo.inf) {
+                lo.t = 0.0f;
+                lo.cdf = 1.0f;
+                lo.ccdf = 0.0f;
+                lo.pdf = 0.0f;
             }
+            Edge hi;
+            hi.t = __shfl_down_sync(0xffffffffu, lo.t, 1);
+            hi.cdf = __shfl_down_sync(0xffffffffu, lo.cdf, 1);
+            hi.ccdf = __shfl_down_sync(0xffffffffu, lo.ccdf, 1);
+            hi.pdf = __shfl_down_sync(0xffffffffu, lo.pdf, 1);
+            hi.e = __shfl_down_sync(0xffffffffu, lo.e, 1);
+            hi.inf = j + 1 > bins;
+            float dM_mu, dM_sd;
+            const float M = ring_mass(lo, hi, mc, sc, &dM_mu, &dM_sd);
+            q += wc * M / Sc;
+            v[c][lane] = M;
+            v[kComponents + c][lane] = dM_mu;
+            v[2 * kComponents + c][lane] = dM_sd;
         }
-#pragma unroll
-        for (int k = 0; k < kComponents; ++k) lo[k] = hi[k];
+        const float yj = lane < 31 && j <= bins ? y[j] : 0.0f;
+        const float qe = q + 1e-12f;
+        v[kSums - 1][lane] = yj > 0.0f ? logf(qe) : 0.0f;
+        cj[lane] = yj > 0.0f ? yj / qe : 0.0f;
+        cj[32 + lane] = -yj;
+        __syncwarp();
+        if (lane < kSums) {
+            const float *f = cj + (lane == kSums - 1 ? 32 : 0), *x = v[lane];
+            const int n = min(31, bins + 1 - j0);
+#pragma unroll 4
+            for (int i = 0; i < n; ++i) sum = fmaf(f[i], x[i], sum);
+        }
+        __syncwarp();
     }
-    *rad_loss = lr;
-    if (dout) {
-        float gw[kComponents], wg = 0.0f;
+    const float A1 = __shfl_sync(0xffffffffu, sum, k), Amu = __shfl_sync(0xffffffffu, sum, kComponents + k);
+    const float Asd = __shfl_sync(0xffffffffu, sum, 2 * kComponents + k);
+    p.rad = __shfl_sync(0xffffffffu, sum, kSums - 1);
+    p.total = ld + lambda * p.rad;
+    const float gw = -A1 / S;
+    float wg = 0.0f;
 #pragma unroll
-        for (int k = 0; k < kComponents; ++k) {
-            gw[k] = -A1[k] / m.S[k];
-            wg += m.w[k] * gw[k];
-        }
-#pragma unroll
-        for (int k = 0; k < kComponents; ++k) {
-            const float f = m.w[k] / m.S[k];
-            const float gmu = -f * (Amu[k] - A1[k] * m.dS_mu[k] / m.S[k]);
-            const float gsd = -f * (Asd[k] - A1[k] * m.dS_sd[k] / m.S[k]);
-            dout[1 + k] = lambda * m.w[k] * (gw[k] - wg);
-            dout[1 + kComponents + k] = lambda * m.dmu[k] * gmu;
-            dout[1 + 2 * kComponents + k] = m.clamped[k] ? 0.0f : lambda * m.sd[k] * gsd;
-        }
-    }
-    return ld + lambda * lr;
+    for (int c = 0; c < kComponents; ++c)
+        wg += __shfl_sync(0xffffffffu, w, c) * __shfl_sync(0xffffffffu, gw, c);
+    const float f = w / S;
+    const float gmu = -f * (Amu - A1 * c0 / S);
+    const float gsd = -f * (Asd - A1 * p0 / S);
+    p.ga = lambda * w * (gw - wg);
+    p.gom = lambda * dmu * gmu;
+    p.gls = clamped ? 0.0f : lambda * sd * gsd;
+    return p;
 }
 
 // ------------------------------------------------------------ kernels
@@ -152,14 +194,16 @@ __device__ __forceinline__ void write_input(const float *f, const float *lo, con
 }
 
 // Training batch: rows drawn with Philox(seed, step, row) from [0, n_train),
-// or the rows [first, first + b) in order when `sequential`.
+// or the rows [first, first + b) in order when `sequential`.  One warp per
+// row, its lanes across the radial categories: a thread per row walked 97
+// uncoalesced counts twice (8,192 rows 34 -> 9 us).
 __global__ void gather_kernel(const float *__restrict__ feat, const int32_t *__restrict__ photons,
                               const int32_t *__restrict__ detected, const uint32_t *__restrict__ radial, int bins,
                               int64_t n_train, int64_t first, int b, bool sequential, uint64_t seed,
-                              const unsigned long long *step, NormParams norm, __nv_bfloat16 *__restrict__ x0,
+                              const unsigned long long *step, const __grid_constant__ NormParams norm, __nv_bfloat16 *__restrict__ x0,
                               float *__restrict__ target, float *__restrict__ ylab, float *__restrict__ has_rad)
 {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (r >= b) return;
     int64_t i;
     if (sequential) {
@@ -170,55 +214,65 @@ __global__ void gather_kernel(const float *__restrict__ feat, const int32_t *__r
         const unsigned long long v = ((unsigned long long)h.x << 32) | h.y;
         i = (int64_t)(v % (unsigned long long)n_train);
     }
-    write_input(feat + i * kFeatures, norm.lo, norm.inv, x0 + (int64_t)r * kInPad);
-    const int32_t N = photons[i];
-    target[r] = N > 0 ? (float)detected[i] / (float)N : 0.0f;
     const uint32_t *h = radial + i * (int64_t)(bins + 1);
-    double tot = 0.0;
-    for (int j = 0; j <= bins; ++j) tot += h[j];
+    // whole numbers: exact in any order
+    unsigned long long n = 0;
+    for (int j = lane; j <= bins; j += 32) n += h[j];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    const double tot = (double)n;
     const float inv = tot > 0.0 ? (float)(1.0 / tot) : 0.0f;
-    for (int j = 0; j <= bins; ++j) ylab[(int64_t)r * (bins + 1) + j] = (float)h[j] * inv;
-    has_rad[r] = tot > 0.0 ? 1.0f : 0.0f;
+    for (int j = lane; j <= bins; j += 32) ylab[(int64_t)r * (bins + 1) + j] = (float)h[j] * inv;
+    static_assert(kInPad == 32, "one input column per lane");
+    x0[(int64_t)r * kInPad + lane] = __float2bfloat16(
+        lane < kFeatures ? 2.0f * (feat[i * kFeatures + lane] - norm.lo[lane & 7]) * norm.inv[lane & 7] - 1.0f : 0.0f);
+    if (lane == 0) {
+        const int32_t N = photons[i];
+        target[r] = N > 0 ? (float)detected[i] / (float)N : 0.0f;
+        has_rad[r] = tot > 0.0 ? 1.0f : 0.0f;
+    }
 }
 
 // Loss (summed into acc[0..2] = total, detection, radial) and, when dout is
-// set, dL/dout / b as BF16 [b][64].
-__global__ void loss_kernel(const float *__restrict__ out, int ldo, const float *__restrict__ target,
-                            const float *__restrict__ ylab, const float *__restrict__ has_rad, int bins,
-                            float r_max, float lambda, int b, float scale, __nv_bfloat16 *__restrict__ dout,
-                            double *acc)
+// set, dL/dout / b as BF16 [b][64].  A warp per row (point_loss); instruction
+// issue bounds it (normal tails, exponentials and divisions of 97 x 8 bin
+// masses).  A thread per row left 8,192 threads, 64 per SM, that waited for
+// their dependent instructions: 8,192 rows 588 us, eight lanes per row 136,
+// this 106.
+__global__ void __launch_bounds__(32 * kLossWarps) loss_kernel(const float *__restrict__ out, int ldo,
+                                                               const float *__restrict__ target,
+                                                               const float *__restrict__ ylab,
+                                                               const float *__restrict__ has_rad, int bins,
+                                                               float r_max, float lambda, int b, float scale,
+                                                               __nv_bfloat16 *__restrict__ dout, double *acc)
 {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    float lt = 0.0f, ld = 0.0f, lrad = 0.0f;
+    __shared__ float v[kLossWarps][kSums][33], cj[kLossWarps][64], s[3][kLossWarps];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, r = blockIdx.x * kLossWarps + wid;
+    PointLoss p{};
     if (r < b) {
-        float o[kOutputs], g[kOutputs];
-        for (int i = 0; i < kOutputs; ++i) o[i] = out[(int64_t)r * ldo + i];
-        const bool rad = has_rad[r] > 0.0f;
-        lt = point_loss(o, target[r], rad ? ylab + (int64_t)r * (bins + 1) : nullptr, bins, r_max, lambda,
-                        dout ? g : nullptr, &ld, &lrad);
+        p = point_loss(out + (int64_t)r * ldo, target[r], ylab + (int64_t)r * (bins + 1), has_rad[r] > 0.0f, bins,
+                       r_max, lambda, v[wid], cj[wid]);
         if (dout) {
-            for (int i = 0; i < kOutputs; ++i) dout[(int64_t)r * kOutPad + i] = __float2bfloat16(g[i] * scale);
-            for (int i = kOutputs; i < kOutPad; ++i) dout[(int64_t)r * kOutPad + i] = __float2bfloat16(0.0f);
+            __nv_bfloat16 *d = dout + (int64_t)r * kOutPad;
+            if (lane < kComponents) {
+                if (lane == 0) d[0] = __float2bfloat16(p.gz * scale);
+                d[1 + lane] = __float2bfloat16(p.ga * scale);
+                d[1 + kComponents + lane] = __float2bfloat16(p.gom * scale);
+                d[1 + 2 * kComponents + lane] = __float2bfloat16(p.gls * scale);
+            }
+            for (int i = kOutputs + lane; i < kOutPad; i += 32) d[i] = __float2bfloat16(0.0f);
         }
     }
-    // block sums
-    __shared__ float s[3][32];
-    for (int off = 16; off > 0; off >>= 1) {
-        lt += __shfl_down_sync(0xffffffffu, lt, off);
-        ld += __shfl_down_sync(0xffffffffu, ld, off);
-        lrad += __shfl_down_sync(0xffffffffu, lrad, off);
-    }
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) {
-        s[0][w] = lt;
-        s[1][w] = ld;
-        s[2][w] = lrad;
+    if (lane == 0) {
+        s[0][wid] = p.total;
+        s[1][wid] = p.det;
+        s[2][wid] = p.rad;
     }
     __syncthreads();
     if (threadIdx.x < 3) {
-        double v = 0.0;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) v += s[threadIdx.x][i];
-        atomicAdd(&acc[threadIdx.x], v);
+        double t = 0.0;
+        for (int i = 0; i < kLossWarps; ++i) t += s[threadIdx.x][i];
+        atomicAdd(&acc[threadIdx.x], t);
     }
 }
 
@@ -248,6 +302,39 @@ __global__ void split_sum_kernel(const float *__restrict__ ws, int splits, int64
         for (int z = 0; z < splits; ++z) s += ws[(int64_t)z * n + i];
         out[i] = s;
     }
+}
+
+// The two reductions of a tcgen05 weight gradient in one launch.  Blocks
+// [0, sum_blocks): out[i] = sum_z ws[z][i] (split_sum_kernel); the others:
+// db[n] = sum_r dyT[n][r], a warp per column on the transposed gradient
+// (rows_pad contiguous rows, zeros past the last), in the order of
+// colsum_kernel: lane l the rows l, l + 32, ..., then the lanes' sums in order.
+// (8,192 rows: the column sums of the untransposed gradient took 41 us on 2 or
+// 8 blocks beside 6 us for the split sum; both now 12.)
+__global__ void __launch_bounds__(256) finish_grad_kernel(const float *__restrict__ ws, int splits, int64_t n,
+                                                          float *__restrict__ out, int sum_blocks,
+                                                          const __nv_bfloat16 *__restrict__ dyT, int rows_pad,
+                                                          int cols, float *__restrict__ db)
+{
+    if ((int)blockIdx.x < sum_blocks) {
+        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)sum_blocks * blockDim.x) {
+            float s = 0.0f;
+#pragma unroll 8
+            for (int z = 0; z < splits; ++z) s += ws[(int64_t)z * n + i];
+            out[i] = s;
+        }
+        return;
+    }
+    const int c = ((int)blockIdx.x - sum_blocks) * (int)(blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (c >= cols) return;
+    const __nv_bfloat16 *p = dyT + (int64_t)c * rows_pad + lane;
+    float s = 0.0f;
+#pragma unroll 16
+    for (int r = 0; r < rows_pad; r += 32) s += __bfloat162float(p[r]);
+    float t = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) t += __shfl_sync(0xffffffffu, s, k);
+    if (lane == 0) db[c] = t;
 }
 
 // Adam on the FP32 masters, then the BF16 copies.  `mask` zeroes the update
@@ -280,23 +367,54 @@ __global__ void to_bf16_kernel(const float *__restrict__ p, __nv_bfloat16 *__res
         pb[i] = __float2bfloat16(p[i]);
 }
 
-// out[c][r] = in[r][c] for r < rows, 0 for rows <= r < rows_pad (BF16,
-// 32 x 32 tiles through shared memory; in is [rows][ld_in], out
-// [cols][rows_pad]).  Feeds the tcgen05 backward products, whose operands
-// must be contiguous along the contraction.
-__global__ void transpose_bf16_kernel(const __nv_bfloat16 *__restrict__ in, int ld_in, int rows, int cols,
-                                      int rows_pad, __nv_bfloat16 *__restrict__ out)
+// out[c][r] = in[r][c] for r < rows, 0 for rows <= r < rows_pad (BF16; in is
+// [rows][ld_in], out [cols][rows_pad]), for up to three matrices (blockIdx.z).
+// Feeds the tcgen05 backward products, whose operands must be contiguous along
+// the contraction.  64 x 64 tiles through shared memory, 16 bytes a thread on
+// both sides: ld_in, cols and rows_pad are multiples of 8 and the matrices
+// 16-byte aligned.  An element at a time took 14 us for a layer's two operands
+// at 8,192 rows, this 4.9.
+struct TransposeArgs {
+    const __nv_bfloat16 *in[3];
+    __nv_bfloat16 *out[3];
+    int ld_in[3], rows[3], cols[3], rows_pad[3];
+};
+
+__global__ void __launch_bounds__(256) transpose_bf16_kernel(const __grid_constant__ TransposeArgs a)
 {
-    __shared__ __nv_bfloat16 t[32][33];
-    const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-        const int r = r0 + i, c = c0 + threadIdx.x;
-        t[i][threadIdx.x] = (r < rows && c < cols) ? in[(int64_t)r * ld_in + c] : __float2bfloat16(0.0f);
+    // 66 elements a row: a column's reads fall on different banks
+    __shared__ __nv_bfloat16 t[64][66];
+    const int m = blockIdx.z, r0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
+    const int rows = a.rows[m], cols = a.cols[m], rows_pad = a.rows_pad[m], ld_in = a.ld_in[m];
+    if (r0 >= rows_pad || c0 >= cols) return;
+    const __nv_bfloat16 *in = a.in[m];
+    __nv_bfloat16 *out = a.out[m];
+    const int piece = (threadIdx.x & 7) * 8, line = threadIdx.x >> 3;
+#pragma unroll
+    for (int p = 0; p < 64; p += 32) {
+        const int r = r0 + line + p, c = c0 + piece;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (r < rows && c < cols) v = *reinterpret_cast<const uint4 *>(in + (int64_t)r * ld_in + c);
+        uint32_t *d = reinterpret_cast<uint32_t *>(&t[line + p][piece]);
+        d[0] = v.x;
+        d[1] = v.y;
+        d[2] = v.z;
+        d[3] = v.w;
     }
     __syncthreads();
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-        const int c = c0 + i, r = r0 + threadIdx.x;
-        if (c < cols && r < rows_pad) out[(int64_t)c * rows_pad + r] = t[threadIdx.x][i];
+#pragma unroll
+    for (int p = 0; p < 64; p += 32) {
+        const int c = c0 + line + p, r = r0 + piece;
+        if (c >= cols || r >= rows_pad) continue;
+        __nv_bfloat16 e[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) e[i] = t[piece + i][line + p];
+        uint4 v;
+        v.x = (uint32_t)__bfloat16_as_ushort(e[0]) | (uint32_t)__bfloat16_as_ushort(e[1]) << 16;
+        v.y = (uint32_t)__bfloat16_as_ushort(e[2]) | (uint32_t)__bfloat16_as_ushort(e[3]) << 16;
+        v.z = (uint32_t)__bfloat16_as_ushort(e[4]) | (uint32_t)__bfloat16_as_ushort(e[5]) << 16;
+        v.w = (uint32_t)__bfloat16_as_ushort(e[6]) | (uint32_t)__bfloat16_as_ushort(e[7]) << 16;
+        *reinterpret_cast<uint4 *>(out + (int64_t)c * rows_pad + r) = v;
     }
 }
 
@@ -322,6 +440,10 @@ unsigned grid_for(int64_t n, int block, int cap = 4096)
 }
 
 }  // namespace
+
+// Blocks of 256 threads with a warp per row.
+static unsigned warps_for(int64_t rows) { return (unsigned)((rows + 7) / 8); }
+static unsigned loss_blocks(int64_t rows) { return (unsigned)((rows + kLossWarps - 1) / kLossWarps); }
 
 fd2_status sg_fail(fd2_sg *s, fd2_status st, const std::string &msg)
 {
@@ -464,12 +586,28 @@ constexpr int kTcSlice = 256;  // batch rows per weight-gradient slice (the cont
 
 int rows_pad(int rows) { return (rows + kTcSlice - 1) / kTcSlice * kTcSlice; }
 
-cudaError_t launch_transpose(cudaStream_t st, const __nv_bfloat16 *in, int ld_in, int rows, int cols,
-                             __nv_bfloat16 *out)
+// The transposes of n <= 3 matrices: {in, ld_in, rows, cols, rows_pad, out}.
+struct Transpose {
+    const __nv_bfloat16 *in;
+    int ld_in, rows, cols, rows_pad;
+    __nv_bfloat16 *out;
+};
+
+cudaError_t launch_transpose(cudaStream_t st, const Transpose *t, int n)
 {
-    const int rp = rows_pad(rows);
-    transpose_bf16_kernel<<<dim3((unsigned)(rp / 32), (unsigned)((cols + 31) / 32)), dim3(32, 8), 0, st>>>(
-        in, ld_in, rows, cols, rp, out);
+    TransposeArgs a{};
+    int x = 1, y = 1;
+    for (int i = 0; i < n; ++i) {
+        a.in[i] = t[i].in;
+        a.out[i] = t[i].out;
+        a.ld_in[i] = t[i].ld_in;
+        a.rows[i] = t[i].rows;
+        a.cols[i] = t[i].cols;
+        a.rows_pad[i] = t[i].rows_pad;
+        x = std::max(x, (t[i].rows_pad + 63) / 64);
+        y = std::max(y, (t[i].cols + 63) / 64);
+    }
+    transpose_bf16_kernel<<<dim3((unsigned)x, (unsigned)y, (unsigned)n), 256, 0, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -556,32 +694,45 @@ bool tc_backward_ok(const fd2_sg *s, int rows)
 // dy_z^T x_z, with dy^T ([M][rows_pad]) and x^T ([K][rows_pad]) staged
 // contiguous along the batch; one CTA per (128-row tile of dW, slice), FP32
 // partial planes summed in slice order (deterministic).
-cudaError_t weight_grad_tc(fd2_sg *s, cudaStream_t st, const __nv_bfloat16 *dy, int ldy, int M,
-                           const __nv_bfloat16 *x, int ldx, int K, int rows, float *dw)
+// The bias gradient (column sums of dy) comes with it.
+// On the layer's own stream and buffers, after what `st` holds: nothing of the
+// backward pass waits for it before its end, so the layers' weight gradients
+// run beside the chain of input gradients (8,192 rows: 64 CTAs a launch on 148
+// SMs).
+cudaError_t weight_grad_tc(fd2_sg *s, cudaStream_t main, int layer, const __nv_bfloat16 *dy, int ldy, int M,
+                           const __nv_bfloat16 *x, int ldx, int K, int rows, float *dw, float *db)
 {
     cudaError_t e;
+    cudaStream_t st = s->side[layer];
+    __nv_bfloat16 *tA = s->tA + layer * s->t_stride, *tB = s->tB + layer * s->t_stride;
+    float *ws = s->ws + layer * s->ws_floats;
     const int rp = rows_pad(rows), z = rp / kTcSlice;
-    if ((int64_t)z * M * K > s->ws_floats) return cudaErrorInvalidValue;
-    if ((e = launch_transpose(st, dy, ldy, rows, M, s->tA)) != cudaSuccess) return e;
-    if ((e = launch_transpose(st, x, ldx, rows, K, s->tB)) != cudaSuccess) return e;
+    if ((int64_t)z * M * K > s->ws_floats || (int64_t)std::max(M, K) * rp > s->t_stride) return cudaErrorInvalidValue;
+    if ((e = cudaEventRecord(s->ev_main[layer], main)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(st, s->ev_main[layer], 0)) != cudaSuccess) return e;
+    const Transpose t2[2] = {{dy, ldy, rows, M, rp, tA}, {x, ldx, rows, K, rp, tB}};
+    if ((e = launch_transpose(st, t2, 2)) != cudaSuccess) return e;
     TcArgs t{};
-    t.A = s->tA;
-    t.B = s->tB;
+    t.A = tA;
+    t.B = tB;
     t.lda = rp;
     t.ldb = rp;
     t.M = M;
     t.N = K;
     t.K = kTcSlice;
     t.epi = kEpiPartialF32;
-    t.C = s->ws;
+    t.C = ws;
     t.ldc = K;
     t.a_split = kTcSlice;
     t.b_split = kTcSlice;
     t.c_split = (long long)M * K;
     t.fault = s->d_tc_fault;
     if ((e = launch_tc(s, st, t, (unsigned)((M + kTcRows - 1) / kTcRows), (unsigned)z)) != cudaSuccess) return e;
-    split_sum_kernel<<<grid_for((int64_t)M * K, 256), 256, 0, st>>>(s->ws, z, (int64_t)M * K, dw);
-    return cudaGetLastError();
+    const unsigned sums = grid_for((int64_t)M * K, 256);
+    finish_grad_kernel<<<sums + (unsigned)((M + 7) / 8), 256, 0, st>>>(ws, z, (int64_t)M * K, dw, (int)sums, tA,
+                                                                       rp, M, db);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    return cudaEventRecord(s->ev_side[layer], st);
 }
 
 // Input gradient on tcgen05: d [rows][H] = (dy [rows][Nout] W [Nout][H]) *
@@ -616,30 +767,30 @@ cudaError_t backward(fd2_sg *s, cudaStream_t st, int rows)
     if (tc_backward_ok(s, rows)) {
         // the weights' transposes (BF16 copies of this step's parameters)
         __nv_bfloat16 *w2T = s->pbT, *w3T = s->pbT + (size_t)H * H, *w4T = s->pbT + 2 * (size_t)H * H;
-        const dim3 tb(32, 8), tg((unsigned)((H + 31) / 32), (unsigned)((H + 31) / 32));
-        transpose_bf16_kernel<<<dim3((unsigned)((kOutPad + 31) / 32), tg.y), tb, 0, st>>>(s->pb + s->off[kW4], H,
-                                                                                          kOutPad, H, kOutPad, w4T);
-        transpose_bf16_kernel<<<tg, tb, 0, st>>>(s->pb + s->off[kW3], H, H, H, H, w3T);
-        transpose_bf16_kernel<<<tg, tb, 0, st>>>(s->pb + s->off[kW2], H, H, H, H, w2T);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        const Transpose tw[3] = {{s->pb + s->off[kW4], H, kOutPad, H, kOutPad, w4T},
+                                 {s->pb + s->off[kW3], H, H, H, H, w3T},
+                                 {s->pb + s->off[kW2], H, H, H, H, w2T}};
+        if ((e = launch_transpose(st, tw, 3)) != cudaSuccess) return e;
         // layer 4
-        if ((e = weight_grad_tc(s, st, s->dout, kOutPad, kOutPad, s->h3, H, H, rows, G + s->off[kW4])) != cudaSuccess)
+        if ((e = weight_grad_tc(s, st, 3, s->dout, kOutPad, kOutPad, s->h3, H, H, rows, G + s->off[kW4],
+                                G + s->off[kB4])) != cudaSuccess)
             return e;
-        colsum_kernel<<<(kOutPad + 31) / 32, 1024, 0, st>>>(s->dout, kOutPad, rows, kOutPad, G + s->off[kB4]);
         if ((e = input_grad_tc(s, st, s->dout, kOutPad, w4T, s->h3, rows, s->d3)) != cudaSuccess) return e;
         // layer 3
-        if ((e = weight_grad_tc(s, st, s->d3, H, H, s->h2, H, H, rows, G + s->off[kW3])) != cudaSuccess) return e;
-        colsum_kernel<<<(H + 31) / 32, 1024, 0, st>>>(s->d3, H, rows, H, G + s->off[kB3]);
+        if ((e = weight_grad_tc(s, st, 2, s->d3, H, H, s->h2, H, H, rows, G + s->off[kW3], G + s->off[kB3])) != cudaSuccess)
+            return e;
         if ((e = input_grad_tc(s, st, s->d3, H, w3T, s->h2, rows, s->d2)) != cudaSuccess) return e;
         // layer 2
-        if ((e = weight_grad_tc(s, st, s->d2, H, H, s->h1, H, H, rows, G + s->off[kW2])) != cudaSuccess) return e;
-        colsum_kernel<<<(H + 31) / 32, 1024, 0, st>>>(s->d2, H, rows, H, G + s->off[kB2]);
+        if ((e = weight_grad_tc(s, st, 1, s->d2, H, H, s->h1, H, H, rows, G + s->off[kW2], G + s->off[kB2])) != cudaSuccess)
+            return e;
         if ((e = input_grad_tc(s, st, s->d2, H, w2T, s->h1, rows, s->d1)) != cudaSuccess) return e;
         // layer 1
-        if ((e = weight_grad_tc(s, st, s->d1, H, H, s->x0, kInPad, kInPad, rows, G + s->off[kW1])) != cudaSuccess)
+        if ((e = weight_grad_tc(s, st, 0, s->d1, H, H, s->x0, kInPad, kInPad, rows, G + s->off[kW1],
+                                G + s->off[kB1])) != cudaSuccess)
             return e;
-        colsum_kernel<<<(H + 31) / 32, 1024, 0, st>>>(s->d1, H, rows, H, G + s->off[kB1]);
-        return cudaGetLastError();
+        for (cudaEvent_t ev : s->ev_side)
+            if ((e = cudaStreamWaitEvent(st, ev, 0)) != cudaSuccess) return e;
+        return cudaSuccess;
     }
     // layer 4
     if ((e = weight_grad(s, st, s->dout, kOutPad, kOutPad, s->h3, H, H, rows, G + s->off[kW4])) != cudaSuccess)
@@ -674,11 +825,11 @@ cudaError_t train_step(fd2_sg *s, cudaStream_t st)
 {
     const int B = s->batch, bins = s->bins;
     cudaError_t e;
-    gather_kernel<<<grid_for(B, 256), 256, 0, st>>>(s->d_feat, s->d_photons, s->d_detected, s->d_radial, bins,
+    gather_kernel<<<warps_for(B), 256, 0, st>>>(s->d_feat, s->d_photons, s->d_detected, s->d_radial, bins,
                                                     s->n_train, 0, B, false, s->seed, s->d_step, s->norm, s->x0,
                                                     s->target, s->ylab, s->has_rad);
     if ((e = sg_forward(s, st, s->x0, B, nullptr, s->h1, s->h2, s->h3, s->out)) != cudaSuccess) return e;
-    loss_kernel<<<grid_for(B, 128), 128, 0, st>>>(s->out, kOutPad, s->target, s->ylab, s->has_rad, bins,
+    loss_kernel<<<loss_blocks(B), 32 * kLossWarps, 0, st>>>(s->out, kOutPad, s->target, s->ylab, s->has_rad, bins,
                                                   (float)s->radial_max, s->lambda, B, 1.0f / (float)B,
                                                   s->dout, s->d_acc);
     if ((e = backward(s, st, B)) != cudaSuccess) return e;
@@ -792,11 +943,14 @@ fd2_status ensure_rows(fd2_sg *s, int rows)
     // tcgen05 backward: transposed operands over the rows padded to 256, and
     // one FP32 partial plane per 256-row slice
     const size_t RP = (size_t)rows_pad(rows);
-    SG_CUDA(s, alloc(&s->tA, std::max<size_t>(H, kOutPad) * RP));
-    SG_CUDA(s, alloc(&s->tB, std::max<size_t>(H, kInPad) * RP));
+    // (for each layer: the four weight gradients run side by side)
+    const size_t ts = std::max<size_t>(H, kOutPad) * RP;
+    SG_CUDA(s, alloc(&s->tA, 4 * ts));
+    SG_CUDA(s, alloc(&s->tB, 4 * ts));
+    s->t_stride = (int64_t)ts;
     const size_t plane = std::max<size_t>(H * H, (size_t)kOutPad * H);
     const size_t wsf = std::max<size_t>((size_t)kMaxSplits, RP / kTcSlice) * plane;
-    SG_CUDA(s, alloc(&s->ws, wsf));
+    SG_CUDA(s, alloc(&s->ws, 4 * wsf));
     s->ws_floats = (int64_t)wsf;
     SG_CUDA(s, alloc(&s->x0, R * kInPad));
     SG_CUDA(s, alloc(&s->h1, R * H));
@@ -882,6 +1036,11 @@ fd2_status fd2_sg_create(const fd2_sg_config *cfg, fd2_sg **out)
     };
     if (cudaSetDevice(s->device) != cudaSuccess) return bail(FD2_ERR_CUDA);
     if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(FD2_ERR_CUDA);
+    for (int l = 0; l < 4; ++l)
+        if (cudaStreamCreateWithFlags(&s->side[l], cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&s->ev_main[l], cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&s->ev_side[l], cudaEventDisableTiming) != cudaSuccess)
+            return bail(FD2_ERR_CUDA);
     layout(s);
     const size_t P = (size_t)s->n_params;
     if (alloc(&s->p, P) || alloc(&s->g, P) || alloc(&s->m, P) || alloc(&s->v, P) || alloc(&s->pb, P) ||
@@ -966,6 +1125,12 @@ void fd2_sg_destroy(fd2_sg *s)
     if (!s) return;
     cudaSetDevice(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
+    for (int l = 0; l < 4; ++l) {
+        if (s->side[l]) cudaStreamSynchronize(s->side[l]);
+        if (s->side[l]) cudaStreamDestroy(s->side[l]);
+        if (s->ev_main[l]) cudaEventDestroy(s->ev_main[l]);
+        if (s->ev_side[l]) cudaEventDestroy(s->ev_side[l]);
+    }
     if (s->graph) cudaGraphExecDestroy(s->graph);
     for (void *p : {(void *)s->p, (void *)s->g, (void *)s->m, (void *)s->v, (void *)s->pb, (void *)s->d_live,
                     (void *)s->d_step, (void *)s->d_acc, (void *)s->d_lr, (void *)s->ws, (void *)s->x0, (void *)s->h1, (void *)s->h2,
@@ -1106,12 +1271,12 @@ fd2_status fd2_sg_eval(fd2_sg *s, float *loss, float *det_loss, float *radial_lo
     SG_CUDA(s, cudaMemsetAsync(s->d_acc, 0, sizeof(double) * 4, s->stream));
     for (int64_t at = 0; at < count; at += s->batch) {
         const int b = (int)std::min<int64_t>(s->batch, count - at);
-        gather_kernel<<<grid_for(b, 256), 256, 0, s->stream>>>(s->d_feat, s->d_photons, s->d_detected, s->d_radial,
+        gather_kernel<<<warps_for(b), 256, 0, s->stream>>>(s->d_feat, s->d_photons, s->d_detected, s->d_radial,
                                                                s->bins, s->n_train, first + at, b, true, s->seed,
                                                                s->d_step, s->norm, s->x0, s->target, s->ylab,
                                                                s->has_rad);
         SG_CUDA(s, sg_forward(s, s->stream, s->x0, b, nullptr, s->h1, s->h2, s->h3, s->out));
-        loss_kernel<<<grid_for(b, 128), 128, 0, s->stream>>>(s->out, kOutPad, s->target, s->ylab, s->has_rad,
+        loss_kernel<<<loss_blocks(b), 32 * kLossWarps, 0, s->stream>>>(s->out, kOutPad, s->target, s->ylab, s->has_rad,
                                                              s->bins, (float)s->radial_max, s->lambda, b,
                                                              1.0f, nullptr, s->d_acc);
         SG_CUDA(s, cudaGetLastError());
@@ -1186,13 +1351,13 @@ fd2_status fd2_sg_loss_grad(fd2_sg *s, const float *features, const int32_t *pho
     if (e == cudaSuccess) e = cudaMemcpy(dr, radial, sizeof(uint32_t) * b * nb, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->d_acc, 0, sizeof(double) * 4, s->stream);
     if (e == cudaSuccess) {
-        gather_kernel<<<grid_for(b, 256), 256, 0, s->stream>>>(df, dp, dd, dr, s->bins, b, 0, b, true, s->seed,
+        gather_kernel<<<warps_for(b), 256, 0, s->stream>>>(df, dp, dd, dr, s->bins, b, 0, b, true, s->seed,
                                                                s->d_step, s->norm, s->x0, s->target, s->ylab,
                                                                s->has_rad);
         e = sg_forward(s, s->stream, s->x0, b, nullptr, s->h1, s->h2, s->h3, s->out);
     }
     if (e == cudaSuccess) {
-        loss_kernel<<<grid_for(b, 128), 128, 0, s->stream>>>(s->out, kOutPad, s->target, s->ylab, s->has_rad,
+        loss_kernel<<<loss_blocks(b), 32 * kLossWarps, 0, s->stream>>>(s->out, kOutPad, s->target, s->ylab, s->has_rad,
                                                              s->bins, (float)s->radial_max, s->lambda, b,
                                                              1.0f / (float)b, s->dout, s->d_acc);
         e = backward(s, s->stream, b);
