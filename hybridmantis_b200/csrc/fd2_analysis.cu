@@ -1,18 +1,25 @@
 // fd2_analysis.cu -- MTF and NNPS of the transport's images (include/fd2_analysis.h).
 //
 // Both are discrete Fourier transforms of modest images (hundreds of pixels
-// a side), taken as two passes of direct sums in FP64 with exact integer
-// phase reduction: pass 1 transforms every row at the wanted column
-// frequencies, pass 2 every resulting column at the wanted row frequencies.
-// A pass is one thread per output value looping over the inputs, the input
-// row staged in shared memory (pass 1) or read coalesced across threads
-// (pass 2), twiddles exp(-2 pi i m / N) from a table.  The magnitudes are
-// reduced into radial bins with FP64 atomics on the device.
+// a side), taken as two passes of direct sums in FP64 with exact integer phase
+// reduction: pass 1 transforms every row at the wanted column frequencies,
+// pass 2 every resulting column at the wanted row frequencies.  The images are
+// real, so only column frequencies >= 0 are computed; the others are their
+// conjugates.  The passes are matrix products with twiddle factors
+// exp(-2 pi i m / N) from a table, bound by FP64 multiply-adds and
+// shared-memory reads: a thread keeps four complex sums in registers, the
+// twiddles of a warp are the same for its lanes (broadcast reads), and the
+// next chunk of a tile is loaded while one is summed.  One thread per output
+// with a table read of its own per multiply-add took 164 us and 323 us for a
+// 501 x 501 image at all frequencies; the passes below take 46 and 45 us.  All
+// regions of all images of a noise spectrum go through them together (144
+// regions of 128 x 128 pixels: 89 and 121 us; region by region 288 launches).
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <mutex>
 #include <vector>
 
 #include "fd2.h"
@@ -21,6 +28,10 @@
 namespace {
 
 constexpr int kThreads = 128;
+constexpr int kFreqs = 16;      // frequencies of a block: 4 warps x 4
+constexpr int kRowTile = 32;    // pass 1: rows of a block, 1 a lane
+constexpr int kColTile = 32;    // pass 2: column frequencies of a block, 1 a lane
+constexpr int kDepth = 32;      // terms staged in shared memory at a time
 
 // tw[m] = exp(-2 pi i m / N), m < N
 __global__ void twiddle_kernel(int n, double2 *tw)
@@ -32,100 +43,233 @@ __global__ void twiddle_kernel(int n, double2 *tw)
     tw[m] = make_double2(c, -s);
 }
 
-// out[r * nk + k] = sum_{c < ncols} (in[(r0 + r) * ld + c0 + c] - sub) tw[(freq[k] c) mod n]
-// grid (ceil(nk / kThreads), nrows); dynamic shared memory: ncols doubles.
-__global__ void dft_rows_kernel(const double *__restrict__ in, int64_t ld, int r0, int c0, int ncols, double sub,
-                                const int *__restrict__ freq, int nk, const double2 *__restrict__ tw, int n,
-                                double2 *__restrict__ out)
+// The regions to transform: rows x cols of every image at the origins of a
+// grid of regions, minus the mean image, or with a single image minus each
+// region's mean (sum / (rows cols)).
+struct Regions {
+    const double *img;
+    int64_t ld, image;          // row and image strides
+    int x0, y0, rows, cols, across, per_image;  // grid of regions: `across` along y
+    const double *mean;         // mean image, or null
+    const double *sums;         // region sums of a single image, or null
+};
+
+// out[z][r][k] = sum_c (in_z[r][c] - mean) tw[(k c) mod n] for k < nk of the
+// region z = first + blockIdx.z.  grid (row tiles, frequency tiles, regions).
+__global__ void __launch_bounds__(kThreads) dft_rows_kernel(const __grid_constant__ Regions g, int first, int nk,
+                                                            const double2 *__restrict__ tw, int n,
+                                                            double2 *__restrict__ out)
 {
-    extern __shared__ double row[];
-    const int r = blockIdx.y;
-    const double *src = in + (int64_t)(r0 + r) * ld + c0;
-    for (int c = threadIdx.x; c < ncols; c += blockDim.x) row[c] = src[c] - sub;
+    __shared__ double tile[kDepth][kRowTile + 1];
+    __shared__ double2 wt[kDepth][kFreqs];
+    const int z = first + blockIdx.z, image = z / g.per_image, q = z % g.per_image;
+    const int ox = g.x0 + q / g.across * g.rows, oy = g.y0 + q % g.across * g.cols;
+    const int64_t origin = (int64_t)ox * g.ld + oy;
+    const double *src = g.img + image * g.image + origin;
+    const double *mean = g.mean ? g.mean + origin : nullptr;
+    const double sub = g.sums ? g.sums[q] / ((double)g.rows * g.cols) : 0.0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r0 = blockIdx.x * kRowTile, k0 = blockIdx.y * kFreqs;
+    double re[4] = {}, im[4] = {};
+    // the next chunk is loaded while this one is summed: a warp takes rows
+    // warp, warp + 4, ... of the tile, its lanes the chunk's columns
+    constexpr int kLoads = kRowTile / 4, kTw = kDepth * kFreqs / kThreads;
+    double next[kLoads];
+    double2 next_w[kTw];
+    auto load = [&](int c0) {
+        const bool in = c0 + lane < g.cols;
+#pragma unroll
+        for (int i = 0; i < kLoads; ++i) {
+            const int r = r0 + warp + 4 * i;
+            const int64_t at = (int64_t)r * g.ld + c0 + lane;
+            double v = 0.0;
+            if (in && r < g.rows) {
+                v = src[at];
+                if (mean) v -= mean[at];
+                else if (g.sums) v -= sub;
+            }
+            next[i] = v;
+        }
+#pragma unroll
+        for (int i = 0; i < kTw; ++i) {
+            const int t = threadIdx.x + i * kThreads;
+            // below 2^32: sides are at most 16,384
+            next_w[i] = tw[(uint32_t)(k0 + t % kFreqs) * (uint32_t)(c0 + t / kFreqs) % (uint32_t)n];
+        }
+    };
+    load(0);
+    for (int c0 = 0; c0 < g.cols; c0 += kDepth) {
+        const int nc = min(kDepth, g.cols - c0);
+#pragma unroll
+        for (int i = 0; i < kLoads; ++i) tile[lane][warp + 4 * i] = next[i];
+#pragma unroll
+        for (int i = 0; i < kTw; ++i) {
+            const int t = threadIdx.x + i * kThreads;
+            wt[t / kFreqs][t % kFreqs] = next_w[i];
+        }
+        __syncthreads();
+        if (c0 + kDepth < g.cols) load(c0 + kDepth);
+#pragma unroll 4
+        for (int c = 0; c < nc; ++c) {
+            const double a = tile[c][lane];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const double2 w = wt[c][warp * 4 + j];
+                re[j] = fma(a, w.x, re[j]);
+                im[j] = fma(a, w.y, im[j]);
+            }
+        }
+        __syncthreads();
+    }
+    double2 *o = out + (int64_t)blockIdx.z * g.rows * nk;
+    const int r = r0 + lane;
+    if (r >= g.rows) return;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int k = k0 + warp * 4 + j;
+        if (k < nk) o[(int64_t)r * nk + k] = make_double2(re[j], im[j]);
+    }
+}
+
+// Pass 2 at the row frequencies s_u = u + shift, u < nu, of every column k of
+// (nrows x nk) matrices: h = sum_r a[r][k] tw[(s_u r) mod n].  power == 0:
+// map[u][k] = |h| of the single matrix.  power == 1: plane blockIdx.z of map
+// [u][k] += |h|^2 over the matrices blockIdx.z, + gridDim.z, ... (one block
+// per element of a plane, so sums run in a fixed order).
+// grid (column tiles, frequency tiles, planes).
+__global__ void __launch_bounds__(kThreads) dft_cols_kernel(const double2 *__restrict__ a, int matrices, int nrows,
+                                                            int nk, int nu, int shift,
+                                                            const double2 *__restrict__ tw, int n, int power,
+                                                            double *__restrict__ map)
+{
+    __shared__ double2 tile[kDepth][kColTile];
+    __shared__ double2 wt[kDepth][kFreqs];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int k0 = blockIdx.x * kColTile, u0 = blockIdx.y * kFreqs, k = k0 + lane;
+    double sum[4] = {};
+    for (int m = blockIdx.z; m < matrices; m += gridDim.z) {
+        const double2 *src = a + (int64_t)m * nrows * nk;
+        double re[4] = {}, im[4] = {};
+        constexpr int kLoads = kDepth / 4, kTw = kDepth * kFreqs / kThreads;
+        double2 next[kLoads], next_w[kTw];
+        auto load = [&](int r0) {
+#pragma unroll
+            for (int i = 0; i < kLoads; ++i) {
+                const int r = r0 + warp + 4 * i;
+                next[i] = r < nrows && k < nk ? src[(int64_t)r * nk + k] : make_double2(0.0, 0.0);
+            }
+#pragma unroll
+            for (int i = 0; i < kTw; ++i) {
+                const int t = threadIdx.x + i * kThreads;
+                const uint32_t f = (uint32_t)((u0 + t % kFreqs + shift) % n + n);  // the signed frequency mod n, plus n
+                next_w[i] = tw[f * (uint32_t)(r0 + t / kFreqs) % (uint32_t)n];
+            }
+        };
+        load(0);
+        for (int r0 = 0; r0 < nrows; r0 += kDepth) {
+            const int nr = min(kDepth, nrows - r0);
+#pragma unroll
+            for (int i = 0; i < kLoads; ++i) tile[warp + 4 * i][lane] = next[i];
+#pragma unroll
+            for (int i = 0; i < kTw; ++i) {
+                const int t = threadIdx.x + i * kThreads;
+                wt[t / kFreqs][t % kFreqs] = next_w[i];
+            }
+            __syncthreads();
+            if (r0 + kDepth < nrows) load(r0 + kDepth);
+#pragma unroll 4
+            for (int r = 0; r < nr; ++r) {
+                const double2 x = tile[r][lane];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const double2 w = wt[r][warp * 4 + j];
+                    re[j] = fma(x.x, w.x, fma(-x.y, w.y, re[j]));
+                    im[j] = fma(x.x, w.y, fma(x.y, w.x, im[j]));
+                }
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sum[j] += power ? re[j] * re[j] + im[j] * im[j] : sqrt(re[j] * re[j] + im[j] * im[j]);
+    }
+    if (k >= nk) return;
+    double *o = map + (int64_t)blockIdx.z * nu * nk;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int u = u0 + warp * 4 + j;
+        if (u >= nu) continue;
+        if (power) o[(int64_t)u * nk + k] += sum[j];
+        else o[(int64_t)u * nk + k] = sum[j];
+    }
+}
+
+// Radial average of a map [nu][nk] of a real image's transform: signed row
+// frequency u + shift (folded to (-wrap / 2, wrap / 2] with wrap > 0), column
+// frequency k >= 0, whose mirror (-u, -k) the map leaves out and counts as a
+// second value (`single`: the column frequency besides 0 that is its own
+// mirror, or -1).  Block b averages the values whose radius rounds to b, each
+// divided by *norm where given.
+__global__ void __launch_bounds__(kThreads) radial_kernel(const double *__restrict__ map, int nu, int nk, int shift,
+                                                          int wrap, int single, const double *__restrict__ norm,
+                                                          double *__restrict__ out)
+{
+    __shared__ double part[kThreads];
+    __shared__ int count[kThreads];
+    const int b = blockIdx.x;
+    const double lo = b - 0.5, hi = b + 0.5;
+    double s = 0.0;
+    int n = 0;
+    for (int u = threadIdx.x; u < nu; u += kThreads) {
+        int su = u + shift;
+        if (wrap > 0 && su > wrap / 2) su -= wrap;
+        const double u2 = (double)su * su;
+        // the columns whose radius can round to b, one more on both sides
+        const int k_lo = max((int)sqrt(fmax(lo * lo - u2, 0.0)) - 1, 0);
+        const int k_hi = min((int)sqrt(fmax(hi * hi - u2, 0.0)) + 1, nk - 1);
+        for (int k = k_lo; k <= k_hi; ++k) {
+            if ((int)llrint(sqrt(u2 + (double)k * k)) != b) continue;
+            const int weight = k == 0 || k == single ? 1 : 2;
+            s += weight * map[(int64_t)u * nk + k];
+            n += weight;
+        }
+    }
+    part[threadIdx.x] = s;
+    count[threadIdx.x] = n;
     __syncthreads();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nk) return;
-    const int f = freq[k];
-    double re = 0.0, im = 0.0;
-    int m = 0;
-    for (int c = 0; c < ncols; ++c) {
-        const double2 w = tw[m];
-        re = fma(row[c], w.x, re);
-        im = fma(row[c], w.y, im);
-        m += f;
-        if (m >= n) m -= n;
+    for (int w = kThreads / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w) {
+            part[threadIdx.x] += part[threadIdx.x + w];
+            count[threadIdx.x] += count[threadIdx.x + w];
+        }
+        __syncthreads();
     }
-    out[(int64_t)r * nk + k] = make_double2(re, im);
-}
-
-// Pass 2 at row frequency rf[u] for every column k of a (nrows x nk) matrix:
-// h = sum_r a[r][k] tw[(rf[u] r) mod n].  mode 0: bin |h| / norm by the
-// radius of (sf_u, sf_k); mode 1: acc[u][k] += |h|^2 (power accumulation).
-// grid (ceil(nk / kThreads), nu).
-__global__ void dft_cols_kernel(const double2 *__restrict__ a, int nrows, int nk, const int *__restrict__ rf,
-                                const int *__restrict__ sf_row, const int *__restrict__ sf_col,
-                                const double2 *__restrict__ tw, int n, int mode, double norm, int nbins,
-                                double *__restrict__ bin_sum, double *__restrict__ bin_cnt, double *__restrict__ acc)
-{
-    const int u = blockIdx.y;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nk) return;
-    const int f = rf[u];
-    double re = 0.0, im = 0.0;
-    int m = 0;
-    for (int r = 0; r < nrows; ++r) {
-        const double2 x = a[(int64_t)r * nk + k];
-        const double2 w = tw[m];
-        re = fma(x.x, w.x, fma(-x.y, w.y, re));
-        im = fma(x.x, w.y, fma(x.y, w.x, im));
-        m += f;
-        if (m >= n) m -= n;
-    }
-    if (mode == 1) {
-        acc[(int64_t)u * nk + k] += re * re + im * im;
-        return;
-    }
-    const double su = (double)sf_row[u], sk = (double)sf_col[k];
-    const int b = (int)llrint(sqrt(su * su + sk * sk));
-    if (b < nbins) {
-        atomicAdd(&bin_sum[b], sqrt(re * re + im * im) / norm);
-        atomicAdd(&bin_cnt[b], 1.0);
+    if (threadIdx.x == 0) {
+        const double v = count[0] > 0 ? part[0] / count[0] : 0.0;
+        out[b] = norm ? v / *norm : v;
     }
 }
 
-// Row and column sums of an image (the two line spread functions).
-__global__ void lsf_kernel(const double *__restrict__ img, int xdim, int ydim, double *__restrict__ lsf_x,
-                           double *__restrict__ lsf_y)
+// out[k] = |h(k, 0)| / total, out[n + k] = |h(0, k)| / total, out[2 n] = total
+// from the map of |h| (row frequency 0 at row `zero`): the transforms of the
+// two line spread functions (row and column sums).  total: the image's sum.
+__global__ void axes_kernel(const double *__restrict__ map, int nk, int zero, const double2 *__restrict__ a, int nrows,
+                            double *__restrict__ out)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < xdim) {
-        double s = 0.0;
-        for (int j = 0; j < ydim; ++j) s += img[(int64_t)t * ydim + j];
-        lsf_x[t] = s;
+    __shared__ double part[kThreads];
+    double s = 0.0;
+    for (int r = threadIdx.x; r < nrows; r += kThreads) s += a[(int64_t)r * nk].x;  // the rows' sums
+    part[threadIdx.x] = s;
+    __syncthreads();
+    for (int w = kThreads / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
+        __syncthreads();
     }
-    if (t < ydim) {
-        double s = 0.0;
-        for (int i = 0; i < xdim; ++i) s += img[(int64_t)i * ydim + t];
-        lsf_y[t] = s;
+    const double total = part[0];
+    for (int k = threadIdx.x; k < nk; k += kThreads) {
+        out[k] = map[(int64_t)(zero + k) * nk] / total;
+        out[nk + k] = map[(int64_t)zero * nk + k] / total;
     }
-}
-
-// |sum_i l[i] tw[(k i) mod n]| / norm for k < nk (one thread per k).
-__global__ void dft_1d_mag_kernel(const double *__restrict__ l, int len, int nk, const double2 *__restrict__ tw,
-                                  int n, double norm, double *__restrict__ out)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nk) return;
-    double re = 0.0, im = 0.0;
-    int m = 0;
-    for (int i = 0; i < len; ++i) {
-        const double2 w = tw[m];
-        re = fma(l[i], w.x, re);
-        im = fma(l[i], w.y, im);
-        m += k;
-        if (m >= n) m -= n;
-    }
-    out[k] = sqrt(re * re + im * im) / norm;
+    if (threadIdx.x == 0) out[2 * nk] = total;
 }
 
 // Per-pixel mean over n images (x n stacked images of `count` values).
@@ -138,61 +282,140 @@ __global__ void mean_images_kernel(const double *__restrict__ imgs, int n, int64
     }
 }
 
-__global__ void sub_kernel(const double *__restrict__ a, const double *__restrict__ b, int64_t count,
-                           double *__restrict__ out)
+// Sums of the regions of an image, a block per region.
+constexpr int kSumThreads = 1024;
+__global__ void __launch_bounds__(kSumThreads) region_sum_kernel(const __grid_constant__ Regions g,
+                                                              double *__restrict__ out)
 {
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < count; p += (int64_t)gridDim.x * blockDim.x)
-        out[p] = a[p] - b[p];
-}
-
-// Sum of an roi x roi region (one block).
-__global__ void region_sum_kernel(const double *__restrict__ img, int64_t ld, int x0, int y0, int roi,
-                                  double *__restrict__ out)
-{
-    __shared__ double part[kThreads];
+    __shared__ double part[kSumThreads];
+    const int q = blockIdx.x;
+    const double *img = g.img + (int64_t)(g.x0 + q / g.across * g.rows) * g.ld + g.y0 + q % g.across * g.cols;
     double s = 0.0;
-    for (int t = threadIdx.x; t < roi * roi; t += blockDim.x) s += img[(int64_t)(x0 + t / roi) * ld + y0 + t % roi];
+    for (int t = threadIdx.x; t < g.rows * g.cols; t += kSumThreads) s += img[(int64_t)(t / g.cols) * g.ld + t % g.cols];
     part[threadIdx.x] = s;
     __syncthreads();
-    for (int w = kThreads / 2; w > 0; w >>= 1) {
+    for (int w = kSumThreads / 2; w > 0; w >>= 1) {
         if (threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *out = part[0];
+    if (threadIdx.x == 0) out[q] = part[0];
 }
 
-// Radial binning of an n x n power map in unsigned DFT order.
-__global__ void bin_map_kernel(const double *__restrict__ map, int n, double scale, int nbins,
-                               double *__restrict__ bin_sum, double *__restrict__ bin_cnt, double *__restrict__ out2d)
+// The scaled power map of an n x n transform from its planes [n][nk] over
+// column frequencies 0..n/2: half[u][k] = scale sum_z planes[z][u][k], and the
+// full map in unsigned DFT order.  scale = factor / m^2 with the mean signal m
+// of the `regions` region sums, kept in *mean_signal.
+__global__ void power_map_kernel(const double *__restrict__ planes, int nplanes, int n, int nk,
+                                 const double *__restrict__ sums, int regions, double factor,
+                                 double *__restrict__ half, double *__restrict__ out2d,
+                                 double *__restrict__ mean_signal)
 {
+    double m = 0.0;
+    for (int q = 0; q < regions; ++q) m += sums[q];
+    m /= (double)regions * n * n;
+    const double scale = factor / (m * m);
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= (int64_t)n * n) return;
-    const int u = (int)(t / n), v = (int)(t % n);
-    const double val = map[t] * scale;
-    if (out2d) out2d[t] = val;
-    const double su = u <= n / 2 ? u : u - n, sv = v <= n / 2 ? v : v - n;
-    const int b = (int)llrint(sqrt(su * su + sv * sv));
-    if (b < nbins) {
-        atomicAdd(&bin_sum[b], val);
-        atomicAdd(&bin_cnt[b], 1.0);
-    }
+    if (t == 0) *mean_signal = m;
+    if (t >= (int64_t)n * nk) return;
+    double s = 0.0;
+    for (int z = 0; z < nplanes; ++z) s += planes[(int64_t)z * n * nk + t];
+    const double val = s * scale;
+    half[t] = val;
+    if (!out2d) return;
+    const int u = (int)(t / nk), k = (int)(t % nk);
+    out2d[(int64_t)u * n + k] = val;
+    if (k > 0 && 2 * k != n) out2d[(int64_t)((n - u) % n) * n + n - k] = val;
 }
 
-struct Dev {
-    std::vector<void *> ptrs;
-    cudaError_t err = cudaSuccess;
+// Offsets of a call's arrays in one device allocation.
+struct Layout {
+    size_t bytes = 0;
     template <typename T>
-    T *alloc(size_t n)
+    size_t add(size_t n)
     {
-        void *p = nullptr;
-        if (err == cudaSuccess) err = cudaMalloc(&p, sizeof(T) * std::max<size_t>(n, 1));
-        if (err == cudaSuccess) ptrs.push_back(p);
-        return (T *)p;
+        const size_t at = bytes;
+        bytes += (sizeof(T) * std::max<size_t>(n, 1) + 255) & ~(size_t)255;
+        return at;
     }
-    ~Dev()
+};
+
+// A call's device memory and stream.  One of each is kept per device between
+// calls (allocating and freeing them took 1 to 5 ms of a 501 x 501 MTF, its
+// kernels 0.12 ms): up to kKept bytes, for one call at a time.  A call that
+// needs more, or that runs beside another on the device, has its own.  The
+// kept ones are freed with the library.
+class Workspace {
+  public:
+    static constexpr size_t kKept = (size_t)128 << 20;
+
+    cudaError_t open(int device, size_t bytes)
     {
-        for (void *p : ptrs) cudaFree(p);
+        Kept &k = kept(device);
+        if (device < kDevices && bytes <= kKept && k.lock.try_lock()) {
+            held_ = &k;
+            if (k.stream) {
+                // a device reset took them away
+                const cudaError_t q = cudaStreamQuery(k.stream);
+                if (q != cudaSuccess && q != cudaErrorNotReady) {
+                    cudaGetLastError();
+                    k.stream = nullptr;
+                    k.base = nullptr;
+                    k.bytes = 0;
+                }
+            }
+            cudaError_t e = k.stream ? cudaSuccess : cudaStreamCreateWithFlags(&k.stream, cudaStreamNonBlocking);
+            if (e == cudaSuccess && k.bytes < bytes) {
+                if (k.base) cudaFree(k.base);
+                k.base = nullptr;
+                k.bytes = 0;
+                e = cudaMalloc((void **)&k.base, bytes);
+                if (e == cudaSuccess) k.bytes = bytes;
+            }
+            base = k.base;
+            stream = k.stream;
+            return e;
+        }
+        cudaError_t e = cudaMalloc((void **)&base, bytes);
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+        return e;
     }
+    template <typename T>
+    T *at(size_t offset) const
+    {
+        return reinterpret_cast<T *>(base + offset);
+    }
+    ~Workspace()
+    {
+        if (held_) {
+            if (stream) cudaStreamSynchronize(stream);  // after an error too: the next call finds it idle
+            held_->lock.unlock();
+            return;
+        }
+        if (stream) cudaStreamDestroy(stream);
+        if (base) cudaFree(base);
+    }
+    cudaStream_t stream = nullptr;
+
+  private:
+    static constexpr int kDevices = 16;
+    struct Kept {
+        std::mutex lock;
+        char *base = nullptr;
+        size_t bytes = 0;
+        cudaStream_t stream = nullptr;
+        ~Kept()
+        {
+            if (base) cudaFree(base);  // fails quietly when the runtime is gone already
+            if (stream) cudaStreamDestroy(stream);
+        }
+    };
+    static Kept &kept(int device)
+    {
+        static Kept k[kDevices];
+        return k[device < kDevices ? device : 0];
+    }
+    char *base = nullptr;
+    Kept *held_ = nullptr;
 };
 
 fd2_status to_status(cudaError_t e)
@@ -202,6 +425,8 @@ fd2_status to_status(cudaError_t e)
            : (e == cudaErrorNoDevice || e == cudaErrorInvalidDevice) ? FD2_ERR_NO_DEVICE
                                                                       : FD2_ERR_CUDA;
 }
+
+unsigned tiles(int64_t n, int tile) { return (unsigned)((n + tile - 1) / tile); }
 
 unsigned blocks_for(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + kThreads - 1) / kThreads, 1 << 20)); }
 
@@ -216,63 +441,51 @@ fd2_status fd2_mtf(int32_t device, const double *image, int32_t xdim, int32_t yd
         return FD2_ERR_INVALID_ARGUMENT;
     const int N = std::max(xdim, ydim);
     if (n_freq > N / 2 + 1) return FD2_ERR_INVALID_ARGUMENT;
-    double total = 0.0;
-    for (int64_t p = 0; p < (int64_t)xdim * ydim; ++p) total += image[p];
-    if (!(total > 0.0) || !std::isfinite(total)) return FD2_ERR_INVALID_ARGUMENT;
     if (freq_per_mm)
         for (int k = 0; k < n_freq; ++k) freq_per_mm[k] = 1000.0 * k / (N * pixel_um);
-    cudaError_t e = cudaSetDevice(device);
-    if (e != cudaSuccess) return to_status(e);
-    Dev d;
-    cudaStream_t s = nullptr;
     const int64_t npx = (int64_t)xdim * ydim;
+    cudaError_t e = cudaSetDevice(device);
+    if (e != cudaSuccess) {
+        // an image without signal is refused whatever the device
+        double total = 0.0;
+        for (int64_t p = 0; p < npx; ++p) total += image[p];
+        return !(total > 0.0) || !std::isfinite(total) ? FD2_ERR_INVALID_ARGUMENT : to_status(e);
+    }
     const int K = n_freq, V = 2 * K - 1;
-    double *d_img = d.alloc<double>((size_t)npx);
-    double2 *d_tw = d.alloc<double2>((size_t)N);
-    double *d_lx = d.alloc<double>((size_t)xdim), *d_ly = d.alloc<double>((size_t)ydim);
-    double *d_mx = d.alloc<double>((size_t)K), *d_my = d.alloc<double>((size_t)K);
-    int *d_f = d.alloc<int>((size_t)V), *d_sf = d.alloc<int>((size_t)V);
-    double2 *d_a = d.alloc<double2>((size_t)xdim * V);
-    double *d_bs = d.alloc<double>((size_t)K), *d_bc = d.alloc<double>((size_t)K);
-    if (d.err == cudaSuccess) d.err = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-    if (d.err != cudaSuccess) return to_status(d.err);
-    std::vector<int> f(V), sf(V);
-    for (int t = 0; t < V; ++t) {
-        sf[t] = t - (K - 1);               // signed frequency index
-        f[t] = ((sf[t] % N) + N) % N;      // its phase step mod N
-    }
-    e = cudaMemcpyAsync(d_img, image, sizeof(double) * npx, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_f, f.data(), sizeof(int) * V, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_sf, sf.data(), sizeof(int) * V, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_bs, 0, sizeof(double) * K, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_bc, 0, sizeof(double) * K, s);
+    Layout l;
+    Workspace d;
+    const size_t o_img = l.add<double>((size_t)npx), o_tw = l.add<double2>((size_t)N);
+    const size_t o_a = l.add<double2>((size_t)xdim * K), o_map = l.add<double>((size_t)V * K);
+    const size_t o_out = l.add<double>(3 * (size_t)K + 1);
+    if ((e = d.open(device, l.bytes)) != cudaSuccess) return to_status(e);
+    const cudaStream_t s = d.stream;
+    double2 *tw = d.at<double2>(o_tw), *a = d.at<double2>(o_a);
+    // out: mtf_x, mtf_y, the image's sum, mtf_r
+    double *map = d.at<double>(o_map), *out = d.at<double>(o_out);
+    e = cudaMemcpyAsync(d.at<double>(o_img), image, sizeof(double) * npx, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
-        twiddle_kernel<<<blocks_for(N), kThreads, 0, s>>>(N, d_tw);
-        lsf_kernel<<<blocks_for(N), kThreads, 0, s>>>(d_img, xdim, ydim, d_lx, d_ly);
-        dft_1d_mag_kernel<<<blocks_for(K), kThreads, 0, s>>>(d_lx, xdim, K, d_tw, N, total, d_mx);
-        dft_1d_mag_kernel<<<blocks_for(K), kThreads, 0, s>>>(d_ly, ydim, K, d_tw, N, total, d_my);
-        if (mtf_r) {
-            const size_t sm = sizeof(double) * (size_t)ydim;
-            if (sm > 48 * 1024) e = cudaFuncSetAttribute(dft_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            if (e == cudaSuccess) {
-                dft_rows_kernel<<<dim3(blocks_for(V), (unsigned)xdim), kThreads, sm, s>>>(d_img, ydim, 0, 0, ydim, 0.0,
-                                                                                          d_f, V, d_tw, N, d_a);
-                dft_cols_kernel<<<dim3(blocks_for(V), (unsigned)V), kThreads, 0, s>>>(
-                    d_a, xdim, V, d_f, d_sf, d_sf, d_tw, N, 0, total, K, d_bs, d_bc, nullptr);
-            }
-        }
-        if (e == cudaSuccess) e = cudaGetLastError();
+        const Regions g{d.at<double>(o_img), ydim, npx, 0, 0, xdim, ydim, 1, 1, nullptr, nullptr};
+        twiddle_kernel<<<blocks_for(N), kThreads, 0, s>>>(N, tw);
+        dft_rows_kernel<<<dim3(tiles(xdim, kRowTile), tiles(K, kFreqs)), kThreads, 0, s>>>(g, 0, K, tw, N, a);
+        dft_cols_kernel<<<dim3(tiles(K, kColTile), tiles(V, kFreqs)), kThreads, 0, s>>>(a, 1, xdim, K, V, 1 - K, tw, N,
+                                                                                      0, map);
+        axes_kernel<<<1, kThreads, 0, s>>>(map, K, K - 1, a, xdim, out);
+        if (mtf_r)
+            radial_kernel<<<(unsigned)K, kThreads, 0, s>>>(map, V, K, 1 - K, 0, -1, out + 2 * K, out + 2 * K + 1);
+        e = cudaGetLastError();
     }
-    std::vector<double> bs(K), bc(K);
-    if (e == cudaSuccess && mtf_x) e = cudaMemcpyAsync(mtf_x, d_mx, sizeof(double) * K, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && mtf_y) e = cudaMemcpyAsync(mtf_y, d_my, sizeof(double) * K, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && mtf_r) e = cudaMemcpyAsync(bs.data(), d_bs, sizeof(double) * K, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && mtf_r) e = cudaMemcpyAsync(bc.data(), d_bc, sizeof(double) * K, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaStreamDestroy(s);
+    std::vector<double> r(3 * (size_t)K + 1);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(r.data(), out, sizeof(double) * (mtf_r ? r.size() : 2 * (size_t)K + 1),
+                            cudaMemcpyDeviceToHost, s);
+    const cudaError_t e2 = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = e2;
     if (e != cudaSuccess) return to_status(e);
-    if (mtf_r)
-        for (int k = 0; k < K; ++k) mtf_r[k] = bc[k] > 0.0 ? bs[k] / bc[k] : 0.0;
+    const double total = r[2 * (size_t)K];
+    if (!(total > 0.0) || !std::isfinite(total)) return FD2_ERR_INVALID_ARGUMENT;
+    if (mtf_x) std::copy(r.begin(), r.begin() + K, mtf_x);
+    if (mtf_y) std::copy(r.begin() + K, r.begin() + 2 * K, mtf_y);
+    if (mtf_r) std::copy(r.begin() + 2 * K + 1, r.end(), mtf_r);
     return FD2_OK;
 }
 
@@ -288,86 +501,74 @@ fd2_status fd2_nnps(int32_t device, const double *images, int32_t n_images, int3
         for (int k = 0; k < n_freq; ++k) freq_per_mm[k] = 1000.0 * k / (roi * pixel_um);
     cudaError_t e = cudaSetDevice(device);
     if (e != cudaSuccess) return to_status(e);
-    Dev d;
-    cudaStream_t s = nullptr;
-    const int64_t npx = (int64_t)xdim * ydim;
-    const int R = roi, K = n_freq, n = n_images;
-    double *d_imgs = d.alloc<double>((size_t)(npx * n));
-    double *d_mean = d.alloc<double>((size_t)npx);
-    double *d_diff = d.alloc<double>((size_t)npx);
-    double2 *d_tw = d.alloc<double2>((size_t)R);
-    int *d_f = d.alloc<int>((size_t)R);
-    double2 *d_a = d.alloc<double2>((size_t)R * R);
-    double *d_acc = d.alloc<double>((size_t)R * R);
-    double *d_sums = d.alloc<double>((size_t)rois_x * rois_y * (n + 1));
-    double *d_bs = d.alloc<double>((size_t)K), *d_bc = d.alloc<double>((size_t)K);
-    double *d_2d = nnps_2d ? d.alloc<double>((size_t)R * R) : nullptr;
-    if (d.err == cudaSuccess) d.err = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-    if (d.err != cudaSuccess) return to_status(d.err);
-    std::vector<int> f(R);
-    for (int t = 0; t < R; ++t) f[t] = t;
-    e = cudaMemcpyAsync(d_imgs, images, sizeof(double) * npx * n, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_f, f.data(), sizeof(int) * R, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_acc, 0, sizeof(double) * R * R, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_bs, 0, sizeof(double) * K, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_bc, 0, sizeof(double) * K, s);
-    const int nroi = rois_x * rois_y;
-    const size_t sm = sizeof(double) * (size_t)R;
-    if (e == cudaSuccess && sm > 48 * 1024)
-        e = cudaFuncSetAttribute(dft_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const int R = roi, K = n_freq, n = n_images, H = R / 2 + 1, nroi = rois_x * rois_y;
+    // regions of all images are transformed together, as many at a time as fit
+    // 128 MiB; pass 2 sums their power in `planes` planes, so that blocks share
+    // the regions of small maps
+    const int64_t all = (int64_t)n * nroi, per_region = (int64_t)R * H;
+    const int batch = (int)std::max<int64_t>(1, std::min<int64_t>({all, 65535, (128ll << 20) / (16 * per_region)}));
+    const unsigned tiles2 = tiles(H, kColTile) * tiles(R, kFreqs);
+    const int planes = (int)std::max<int64_t>(1, std::min<int64_t>(batch, 1184 / tiles2));
+    Layout l;
+    Workspace d;
+    // only the regions' pixels are copied
+    const int wx = rois_x * R, wy = rois_y * R;
+    const int64_t npx = (int64_t)wx * wy;
+    const size_t o_imgs = l.add<double>((size_t)(npx * n)), o_mean = l.add<double>((size_t)npx);
+    const size_t o_tw = l.add<double2>((size_t)R), o_a = l.add<double2>((size_t)(per_region * batch));
+    const size_t o_planes = l.add<double>((size_t)(per_region * planes)), o_half = l.add<double>((size_t)per_region);
+    const size_t o_sums = l.add<double>((size_t)nroi), o_out = l.add<double>((size_t)K + 1);
+    const size_t o_2d = nnps_2d ? l.add<double>((size_t)R * R) : 0;
+    if ((e = d.open(device, l.bytes)) != cudaSuccess) return to_status(e);
+    const cudaStream_t s = d.stream;
+    double *imgs = d.at<double>(o_imgs), *mean = d.at<double>(o_mean), *sums = d.at<double>(o_sums);
+    double *acc = d.at<double>(o_planes), *half = d.at<double>(o_half), *out = d.at<double>(o_out);
+    double *out2d = nnps_2d ? d.at<double>(o_2d) : nullptr;
+    double2 *tw = d.at<double2>(o_tw), *a = d.at<double2>(o_a);
+    for (int i = 0; e == cudaSuccess && i < n; ++i)
+        e = cudaMemcpy2DAsync(imgs + i * npx, sizeof(double) * wy, images + ((int64_t)i * xdim + x0) * ydim + y0,
+                              sizeof(double) * ydim, sizeof(double) * wy, (size_t)wx, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(acc, 0, sizeof(double) * per_region * planes, s);
     if (e == cudaSuccess) {
-        twiddle_kernel<<<blocks_for(R), kThreads, 0, s>>>(R, d_tw);
-        mean_images_kernel<<<blocks_for(npx), kThreads, 0, s>>>(d_imgs, n, npx, d_mean);
-        // region sums of the mean image (signal) and, with one image, of the image (its mean)
-        for (int q = 0; q < nroi; ++q)
-            region_sum_kernel<<<1, kThreads, 0, s>>>(d_mean, ydim, x0 + (q / rois_y) * R, y0 + (q % rois_y) * R, R,
-                                                     d_sums + q);
-        e = cudaGetLastError();
-    }
-    std::vector<double> sums((size_t)nroi);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(sums.data(), d_sums, sizeof(double) * nroi, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    double m = 0.0;
-    for (double v : sums) m += v;
-    m /= (double)nroi * R * R;
-    if (e == cudaSuccess && !(m > 0.0)) e = cudaErrorInvalidValue;
-    for (int r = 0; e == cudaSuccess && r < n; ++r) {
-        const double *src = d_imgs + (int64_t)r * npx;
+        Regions g{imgs, wy, npx, 0, 0, R, R, rois_y, nroi, nullptr, nullptr}, gm = g;
+        twiddle_kernel<<<blocks_for(R), kThreads, 0, s>>>(R, tw);
         if (n > 1) {
-            sub_kernel<<<blocks_for(npx), kThreads, 0, s>>>(src, d_mean, npx, d_diff);
-            src = d_diff;
+            mean_images_kernel<<<blocks_for(npx), kThreads, 0, s>>>(imgs, n, npx, mean);
+            gm.img = g.mean = mean;
+        } else {
+            g.sums = sums;  // one image: each region's own mean is subtracted
         }
-        for (int q = 0; q < nroi && e == cudaSuccess; ++q) {
-            const int rx = x0 + (q / rois_y) * R, ry = y0 + (q % rois_y) * R;
-            // one image: subtract the region's mean (the mean image is the image)
-            const double sub = n > 1 ? 0.0 : sums[(size_t)q] / ((double)R * R);
-            dft_rows_kernel<<<dim3(blocks_for(R), (unsigned)R), kThreads, sm, s>>>(src, ydim, rx, ry, R, sub, d_f, R,
-                                                                                  d_tw, R, d_a);
-            dft_cols_kernel<<<dim3(blocks_for(R), (unsigned)R), kThreads, 0, s>>>(d_a, R, R, d_f, nullptr, nullptr,
-                                                                                  d_tw, R, 1, 1.0, 0, nullptr,
-                                                                                  nullptr, d_acc);
-            e = cudaGetLastError();
+        // region sums of the mean image (the signal)
+        region_sum_kernel<<<(unsigned)nroi, kSumThreads, 0, s>>>(gm, sums);
+        for (int64_t first = 0; first < all; first += batch) {
+            const int m = (int)std::min<int64_t>(batch, all - first);
+            dft_rows_kernel<<<dim3(tiles(R, kRowTile), tiles(H, kFreqs), (unsigned)m), kThreads, 0, s>>>(
+                g, (int)first, H, tw, R, a);
+            dft_cols_kernel<<<dim3(tiles(H, kColTile), tiles(R, kFreqs), (unsigned)planes), kThreads, 0, s>>>(
+                a, m, R, H, R, 0, tw, R, 1, acc);
         }
-    }
-    // NNPS = pixel^2 (mm^2) / roi^2 * <|F|^2> * n/(n-1) / m^2
-    const double px_mm = pixel_um / 1000.0;
-    const double corr = n > 1 ? (double)n / (double)(n - 1) : 1.0;
-    const double scale = px_mm * px_mm / ((double)R * R) * corr / ((double)n * nroi) / (m * m);
-    if (e == cudaSuccess) {
-        bin_map_kernel<<<blocks_for((int64_t)R * R), kThreads, 0, s>>>(d_acc, R, scale, K, d_bs, d_bc, d_2d);
+        // NNPS = pixel^2 (mm^2) / roi^2 * <|F|^2> * n/(n-1) / m^2
+        const double px_mm = pixel_um / 1000.0;
+        const double corr = n > 1 ? (double)n / (double)(n - 1) : 1.0;
+        const double factor = px_mm * px_mm / ((double)R * R) * corr / ((double)n * nroi);
+        power_map_kernel<<<blocks_for(per_region), kThreads, 0, s>>>(acc, planes, R, H, sums, nroi, factor, half,
+                                                                     out2d, out + K);
+        radial_kernel<<<(unsigned)K, kThreads, 0, s>>>(half, R, H, 0, R, R % 2 == 0 ? R / 2 : -1, nullptr, out);
         e = cudaGetLastError();
     }
-    std::vector<double> bs(K), bc(K);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(bs.data(), d_bs, sizeof(double) * K, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(bc.data(), d_bc, sizeof(double) * K, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && nnps_2d)
-        e = cudaMemcpyAsync(nnps_2d, d_2d, sizeof(double) * R * R, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaStreamDestroy(s);
-    if (e == cudaErrorInvalidValue && !(m > 0.0)) return FD2_ERR_INVALID_ARGUMENT;
+    std::vector<double> r((size_t)K + 1);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(r.data(), out, sizeof(double) * r.size(), cudaMemcpyDeviceToHost, s);
+    cudaError_t e2 = cudaStreamSynchronize(s);
+    const double m = r[(size_t)K];
+    const bool signal = e == cudaSuccess && e2 == cudaSuccess && m > 0.0;
+    if (signal && nnps_2d) {
+        e = cudaMemcpyAsync(nnps_2d, out2d, sizeof(double) * R * R, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    }
+    if (e == cudaSuccess) e = e2;
     if (e != cudaSuccess) return to_status(e);
-    if (nnps_r)
-        for (int k = 0; k < K; ++k) nnps_r[k] = bc[k] > 0.0 ? bs[k] / bc[k] : 0.0;
+    if (!signal) return FD2_ERR_INVALID_ARGUMENT;
+    if (nnps_r) std::copy(r.begin(), r.begin() + K, nnps_r);
     if (mean_signal) *mean_signal = m;
     return FD2_OK;
 }

@@ -1,0 +1,31 @@
+"""Loss and gradients of the training step where its kernels' tiles end: rows
+around a warp's, a block's and a 256-row slice's, categories around a pass of
+31, points without a radial label, against the numpy oracle."""
+import numpy as np
+import pytest
+
+import hybridmantis_b200.surrogate as sgm
+from oracle import sg_oracle as so
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,bins", [(1, 96), (3, 30), (4, 31), (5, 32), (31, 61), (64, 62), (65, 63), (255, 1),
+                                       (257, 96), (513, 130)])
+def test_loss_and_gradient_at_tile_edges(require_gpu, rows, bins):
+    rng = np.random.default_rng(rows)
+    f = rng.uniform(-1, 1, (rows, 8)).astype(np.float32)
+    ph = np.full(rows, 1000, np.int32)
+    det = rng.integers(0, 1001, rows).astype(np.int32)
+    rad = rng.integers(0, 40, (rows, bins + 1)).astype(np.uint32)
+    rad[:, bins // 2:] *= rng.integers(0, 2, (rows, bins + 1 - bins // 2)).astype(np.uint32)
+    rad[::5] = 0  # no radial label
+    with sgm.Surrogate(hidden=64, radial_bins=bins, radial_max_um=200.0, batch=640) as s:
+        s.set_hull(np.full(8, -1.0), np.full(8, 1.0))
+        loss, g = s.loss_grad(f, ph, det, rad)
+        want, wg = so.loss_grad(s.params(), 64, f, np.full(8, -1.0), np.full(8, 1.0), ph, det, rad, bins, 200.0)
+    # FP32 sums of up to 131 categories and 513 rows of terms of mixed sign
+    # beside FP64 ones: 1e-4 of the gradient's norm (BF16 roundings that fall
+    # the other way are 2^-9 of single entries)
+    assert loss == pytest.approx(want, rel=1e-5)
+    assert np.linalg.norm(g - wg) <= 2e-3 * np.linalg.norm(wg)
