@@ -419,10 +419,18 @@ __global__ void __launch_bounds__(256) transpose_bf16_kernel(const __grid_consta
 }
 
 // Normalised inputs of host-given feature rows.
-__global__ void input_kernel(const float *__restrict__ feat, int64_t n, NormParams norm, __nv_bfloat16 *__restrict__ x0)
+__global__ void input_kernel(const float *__restrict__ feat, int64_t n, const __grid_constant__ NormParams norm, __nv_bfloat16 *__restrict__ x0)
 {
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
         write_input(feat + r * kFeatures, norm.lo, norm.inv, x0 + r * kInPad);
+}
+
+// The network's outputs without the padding of their rows: out[r][k] =
+// in[r][k], k < kOutputs, in [rows][kOutPad].
+__global__ void pack_outputs_kernel(const float *__restrict__ in, int64_t n, float *__restrict__ out)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n * kOutputs; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = in[i / kOutputs * kOutPad + i % kOutputs];
 }
 
 }  // namespace sg
@@ -1136,7 +1144,8 @@ void fd2_sg_destroy(fd2_sg *s)
                     (void *)s->d_step, (void *)s->d_acc, (void *)s->d_lr, (void *)s->ws, (void *)s->x0, (void *)s->h1, (void *)s->h2,
                     (void *)s->h3, (void *)s->d1, (void *)s->d2, (void *)s->d3, (void *)s->out, (void *)s->dout,
                     (void *)s->target, (void *)s->has_rad, (void *)s->ylab, (void *)s->d_feat, (void *)s->d_photons,
-                    (void *)s->d_detected, (void *)s->d_radial, (void *)s->d_tc_fault, (void *)s->pbT, (void *)s->tA,
+                    (void *)s->d_detected, (void *)s->d_radial, (void *)s->d_tc_fault, (void *)s->pbT, (void *)s->pf, (void *)s->px,
+                    (void *)s->pha, (void *)s->phb, (void *)s->pout, (void *)s->ppack, (void *)s->tA,
                     (void *)s->tB})
         if (p) cudaFree(p);
     sg_free_run_buffers(s);
@@ -1383,28 +1392,42 @@ fd2_status fd2_sg_predict(fd2_sg *s, const float *features, int64_t n, float *ou
     if (!s || !features || !out || n < 0) return FD2_ERR_INVALID_ARGUMENT;
     if (n == 0) return FD2_OK;
     SG_CUDA(s, cudaSetDevice(s->device));
-    fd2_status st = ensure_rows(s, s->batch);
-    if (st != FD2_OK) return st;
-    float *df = nullptr;
-    SG_CUDA(s, cudaMalloc(&df, sizeof(float) * (size_t)std::min<int64_t>(n, s->batch) * kFeatures));
-    std::vector<float> o((size_t)s->batch * kOutPad);
+    // up to kPredictRows rows a pass (fewer with wider layers): enough tiles for
+    // every SM, where the training batch's 8,192 rows are 64.  The outputs leave
+    // the device packed, straight into the caller's array (50,001 rows: seven
+    // batches of padded rows, each waited for and unpadded on the host, 2.5 ms;
+    // one pass 0.9)
+    const int64_t most = std::min<int64_t>(kPredictRows, ((int64_t)kPredictRows * 256) / s->hidden);
+    const int64_t cap = std::min(n, most);
+    if (cap > s->predict_cap) {
+        const size_t C = (size_t)cap, H = (size_t)s->hidden;
+        s->predict_cap = 0;
+        SG_CUDA(s, alloc(&s->pf, C * kFeatures));
+        SG_CUDA(s, alloc(&s->px, C * kInPad));
+        SG_CUDA(s, alloc(&s->pha, C * H));
+        SG_CUDA(s, alloc(&s->phb, C * H));
+        SG_CUDA(s, alloc(&s->pout, C * kOutPad));
+        SG_CUDA(s, alloc(&s->ppack, C * kOutputs));
+        s->predict_cap = cap;
+    }
     cudaError_t e = cudaSuccess;
-    for (int64_t at = 0; at < n && e == cudaSuccess; at += s->batch) {
-        const int b = (int)std::min<int64_t>(s->batch, n - at);
-        e = cudaMemcpyAsync(df, features + at * kFeatures, sizeof(float) * b * kFeatures, cudaMemcpyHostToDevice,
+    for (int64_t at = 0; at < n && e == cudaSuccess; at += most) {
+        const int b = (int)std::min<int64_t>(most, n - at);
+        e = cudaMemcpyAsync(s->pf, features + at * kFeatures, sizeof(float) * b * kFeatures, cudaMemcpyHostToDevice,
                             s->stream);
         if (e != cudaSuccess) break;
-        input_kernel<<<grid_for(b, 256), 256, 0, s->stream>>>(df, b, s->norm, s->x0);
-        e = sg_forward(s, s->stream, s->x0, b, nullptr, s->h1, s->h2, s->h3, s->out);
+        input_kernel<<<grid_for(b, 256), 256, 0, s->stream>>>(s->pf, b, s->norm, s->px);
+        e = sg_forward(s, s->stream, s->px, b, nullptr, s->pha, s->phb, s->pha, s->pout);
+        if (e != cudaSuccess) break;
+        pack_outputs_kernel<<<grid_for((int64_t)b * kOutputs, 256), 256, 0, s->stream>>>(s->pout, b, s->ppack);
+        e = cudaGetLastError();
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(o.data(), s->out, sizeof(float) * b * kOutPad, cudaMemcpyDeviceToHost, s->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-        if (e == cudaSuccess)
-            for (int r = 0; r < b; ++r)
-                for (int k = 0; k < kOutputs; ++k) out[(at + r) * kOutputs + k] = o[(size_t)r * kOutPad + k];
+            e = cudaMemcpyAsync(out + at * kOutputs, s->ppack, sizeof(float) * b * kOutputs, cudaMemcpyDeviceToHost,
+                                s->stream);
     }
-    cudaFree(df);
+    const cudaError_t e2 = cudaStreamSynchronize(s->stream);
     SG_CUDA(s, e);
+    SG_CUDA(s, e2);
     return sg_tc_check(s);
 }
 
