@@ -59,6 +59,7 @@ struct fd2_ctx {
     uint32_t *d_radial = nullptr;  // label mode: [n_prim][radial_bins + 1]
     int64_t radial_len = 0;
     double *d_distance = nullptr, *d_moments = nullptr;
+    double *d_sums = nullptr;     // coordinate and energy sums of a device submission
 
     // abort flag in mapped host memory
     int *h_abort = nullptr, *d_abort = nullptr;

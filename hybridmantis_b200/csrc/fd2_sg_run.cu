@@ -233,23 +233,35 @@ struct LaneRng {
 // u picks the region.  All three come from one Box-Muller pair: rho =
 // sqrt(-2 ln u1) is the Rayleigh, rho |cos(2 pi u2)| the half-normal, and its
 // negative, kept when it is >= t0 and passes the thinning, the third region
-// (retried with fresh draws otherwise), so the regions share their costly part.
-__device__ __forceinline__ float ring_radius(float mu, float sd, float S, float u, LaneRng &rng)
+// (tried again with fresh draws otherwise), so the regions share their costly
+// part.  One attempt; false: not accepted.
+enum { kHalfNormal, kRayleigh, kInner };
+
+__device__ __forceinline__ int ring_region(float mu, float sd, float S, float u)
 {
     const float m1 = 0.5f * mu, m2 = sd * 0.3989422804014327f;
     const float x = u * S;
     const bool rayleigh = x >= m1 && (x < m1 + m2 || mu <= 0.0f);
-    const bool upper = x < m1;
-    const float t0 = -mu / sd;
-    for (uint32_t k = 0; k < 64; ++k) {
-        const float rho = sqrtf(-2.0f * logf(rng.u()));
-        if (rayleigh) return mu + sd * rho;
-        const float z = rho * fabsf(__cosf(6.283185307179586f * rng.u()));
-        if (upper) return mu + sd * z;
-        if (-z >= t0 && rng.u() <= 1.0f - sd * z / mu) return fmaxf(mu - sd * z, 0.0f);
-    }
-    return 0.5f * mu;  // not reached in practice
+    return rayleigh ? kRayleigh : x < m1 ? kHalfNormal : kInner;
 }
+
+__device__ __forceinline__ bool ring_radius(int region, float mu, float sd, LaneRng &rng, float &rad)
+{
+    const float rho = sqrtf(-2.0f * logf(rng.u()));
+    if (region == kRayleigh) {
+        rad = mu + sd * rho;
+        return true;
+    }
+    const float z = rho * fabsf(__cosf(6.283185307179586f * rng.u()));
+    if (region == kHalfNormal) {
+        rad = mu + sd * z;
+        return true;
+    }
+    rad = fmaxf(mu - sd * z, 0.0f);
+    return -z >= -mu / sd && rng.u() <= 1.0f - sd * z / mu;
+}
+
+constexpr int kRadiusTries = 64, kAzimuthTries = 32;  // then the ring's half radius, the last azimuth
 
 // Detected photons of one row and their PRF pixels; one warp per row, the
 // warps taking rows from a counter in batches, so that rows of very
@@ -257,7 +269,7 @@ __device__ __forceinline__ float ring_radius(float mu, float sd, float S, float 
 __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SampleArgs a)
 {
     const int lane = threadIdx.x & 31;
-    __shared__ float s_mix[kSampleThreads / 32][4][kComponents];
+    __shared__ __align__(16) float s_mix[kSampleThreads / 32][4][kComponents];
     float(*mix)[kComponents] = s_mix[threadIdx.x >> 5];
     const int rows = *a.count;
     const uint32_t run = *a.run_tag;
@@ -335,62 +347,105 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SampleArgs
         // the event's mixture in the warp's shared-memory table (every lane
         // draws from the same one; an indexed table in registers would go to
         // local memory): cumulative weight, mu, sd and normaliser per ring
+        // (decode_mix, a component per lane: all lanes decoding all of them was
+        // a third of the kernel's thread instructions)
         {
-            Mix m;
-            decode_mix(o, m);
-            float acc = 0.0f;
-            __syncwarp();  // the previous event's photons are placed
+            const int c = lane % kComponents;
+            const float w0 = o[1 + c], om = o[1 + kComponents + c], ls = o[1 + 2 * kComponents + c];
+            float top = w0;
 #pragma unroll
-            for (int c = 0; c < kComponents; ++c) {
-                acc += m.w[c];
-                if (lane == c) {
-                    mix[0][c] = c == kComponents - 1 ? 2.0f : acc;
-                    mix[1][c] = m.mu[c];
-                    mix[2][c] = m.sd[c];
-                    mix[3][c] = m.S[c];
-                }
+            for (int d = kComponents / 2; d > 0; d >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, d));
+            const float ew = expf(w0 - top);
+            float s = 0.0f;
+#pragma unroll
+            for (int k = 0; k < kComponents; ++k) s += __shfl_sync(0xffffffffu, ew, k);
+            const float w = ew / s;
+            float acc = 0.0f;  // the weights up to the lane's, added in order
+#pragma unroll
+            for (int k = 0; k < kComponents; ++k) {
+                const float v = __shfl_sync(0xffffffffu, w, k);
+                acc = k <= c ? acc + v : acc;
+            }
+            const float mu = kMuScale * (fmaxf(om, 0.0f) + log1pf(expf(-fabsf(om))));
+            const float sd = kSdScale * expf(fminf(fmaxf(ls, kLogSdMin), kLogSdMax));
+            const float t0 = -mu / sd;
+            const float S = fmaxf(mu * normcdff(-t0) + sd * norm_pdf(t0), 1e-30f);
+            __syncwarp();  // the previous event's photons are placed
+            if (lane < kComponents) {
+                mix[0][c] = c == kComponents - 1 ? 2.0f : acc;
+                mix[1][c] = mu;
+                mix[2][c] = sd;
+                mix[3][c] = S;
             }
             __syncwarp();
         }
+        // the cumulative weights, the same for all lanes
+        const float4 cw0 = *reinterpret_cast<const float4 *>(&mix[0][0]);
+        const float4 cw1 = *reinterpret_cast<const float4 *>(&mix[0][4]);
         int32_t in_prf = 0;
         // a power-of-two pixel divides exactly as a multiplication by its
         // reciprocal (the same correctly rounded quotient)
         const bool pow2 = (__float_as_uint(g.pixel) & 0x7fffffu) == 0u && g.pixel > 0.0f;
         const float inv_pixel = 1.0f / g.pixel;
-        for (int32_t i = lane; i < total; i += 32) {
-            // the component: the first whose cumulative weight exceeds u,
-            // i.e. the number of cumulative weights <= u (they do not
-            // decrease), counted without a data-dependent loop
-            const float u = rng.u();
-            int c = 0;
-#pragma unroll
-            for (int j = 0; j < kComponents - 1; ++j) c += u >= mix[0][j] ? 1 : 0;
-            const float ur = rng.u();
-            const float rad = ring_radius(mix[1][c], mix[2][c], mix[3][c], ur, rng);
-            float sn, cs;
-            sincospif(2.0f * rng.u(), &sn, &cs);
-            for (uint32_t k = 0; k < 32; ++k) {
-                const float tx = pos.x + rad * cs, ty = pos.y + rad * sn;
-                bool ok = tx >= 0.0f && tx <= g.xdet && ty >= 0.0f && ty <= g.ydet;
-                if (ok && a.edge_amp > 0.0f) {
-                    const float W = (1.0f - a.edge_amp * __expf(-tx * a.edge_inv_len)) *
-                                    (1.0f - a.edge_amp * __expf(-(g.xdet - tx) * a.edge_inv_len)) *
-                                    (1.0f - a.edge_amp * __expf(-ty * a.edge_inv_len)) *
-                                    (1.0f - a.edge_amp * __expf(-(g.ydet - ty) * a.edge_inv_len));
-                    ok = rng.u() < W;
+        // Every pass of the loop is one attempt at a radius and, where the lane
+        // has one, at an azimuth: a lane that has to try again does so beside
+        // the others' next photons (its draws keep their order: the lane's
+        // stream is its own).  Retrying in place ran the logarithm, sine and
+        // exponentials again for one or two lanes of the warp.
+        int region = 0, tries = 0;
+        float rad = 0.0f, mu = 0.0f, sd = 1.0f;
+        enum { kNew, kRadius, kAzimuth } stage = kNew;
+        for (int32_t i = lane; i < total;) {
+            if (stage != kAzimuth) {
+                if (stage == kNew) {
+                    // the component: the first whose cumulative weight exceeds
+                    // u, i.e. the number of cumulative weights <= u (they do
+                    // not decrease), counted without a data-dependent loop
+                    const float u = rng.u();
+                    const int c = (u >= cw0.x) + (u >= cw0.y) + (u >= cw0.z) + (u >= cw0.w) + (u >= cw1.x) +
+                                  (u >= cw1.y) + (u >= cw1.z);
+                    mu = mix[1][c];
+                    sd = mix[2][c];
+                    region = ring_region(mu, sd, mix[3][c], rng.u());
+                    tries = 0;
                 }
-                if (ok) break;
-                sincospif(2.0f * rng.u(), &sn, &cs);
+                bool ok = ring_radius(region, mu, sd, rng, rad);
+                if (!ok && ++tries == kRadiusTries) {
+                    rad = 0.5f * mu;  // not reached in practice
+                    ok = true;
+                }
+                stage = ok ? kAzimuth : kRadius;
+                tries = ok ? 0 : tries;
             }
-            const float x = pos.x + rad * cs, y = pos.y + rad * sn;
-            if (x <= g.ub_x && y <= g.ub_y && x >= g.lb_x && y >= g.lb_y) {
-                const float qx = pow2 ? __fmul_rn(x - g.lb_x, inv_pixel) : __fdiv_rn(x - g.lb_x, g.pixel);
-                const float qy = pow2 ? __fmul_rn(y - g.lb_y, inv_pixel) : __fdiv_rn(y - g.lb_y, g.pixel);
-                const int ii = (int)floorf(qx);
-                const int jj = (int)floorf(qy);
-                if (ii >= 0 && jj >= 0 && ii < g.xdim && jj < g.ydim) {
-                    atomicAdd(&a.prf[g.prf_offset + (long long)ii * g.ydim + jj], 1ull);
-                    ++in_prf;
+            if (stage == kAzimuth) {
+                float sn, cs;
+                sincospif(2.0f * rng.u(), &sn, &cs);
+                const float x = pos.x + rad * cs, y = pos.y + rad * sn;
+                bool ok = tries == kAzimuthTries;
+                if (!ok) {
+                    ok = x >= 0.0f && x <= g.xdet && y >= 0.0f && y <= g.ydet;
+                    if (ok && a.edge_amp > 0.0f) {
+                        const float W = (1.0f - a.edge_amp * __expf(-x * a.edge_inv_len)) *
+                                        (1.0f - a.edge_amp * __expf(-(g.xdet - x) * a.edge_inv_len)) *
+                                        (1.0f - a.edge_amp * __expf(-y * a.edge_inv_len)) *
+                                        (1.0f - a.edge_amp * __expf(-(g.ydet - y) * a.edge_inv_len));
+                        ok = rng.u() < W;
+                    }
+                    ++tries;
+                }
+                if (ok) {
+                    if (x <= g.ub_x && y <= g.ub_y && x >= g.lb_x && y >= g.lb_y) {
+                        const float qx = pow2 ? __fmul_rn(x - g.lb_x, inv_pixel) : __fdiv_rn(x - g.lb_x, g.pixel);
+                        const float qy = pow2 ? __fmul_rn(y - g.lb_y, inv_pixel) : __fdiv_rn(y - g.lb_y, g.pixel);
+                        const int ii = (int)floorf(qx);
+                        const int jj = (int)floorf(qy);
+                        if (ii >= 0 && jj >= 0 && ii < g.xdim && jj < g.ydim) {
+                            atomicAdd(&a.prf[g.prf_offset + (long long)ii * g.ydim + jj], 1ull);
+                            ++in_prf;
+                        }
+                    }
+                    stage = kNew;
+                    i += 32;
                 }
             }
         }
@@ -428,52 +483,64 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SampleArgs
 
 // Compact copies of the audited rows (position, photons, geometry, event) and
 // their pooled predictions: sum N p q_j over the radial categories j, sum N p,
-// sum N p (1 - p) and sum N (one thread per row; each warp sums its rows'
-// terms with shuffles and adds them with one FP64 atomic per term, so the
-// pool's few addresses see one atomic per 32 rows).
-__device__ __forceinline__ void warp_pool_add(double *dst, double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(dst, v);
-}
+// sum N p (1 - p) and sum N.  A warp per row, a lane per category edge (31
+// categories a pass, the upper edge from the next lane), the components in
+// order; a block adds its rows in shared memory and then once to the pool.  A
+// thread per row left 2,502 rows (1 % of 250,000 events) on 20 blocks: 496 us,
+// now 40.
+constexpr int kGatherThreads = 256;
 
-__global__ void audit_gather_kernel(const int *count, const int32_t *audit_row, const int32_t *sg_event,
-                                    const int32_t *sg_n, const float *out, const float4 *ev_pos,
-                                    const uint16_t *ev_geom, int bins, float r_max, float4 *a_pos, int32_t *a_n,
-                                    int32_t *a_geom, int32_t *a_ev, double *pool)
+__global__ void __launch_bounds__(kGatherThreads) audit_gather_kernel(
+    const int *count, const int32_t *audit_row, const int32_t *sg_event, const int32_t *sg_n, const float *out,
+    const float4 *ev_pos, const uint16_t *ev_geom, int bins, float r_max, float4 *a_pos, int32_t *a_n, int32_t *a_geom,
+    int32_t *a_ev, double *pool)
 {
-    const int n = count[1];
-    const int lane = threadIdx.x & 31;
-    const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    // the warp's lanes take rows base + lane together (the shuffles need all 32)
-    for (long long base = warp0 * 32; base < n; base += nwarps * 32) {
-        const long long i = base + lane;
-        const bool live = i < n;
-        double np = 0.0, q = 0.0, nn = 0.0;
-        Mix m;
-        if (live) {
-            const int r = audit_row[i];
+    extern __shared__ double s_pool[];  // [bins + 4]
+    for (int j = threadIdx.x; j < bins + 4; j += blockDim.x) s_pool[j] = 0.0;
+    __syncthreads();
+    const int n = count[1], lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    for (int i = warp; i < n; i += warps) {
+        const int r = audit_row[i];
+        const int32_t N = sg_n[r];
+        const float *o = out + (int64_t)r * kOutPad;
+        const float p = 1.0f / (1.0f + expf(-o[0]));
+        const double np = (double)N * p;
+        if (lane == 0) {
             const int32_t e = sg_event[r];
-            const int32_t N = sg_n[r];
             a_pos[i] = ev_pos[e];
             a_n[i] = N;
             a_geom[i] = ev_geom ? ev_geom[e] : 0;
             a_ev[i] = e;
-            const float *o = out + (int64_t)r * kOutPad;
-            const float p = 1.0f / (1.0f + expf(-o[0]));
-            decode_mix(o, m);
-            np = (double)N * p;
-            q = np * (1.0 - (double)p);
-            nn = (double)N;
+            atomicAdd(&s_pool[bins + 1], np);
+            atomicAdd(&s_pool[bins + 2], np * (1.0 - (double)p));
+            atomicAdd(&s_pool[bins + 3], (double)N);
         }
-        for (int j = 0; j <= bins; ++j)
-            warp_pool_add(&pool[j], live ? np * (double)bin_prob(m, j, bins, r_max) : 0.0);
-        warp_pool_add(&pool[bins + 1], np);
-        warp_pool_add(&pool[bins + 2], q);
-        warp_pool_add(&pool[bins + 3], nn);
+        Mix m;
+        decode_mix(o, m);
+        for (int j0 = 0; j0 <= bins; j0 += 31) {
+            const int j = j0 + lane;
+            const bool top = j > bins;
+            const float e_lo = top ? 0.0f : radial_edge(j, bins, r_max);
+            float q = 0.0f;
+#pragma unroll
+            for (int k = 0; k < kComponents; ++k) {
+                const Edge lo = edge_at(e_lo, top, m.mu[k], m.sd[k]);
+                Edge hi;
+                hi.t = __shfl_down_sync(0xffffffffu, lo.t, 1);
+                hi.cdf = __shfl_down_sync(0xffffffffu, lo.cdf, 1);
+                hi.ccdf = __shfl_down_sync(0xffffffffu, lo.ccdf, 1);
+                hi.pdf = __shfl_down_sync(0xffffffffu, lo.pdf, 1);
+                hi.e = __shfl_down_sync(0xffffffffu, lo.e, 1);
+                hi.inf = j + 1 > bins;
+                q += m.w[k] * ring_mass(lo, hi, m.mu[k], m.sd[k], nullptr, nullptr) / m.S[k];
+            }
+            if (lane < 31 && j <= bins) atomicAdd(&s_pool[j], np * (double)q);
+        }
     }
+    __syncthreads();
+    for (int j = threadIdx.x; j < bins + 4; j += blockDim.x)
+        if (s_pool[j] != 0.0) atomicAdd(&pool[j], s_pool[j]);
 }
 
 // Per-category totals of the audit's label-mode tally (rows [0, na) of a
@@ -664,7 +731,9 @@ extern "C" fd2_status fd2_sg_run(fd2_sg *s, fd2_ctx *c, double audit_fraction, f
             return sg_fail(s, FD2_ERR_OUT_OF_MEMORY, "audit buffers");
         e = cudaMemsetAsync(B->a_pool, 0, sizeof(double) * (nb + 3), q);
         if (e == cudaSuccess) {
-            audit_gather_kernel<<<(unsigned)std::min((na + 127) / 128, 4096), 128, 0, q>>>(
+            const int rows = kGatherThreads / 32;  // of a block
+            audit_gather_kernel<<<(unsigned)std::min((na + rows - 1) / rows, 4 * c->sm_count), kGatherThreads,
+                                  sizeof(double) * (s->bins + 4), q>>>(
                 R->d_count, R->audit_row, R->sg_event, R->sg_n, R->out, c->d_ev_pos,
                 c->has_geom ? c->d_ev_geom : nullptr, s->bins, (float)s->radial_max, B->a_pos, B->a_n, B->a_geom,
                 B->a_ev, B->a_pool);
