@@ -723,6 +723,12 @@ static fd2_status submit_common(fd2_ctx *c, int64_t n, const float *xs, const fl
     const size_t G = c->geoms.size();
     c->hist_per_geom.assign(G, 0.0);
     if (G == 1) c->hist_per_geom[0] = c->params.num_hist;
+    // A run of a few photons per lane takes as long as its longest walks, which
+    // go faster beside fewer warps: two CTAs per SM below 500,000 expected
+    // photons (config 0, 25 / 100 / 400 x-rays: 0.28 / 0.41 / 0.70 ms against
+    // 0.34 / 0.48 / 0.73 with four; 936,000 photons 1.55 against 1.48)
+    const bool few = c->mu_total < 5e5 && !c->opt.ctas_per_sm && !c->tuned && G == 1 && !c->opt.column_grid;
+    c->cfg.grid_ctas = few ? std::min(2, c->cfg.ctas_per_sm) : 0;
     if (xs) choose_window(c, xs, ys, geom, n);
     else choose_window_sums(c, sums ? sums[0] : 0.0, sums ? sums[1] : 0.0, n);
     fd2_status st = ensure_chunks(c);
@@ -1109,7 +1115,7 @@ fd2_status fd2_get_timing(fd2_ctx *c, fd2_timing *out)
         FD2_CUDA(c, cudaEventElapsedTime(&out->pipeline_ms, c->ev_start, c->ev_end));
     }
     out->photons = c->last_photons;
-    out->grid = c->sm_count * c->cfg.ctas_per_sm;
+    out->grid = c->sm_count * (c->cfg.grid_ctas ? c->cfg.grid_ctas : c->cfg.ctas_per_sm);
     out->block = c->cfg.block;
     out->chunk = c->cfg.chunk;
     out->refill = c->cfg.refill;
@@ -1220,6 +1226,8 @@ fd2_status fd2_autotune(fd2_ctx *c, int32_t budget_runs)
     if (c->n_events <= 0) return fail(c, FD2_ERR_STATE, "submit events before tuning");
     fd2_status st = fd2_wait(c);
     if (st != FD2_OK) return st;
+    c->tuned = true;
+    c->cfg.grid_ctas = 0;
     fd2::TransportConfig best = c->cfg;
     if (tune_cache_lookup(c, &best)) return set_config(c, best);
     auto time_cfg = [&](const fd2::TransportConfig &k, float *ms) -> fd2_status {

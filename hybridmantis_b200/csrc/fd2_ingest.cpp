@@ -211,6 +211,7 @@ void release(fd2_ingest *in)
     c->opt.event_base = in->base0;
     c->n_events = 0;
     c->mu_total = 0.0;
+    c->cfg.grid_ctas = 0;  // every batch the full grid
     c->counts_ready = false;
     c->graph_valid = false;
     c->ingest_active = false;

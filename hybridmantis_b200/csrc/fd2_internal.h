@@ -13,6 +13,7 @@ namespace fd2 {
 struct TransportConfig {
     int block = 256;     // threads per CTA (multiple of 32, <= 1024)
     int ctas_per_sm = 2; // persistent grid = SMs * ctas_per_sm
+    int grid_ctas = 0;   // CTAs per SM launched where fewer than ctas_per_sm do (0: ctas_per_sm)
     int chunk = 32;      // photons per work-queue chunk
     int refill = 1;      // idle lanes that trigger a warp refill
     int window = 0;      // shared-memory PRF window edge (0 = off)

@@ -332,8 +332,10 @@ constexpr int kParkKind = kPark * kParkWords;  // words from one kind's photons 
 // Ended photons a warp holds: fewer than 32 wait, and up to 32 end in a pass.
 constexpr int kEnded = 64;
 // Waiting photons that start a pass once the queue and the ready photons are
-// used up: waiting for more would only idle lanes then.
-constexpr int kTailBatch = 8;
+// used up: waiting for more would only hold up the last photons, whose serial
+// walks are what a small run takes (25 / 400 / 2,311 x-rays with 1: 0.35 /
+// 0.74 / 5.60 ms, with 2: 0.37 / 0.74 / 5.61, with 8: 0.49 / 0.85 / 5.84).
+constexpr int kTailBatch = 1;
 
 // A warp's shared memory: its parked photons (those that wait at a wall, and
 // those that wait for a hop), its ended photons and its ring of chunks.
@@ -983,7 +985,8 @@ cudaError_t launch_transport(cudaStream_t s, const TransportConfig &cfg, int sm_
     // registers without a spill; 64 geometries x 100 points x 4,000 photons:
     // 22.9 ms, 28.5 ms with two)
     const int per_sm_label = !multi && cfg.ctas_per_sm >= 4 ? 4 : 3;
-    const unsigned grid = (unsigned)(sm_count * (a.radial ? per_sm_label : cfg.ctas_per_sm));
+    const unsigned grid = (unsigned)(sm_count * (cfg.grid_ctas ? cfg.grid_ctas
+                                                    : a.radial ? per_sm_label : cfg.ctas_per_sm));
     a.refill = std::min(std::max(a.refill, 1), 32);
     a.fresnel_batch = std::min(std::max(a.fresnel_batch, 1), kPark);
     // a refill takes 1 / 2^pull_shift of the chunks left: at most half of a

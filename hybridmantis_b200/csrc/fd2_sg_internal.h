@@ -19,7 +19,7 @@ constexpr int kComponents = FD2_SG_COMPONENTS;
 constexpr int kInPad = 32;   // input width seen by the first GEMM (K multiple of 32)
 constexpr int kOutPad = 64;  // output width of the last GEMM
 constexpr int kMaxSplits = 16;
-constexpr int kPredictRows = 1 << 16;  // rows of one prediction pass at 256 hidden units
+constexpr int kPredictRows = 2 * 148 * 128;  // rows of one prediction pass at 256 hidden units
 constexpr float kMuScale = 50.0f;  // ring radius = kMuScale * softplus(output), um (>= 0)
 constexpr float kSdScale = 10.0f;  // um
 constexpr float kLateralUnitUm = 50.0f;  // unit of feature 2, the deposition's distance from the detector centre
@@ -93,7 +93,7 @@ struct fd2_sg {
     float *out = nullptr, *target = nullptr, *ylab = nullptr, *has_rad = nullptr;
     cudaGraphExec_t graph = nullptr;
 
-    // fd2_sg_predict's rows (predict_cap of them; grown, kept)
+    // fd2_sg_predict's rows (predict_cap of them; grown, kept): one allocation at pout
     int64_t predict_cap = 0;
     float *pf = nullptr, *pout = nullptr, *ppack = nullptr;
     __nv_bfloat16 *px = nullptr, *pha = nullptr, *phb = nullptr;

@@ -1144,8 +1144,7 @@ void fd2_sg_destroy(fd2_sg *s)
                     (void *)s->d_step, (void *)s->d_acc, (void *)s->d_lr, (void *)s->ws, (void *)s->x0, (void *)s->h1, (void *)s->h2,
                     (void *)s->h3, (void *)s->d1, (void *)s->d2, (void *)s->d3, (void *)s->out, (void *)s->dout,
                     (void *)s->target, (void *)s->has_rad, (void *)s->ylab, (void *)s->d_feat, (void *)s->d_photons,
-                    (void *)s->d_detected, (void *)s->d_radial, (void *)s->d_tc_fault, (void *)s->pbT, (void *)s->pf, (void *)s->px,
-                    (void *)s->pha, (void *)s->phb, (void *)s->pout, (void *)s->ppack, (void *)s->tA,
+                    (void *)s->d_detected, (void *)s->d_radial, (void *)s->d_tc_fault, (void *)s->pbT, (void *)s->pout, (void *)s->tA,
                     (void *)s->tB})
         if (p) cudaFree(p);
     sg_free_run_buffers(s);
@@ -1392,22 +1391,24 @@ fd2_status fd2_sg_predict(fd2_sg *s, const float *features, int64_t n, float *ou
     if (!s || !features || !out || n < 0) return FD2_ERR_INVALID_ARGUMENT;
     if (n == 0) return FD2_OK;
     SG_CUDA(s, cudaSetDevice(s->device));
-    // up to kPredictRows rows a pass (fewer with wider layers): enough tiles for
-    // every SM, where the training batch's 8,192 rows are 64.  The outputs leave
-    // the device packed, straight into the caller's array (50,001 rows: seven
-    // batches of padded rows, each waited for and unpadded on the host, 2.5 ms;
-    // one pass 0.9)
+    // up to kPredictRows rows a pass (fewer with wider layers): two tiles for
+    // every SM, where the training batch's 8,192 rows are 64 tiles in all.  The
+    // outputs leave the device packed, straight into the caller's array (50,001
+    // rows: seven batches of padded rows, each waited for and unpadded on the
+    // host, 2.5 ms; two passes 0.9)
     const int64_t most = std::min<int64_t>(kPredictRows, ((int64_t)kPredictRows * 256) / s->hidden);
     const int64_t cap = std::min(n, most);
     if (cap > s->predict_cap) {
-        const size_t C = (size_t)cap, H = (size_t)s->hidden;
+        // one allocation: outputs, packed outputs and features in FP32, then
+        // the network's input and two layers in BF16, each 256-byte aligned
+        const size_t C = ((size_t)cap + 63) / 64 * 64, H = (size_t)s->hidden;
         s->predict_cap = 0;
-        SG_CUDA(s, alloc(&s->pf, C * kFeatures));
-        SG_CUDA(s, alloc(&s->px, C * kInPad));
-        SG_CUDA(s, alloc(&s->pha, C * H));
-        SG_CUDA(s, alloc(&s->phb, C * H));
-        SG_CUDA(s, alloc(&s->pout, C * kOutPad));
-        SG_CUDA(s, alloc(&s->ppack, C * kOutputs));
+        SG_CUDA(s, alloc(&s->pout, C * (kOutPad + kOutputs + kFeatures) + C * (kInPad + 2 * H) / 2));
+        s->ppack = s->pout + C * kOutPad;
+        s->pf = s->ppack + C * kOutputs;
+        s->px = reinterpret_cast<__nv_bfloat16 *>(s->pf + C * kFeatures);
+        s->pha = s->px + C * kInPad;
+        s->phb = s->pha + C * H;
         s->predict_cap = cap;
     }
     cudaError_t e = cudaSuccess;

@@ -31,14 +31,14 @@ def test_loss_and_gradient_at_tile_edges(require_gpu, rows, bins):
     assert np.linalg.norm(g - wg) <= 2e-3 * np.linalg.norm(wg)
 
 
-@pytest.mark.parametrize("rows", [1, 127, 129, 8193, 65535, 65539])
+@pytest.mark.parametrize("rows", [1, 127, 129, 8193, 37887, 37891, 75780])
 def test_predict_at_pass_edges(require_gpu, rows):
     f = np.random.default_rng(rows).uniform(-1, 1, (rows, 8)).astype(np.float32)
     with sgm.Surrogate() as s:
         s.set_hull(np.full(8, -1.0), np.full(8, 1.0))
         out = s.predict(f)
         # rows do not depend on the rows around them
-        for a, b in ((0, min(rows, 70)), (max(rows - 70, 0), rows), (max(65536 - 3, 0), rows)):
+        for a, b in ((0, min(rows, 70)), (max(rows - 70, 0), rows), (37888 - 3, min(rows, 37888 + 40))):
             if a < b:
                 assert np.array_equal(out[a:b], s.predict(f[a:b]))
         want, _ = so.forward(s.params(), 256, f[-64:], np.full(8, -1.0), np.full(8, 1.0))
