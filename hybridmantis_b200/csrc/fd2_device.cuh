@@ -68,15 +68,16 @@ __device__ __forceinline__ float u01(uint32_t r)
     return __uint_as_float(__funnelshift_r(r, 0x7Fu, 9)) - 0.99999994039535522461f;
 }
 
-// Internal step result: the photon waits at a column wall for the Fresnel
-// part of its surface interaction (not a fate).
-constexpr int kNeedsFresnel = 100;
-// Internal step results of the crosstalk path: the photon crosses into the
-// adjacent column and needs that column's normal (crosstalk_normal), or its
-// attempt was rejected and is retried in the next round.
-constexpr int kNeedsHop = 103;  // the photon has left the column and hops to the next
-constexpr int kNeedsNormal = 101;
-constexpr int kRetryNormal = 102;
+// What a part of the walk returns, and the state of the lane that holds the
+// photon (a lane without one: 0): a fate (1 to 7), or one of these.  Bit 3:
+// the photon is in flight; bit 1: it waits for a part that runs later.
+enum Flight : int {
+    kFlies = 8,       // goes on with its next step
+    kRetryNormal = 9, // its crosstalk normal was rejected: tried again in the next step
+    kWaits = 10,      // at a column wall or the top reflector: surface_wait
+    kHops = 11,       // has left its column: surface_wait from the hop on
+    kNeedsNormal = 16 // crosses into the adjacent column: crosstalk_normal next
+};
 
 // Warp-uniform part of a photon's seed: the Philox round keys of the run
 // seed (the kernel keeps them in shared memory) and the run counter.
@@ -310,15 +311,15 @@ struct Walker {
                 ++moved;
             }
         }
-        int fate = lost ? kLost : r > thr ? kOutOfCol : outside_detector(g) ? kLost : kAlive;
-        dist += fate == kAlive ? d : 0.0f;
+        int fate = lost ? kLost : r > thr ? kOutOfCol : outside_detector(g) ? kLost : kFlies;
+        dist += fate == kFlies ? d : 0.0f;
         if (g.neg_inv_mu != 0.0f) {
             // bulk absorption: one Exp(1) budget of absorption lengths per
             // photon, spent flight by flight; by the exponential's lack of
             // memory the same law as the reference's fresh draw per flight
             // (absorbed when d >= -ln(u) / mu)
             const float da = d * g.mu;
-            fate = fate == kAlive && da >= budget && d >= 0.0f ? kAbsBulk : fate;
+            fate = fate == kFlies && da >= budget && d >= 0.0f ? kAbsBulk : fate;
             budget -= da;
         }
         return fate;
@@ -333,7 +334,7 @@ struct Walker {
         for (;;) {
             flat_rough(ix, iy, iz);
             if (always_rough || g.beta > 0.0f) roughen(g.beta);
-            if (!(sum3(iy, ny, ix, nx, iz, nz) < kCos157)) return kAlive;
+            if (!(sum3(iy, ny, ix, nx, iz, nz) < kCos157)) return kFlies;
             if (tries < 100) {
                 ++tries;
                 continue;
@@ -433,7 +434,7 @@ struct Walker {
                 // after a sensor hop: around the hop's own reversed direction
                 const float ax = after_sensor ? -dx : ix, ay = after_sensor ? -dy : iy, az = after_sensor ? -dz : iz;
                 const int f = new_column_normal(g, ax, ay, az, t, after_sensor);
-                if (f != kAlive) return f;
+                if (f != kFlies) return f;
                 if (after_sensor) {
                     st = kAfterSensor;
                 } else {
@@ -456,7 +457,7 @@ struct Walker {
                 } else {
                     // a sensor hop that reached the top ends at the top
                     // reflector (the hop's end check finds the top at once)
-                    if (!at_top(g)) return kAlive;
+                    if (!at_top(g)) return kFlies;
                     st = kEnd;
                 }
             } else {
@@ -474,7 +475,7 @@ struct Walker {
                     if ((counts & kTopMask) == ((uint32_t)kMaxTopLoops << 16)) return kCapped;
                     st = kHop;
                 } else {
-                    if (fabsf(pz + g.half) >= kEps) return kAlive;
+                    if (fabsf(pz + g.half) >= kEps) return kFlies;
                     counts |= kFromEnd;
                     st = kSensor;
                 }
@@ -493,12 +494,12 @@ struct Walker {
         __sincosf(kPi * (2.0f * u() - 1.0f), &s, &c);
         dx = rr * c;
         dy = rr * s;
-        return kAlive;
+        return kFlies;
     }
 
     // Interaction with a column wall (boundary_analysis), first part: whether
     // the photon crosses into the adjacent column (kNeedsNormal) or meets the
-    // wall (kNeedsFresnel); the rest (crosstalk_normal, surface_wait) can run
+    // wall (kWaits); the rest (crosstalk_normal, surface_wait) can run
     // later, from the photon state alone.
     template <class G>
     __device__ __forceinline__ int surface_entry(const G &g)
@@ -509,12 +510,12 @@ struct Walker {
         float cct = pz < 0.0f && pz >= -g.half ? below : 0.0f;
         cct = pz < g.cct_band_lo && pz >= 0.0f ? above : cct;
         cct = pz <= g.half && pz >= g.cct_band_lo ? 1.0f : cct;
-        return u() < cct ? kNeedsNormal : kNeedsFresnel;
+        return u() < cct ? kNeedsNormal : kWaits;
     }
 
     // Crosstalk into the adjacent column (transmit with crosstalk): one
     // attempt at the new column's normal, a random normal within 1.57 rad of
-    // the reversed direction, flattened and roughened.  Returns kAlive (the
+    // the reversed direction, flattened and roughened.  Returns kFlies (the
     // photon is in the new column), kTheta1 (no normal after 100 retries) or
     // kRetryNormal (rejected: the kernel retries in its next round, beside
     // the other lanes' first attempts, instead of looping here with the few
@@ -528,7 +529,7 @@ struct Walker {
         if (!(sum3(iy, ny, ix, nx, iz, nz) < kCos157)) {
             xc = fmaf(-g.R, nx, px);
             yc = fmaf(-g.R, ny, py);
-            return kAlive;
+            return kFlies;
         }
         if (tries < 100) {
             ++tries;
@@ -537,16 +538,17 @@ struct Walker {
         return kTheta1;
     }
 
-    // Retry counts of a wall interaction, kept in a word of the photon while
-    // it waits for a hop: tries at an incidence angle and at a next normal (at
+    // The photon's tag: its geometry in bits 0-7, bit 8 just reflected by the
+    // sensor, above it the retry counts of a wall interaction while it waits: tries at an incidence angle and at a next normal (at
     // most 100 each), perturbations (3) and smooth attempts (25).
+    static constexpr uint32_t kGeomBits = 0xffu, kReflected = 1u << 8;
     static constexpr int kTheta = 9, kPerturb = 16, kSmooth = 18, kNormalTry = 23;
     static constexpr uint32_t kCounts = (0x7fu << kTheta) | (3u << kPerturb) | (0x1fu << kSmooth) | (0x7fu << kNormalTry);
 
     // What a waiting photon waits for: the top reflector, or Fresnel reflection
     // / refraction on the rough wall (boundary_analysis, second part).  A
     // photon that refracts out of its column waits again, for its hop
-    // (kNeedsHop); with `hop` it continues there, until it is back inside a
+    // (kHops); with `hop` it continues there, until it is back inside a
     // column or meets the next column's wall from outside and hops again.  One
     // in five wall interactions leaves the column: run to their end beside the
     // others, the hops took half of the pass at 2 to 3 lanes.  `counts` keeps
@@ -564,7 +566,7 @@ struct Walker {
         float st = 0.0f, ct = 1.0f;            // sin, cos of the last refraction angle
         float kx = 0, ky = 0, kz = 0, kdx = 0, kdy = 0, kdz = 0;
         enum { kLeave, kNewSurface, kRestore, kIncidence } stage = hop ? kLeave : kNewSurface;
-        int fate = kAlive;
+        int fate = kFlies;
         for (int loop = 0; loop < kMaxSurfaceLoops; ++loop) {
             if (stage == kNewSurface) {
                 if (!outside) {
@@ -597,7 +599,7 @@ struct Walker {
                 if (c1 > 1.0f || c1 < 0.0f) {
                     if (outside) {
                         const int f = new_column_normal(g, -dx, -dy, -dz, tries_normal, false);
-                        if (f != kAlive) {
+                        if (f != kFlies) {
                             fate = f;
                             break;
                         }
@@ -609,7 +611,7 @@ struct Walker {
                             // over: tried again in the next pass
                             counts |= (uint32_t)tries_theta << kTheta | (uint32_t)reperturbs << kPerturb |
                                       (uint32_t)smooth << kSmooth;
-                            return kNeedsFresnel;
+                            return kWaits;
                         }
                         stage = kNewSurface;
                         continue;
@@ -672,12 +674,12 @@ struct Walker {
                 if (!g.stale_out) {
                     counts |= (uint32_t)tries_theta << kTheta | (uint32_t)tries_normal << kNormalTry |
                               (uint32_t)reperturbs << kPerturb | (uint32_t)smooth << kSmooth;
-                    return kNeedsHop;
+                    return kHops;
                 }
             }
             // kLeave: hop between columns
             const int f = leave_column(g);
-            if (f != kAlive) {
+            if (f != kFlies) {
                 fate = f;
                 break;
             }
@@ -760,7 +762,7 @@ struct Walker {
             return kDetect;
         }
         dz = -dz;
-        return kAlive;
+        return kFlies;
     }
 
     // A wall of the column centred at (cx, cy), met at (px, py); `inside`:
@@ -798,7 +800,7 @@ struct Walker {
             dy = fmaf(2.0f * c1, ny, dy);
             dz = fmaf(2.0f * c1, nz, dz);
             renorm(dx, dy, dz);
-            return kAlive;
+            return kFlies;
         }
         const float k = eta * c1 - ct;
         dx = fmaf(eta, dx, k * nx);
@@ -810,7 +812,7 @@ struct Walker {
             xc = cx;
             yc = cy;
         }
-        return kAlive;
+        return kFlies;
     }
 
     // The flight of a lattice segment: to a plane (kToPlane), to the wall of
@@ -988,25 +990,25 @@ struct Walker {
     // One transport step (the body of the reference's step function algo):
     // flight, sensor, trapped-photon restart (from `*event`, the x, y, z of
     // the photon's event), or a surface interaction up to the part that waits.
-    // Returns the photon's fate, kAlive while it is in flight, kNeedsNormal
-    // (run crosstalk_normal next) or kNeedsFresnel (surface_wait next).  A
+    // Returns the photon's fate, kFlies while it is in flight, kNeedsNormal
+    // (run crosstalk_normal next) or kWaits (surface_wait next).  A
     // photon reflected by the sensor inside a column flies on in its next step,
-    // beside the warp's others; `reflected` then keeps it from meeting the
+    // beside the warp's others; a bit of its tag then keeps it from meeting the
     // sensor again where it stands.
     template <class G>
-    __device__ __forceinline__ int step(const G &g, const float4 *event, bool &reflected)
+    __device__ __forceinline__ int step(const G &g, const float4 *event, uint32_t &tag)
     {
         const int f = flight(g);
-        if (f != kAlive) return f;
-        const bool sensor = !reflected && fabsf(pz + g.half) < kEps;
-        reflected = false;
+        if (f != kFlies) return f;
+        const bool sensor = !(tag & kReflected) && fabsf(pz + g.half) < kEps;
+        tag &= ~kReflected;
         if (sensor) {
             // sensor plane inside a column (detection)
             if (!(g.sensor_refl > 0.0f && u() < g.sensor_refl)) return kDetect;
             dz = -dz;  // specular reflection on the flat sensor
             renorm(dx, dy, dz);
-            reflected = true;
-            return kAlive;
+            tag |= kReflected;
+            return kFlies;
         }
         if (fabsf(dz) < kEps) {
             // trapped travelling horizontally: restart from the event position,
@@ -1014,10 +1016,10 @@ struct Walker {
             const float4 e = *event;
             px = e.x; py = e.y; pz = e.z;
             emit(false);
-            return kAlive;
+            return kFlies;
         }
         if (++rebound > kMaxBoundaryCalls) return kCapped;
-        if (at_top(g)) return kNeedsFresnel;
+        if (at_top(g)) return kWaits;
         return surface_entry(g);
     }
 };

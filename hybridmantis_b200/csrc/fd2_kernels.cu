@@ -331,11 +331,6 @@ constexpr int kParkWords = 4;
 constexpr int kParkKind = kPark * kParkWords;  // words from one kind's photons to the other's
 // Ended photons a warp holds: fewer than 32 wait, and up to 32 end in a pass.
 constexpr int kEnded = 64;
-// Waiting photons that start a pass once the queue and the ready photons are
-// used up: waiting for more would only hold up the last photons, whose serial
-// walks are what a small run takes (25 / 400 / 2,311 x-rays with 1: 0.35 /
-// 0.74 / 5.60 ms, with 2: 0.37 / 0.74 / 5.61, with 8: 0.49 / 0.85 / 5.84).
-constexpr int kTailBatch = 1;
 
 // A warp's shared memory: its parked photons (those that wait at a wall, and
 // those that wait for a hop), its ended photons and its ring of chunks.
@@ -470,14 +465,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
         m.used = 0;
     }
     bool exhausted = false;
-    // The lane: without a photon, running one, or holding one that waits (at a
-    // wall or for a hop); the
-    // fate of one that has ended and is not yet recorded; a crosstalk normal
-    // that is retried in the next step
-    enum { kEmpty, kRun, kWait, kHop };
-    int state = kEmpty, fate = kAlive;
-    bool xretry = false;
-    int xtries = 0;
+    int state = 0;  // of the lane: no photon, a fate not yet recorded, or Flight
+    int xtries = 0; // tries at the crosstalk normal of a kRetryNormal photon
     // Philox round keys and run counter, shared by the CTA
     __shared__ uint32_t s_rk[20];
     __shared__ uint32_t s_run;
@@ -485,11 +474,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
     if (threadIdx.x == 0) s_run = *a.run_tag;
 
     Walker w;
-    // The photon's event, and its tag: the geometry in bits 0-7, bit 8 a photon
-    // just reflected by the sensor, above it the retry counts of a wall
-    // interaction (Walker::kCounts).
-    constexpr uint32_t kGeomBits = 0xffu, kReflected = 1u << 8;
-    uint32_t tag = 0, event = 0;
+    constexpr uint32_t kGeomBits = Walker::kGeomBits;
+    uint32_t tag = 0, event = 0;  // the photon's tag (Walker::kGeomBits ...) and event
     w.dist = 0.0f;
     // the lane's path-length sum
     __shared__ float s_ldist[kMaxThreads];
@@ -508,29 +494,32 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
         // fate and geometry) until a warp's worth is tallied together.  One to
         // two photons end in a step, and their pixel's two divisions and their
         // reductions cost the warp as many instructions as 32 photons' do.
-        const unsigned over = __ballot_sync(kFull, fate != kAlive);
-        if (over) {
-            if (fate != kAlive) {
+        const unsigned live = __ballot_sync(kFull, state >= kFlies);
+        const unsigned some = __ballot_sync(kFull, state != 0);
+        const unsigned odd = __ballot_sync(kFull, (state & 1) != 0);
+        const unsigned late = __ballot_sync(kFull, (state & 2) != 0) & live;
+        unsigned run = live & ~late;
+        const unsigned held = kGrid ? late : late & ~odd, hops = kGrid ? 0u : late & odd;
+        if (some != live) {
+            const unsigned over = some & ~live;
+            if (state != 0 && state < kFlies) {
                 m.ended[n_ended + __popc(over & lanemask_lt())] =
-                    make_float4(w.px, w.py, __uint_as_float(event), __int_as_float((int)(tag & kGeomBits) << 8 | fate));
+                    make_float4(w.px, w.py, __uint_as_float(event), __int_as_float((int)(tag & kGeomBits) << 8 | state));
                 if (kMulti) {
                     atomicAdd(&s_dist[tag & kGeomBits], w.dist);
                 } else {
                     s_ldist[threadIdx.x] += w.dist;  // lane-private: no atomic
                     w.dist = 0.0f;
                 }
-                fate = kAlive;
+                state = 0;
             }
             n_ended += __popc(over);
         }
         // ---- which pass: steps of the lanes' photons, or the waiting ones
-        const unsigned odd = __ballot_sync(kFull, (state & 1) != 0), upper = __ballot_sync(kFull, state >= kWait);
-        unsigned run = odd & ~upper;
-        const unsigned held = upper & ~odd, hops = kGrid ? 0u : upper & odd, none = ~(upper | odd);
         const int n_held = __popc(held), n_hops = __popc(hops);
         const int waiting = n_wait + n_held, hopping = n_hop + n_hops;
         bool supply = n_ready + n_hready > 0 || !exhausted;
-        const bool finished = !run && waiting + hopping == 0 && !supply;
+        const bool finished = !run && !supply && waiting + hopping == 0;
         while (n_ended >= 32 || (finished && n_ended > 0)) {
             const int n = min(n_ended, 32);
             n_ended -= n;
@@ -544,18 +533,21 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
         int at = -1;     // the parked photon this lane exchanges its own with
         int moved = 0;   // lanes that do
         bool flush = false, hop = false, deal = false;
-        const int batch = supply ? a.fresnel_batch : min(a.fresnel_batch, kTailBatch);
-        if (waiting >= batch || hopping >= batch || (!run && !supply)) {
+        // Once the queue and the ready photons are used up every waiting photon
+        // starts a pass: more would only hold up the last photons, whose serial
+        // walks are what a small run takes (25 / 400 / 2,311 x-rays with passes
+        // from 1 photon 0.35 / 0.74 / 5.60 ms, from 2 0.37 / 0.74 / 5.61, from
+        // 8 0.49 / 0.85 / 5.84).
+        const int batch = supply ? a.fresnel_batch : 1;
+        if (waiting >= batch || hopping >= batch) {
             // waiting photons into the lanes that hold none of their kind:
             // first the empty lanes (when no photon is ready among them), then
             // lanes whose photon can wait as a ready one.  Without a lane that
             // can run one, the others step first.
-            const unsigned other = run & ~__ballot_sync(kFull, xretry);
+            const unsigned none = ~live, other = run & ~odd;
             const int n_none = __popc(none), n_other = __popc(other);
-            hop = !kGrid && (hopping >= batch || waiting == 0) &&
-                  (n_hops > 0 || n_other > 0 || (n_hready == 0 && n_none > 0));
-            flush = hop || ((waiting >= batch || (!run && !supply)) &&
-                            (n_held > 0 || n_other > 0 || (n_ready == 0 && n_none > 0)));
+            hop = !kGrid && hopping >= batch && (n_hops > 0 || n_other > 0 || (n_hready == 0 && n_none > 0));
+            flush = hop || (waiting >= batch && (n_held > 0 || n_other > 0 || (n_ready == 0 && n_none > 0)));
             if (flush) {
                 const int nw = hop ? n_hop : n_wait, nr = hop ? n_hready : n_ready;
                 const unsigned take = nr == 0 ? none : 0u;
@@ -573,17 +565,17 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
             // lanes with a waiting photon park it, for a ready one of its kind
             // if there is one; empty lanes take ready ones; the rest get new
             // photons
-            const int n_none = __popc(none);
+            const int n_none = 32 - __popc(live);
             const int left = max(n_ready - n_held, 0), hleft = max(n_hready - n_hops, 0);
             const int taken = min(left, n_none), htaken = min(hleft, n_none - taken);
-            if (state != kRun) {
-                const unsigned same = state == kWait ? held : !kGrid && state == kHop ? hops : none;
+            if (!((run >> lane) & 1u)) {
+                const unsigned same = state == kWaits ? held : !kGrid && state == kHops ? hops : ~live;
                 const int rank = __popc(same & lanemask_lt());
                 bool got;
-                if (state == kWait) {
+                if (state == kWaits) {
                     at = n_wait + rank;
                     got = rank < n_ready;
-                } else if (!kGrid && state == kHop) {
+                } else if (!kGrid && state == kHops) {
                     at = kParkKind + n_hop + rank;
                     got = rank < n_hready;
                 } else {
@@ -591,7 +583,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                     if (got) at = rank < taken ? n_wait + n_ready - 1 - rank
                                                : kParkKind + n_hop + n_hready - 1 - (rank - taken);
                 }
-                state = got ? kRun : kEmpty;
+                state = got ? kFlies : 0;
             }
             moved = n_held + n_hops + taken + htaken;
             n_wait += n_held;
@@ -625,29 +617,25 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                                            __uint_as_float(w.s3));
                 w.s0 = __float_as_uint(t.x), w.s1 = __float_as_uint(t.y);
                 w.s2 = __float_as_uint(t.z), w.s3 = __float_as_uint(t.w);
-                if (flush) state = !kGrid && hop ? kHop : kWait;
+                if (flush) state = !kGrid && hop ? kHops : kWaits;
                 if (kGrid) w.in_gap = flush;
             }
             __syncwarp();
         }
         if (flush) {
             // ---- the waiting photons' pass
-            if (state == (!kGrid && hop ? kHop : kWait)) {
+            if (state == (!kGrid && hop ? kHops : kWaits)) {
                 if constexpr (kGrid) {
-                    fate = w.grid_segment(a.g0);
-                    state = fate != kAlive ? kEmpty : w.in_gap ? kWait : kRun;
+                    state = w.grid_segment(a.g0);
+                    if (state == kFlies && w.in_gap) state = kWaits;
                 } else {
-                    const int f = kMulti ? w.surface_wait(s_geom[tag & kGeomBits], hop, tag)
-                                         : w.surface_wait(a.g0, hop, tag);
-                    const bool waits = f == kNeedsHop || f == kNeedsFresnel;
-                    state = f == kAlive ? kRun : f == kNeedsHop ? kHop : waits ? kWait : kEmpty;
-                    fate = waits ? kAlive : f;
+                    state = kMulti ? w.surface_wait(s_geom[tag & kGeomBits], hop, tag) : w.surface_wait(a.g0, hop, tag);
                 }
             }
             continue;
         }
         // ---- hand out photons to idle lanes
-        unsigned needy = __ballot_sync(kFull, state == kEmpty);
+        unsigned needy = __ballot_sync(kFull, state == 0);
         if (deal && needy && (__popc(needy) >= a.refill || needy == kFull)) {
             int slot = m.slot, len = m.len;
             uint32_t used = m.used;
@@ -718,10 +706,10 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                     event = s.event;
                     if (kMulti) w.dist = 0.0f;
                     w.start(s.pos.x, s.pos.y, s.pos.z, k, (uint32_t)(a.event_base + s.event), k == 0, key);
-                    state = kRun;
+                    state = kFlies;
                     if constexpr (kGrid) {
                         w.grid_place(a.g0);
-                        state = w.in_gap ? kWait : kRun;
+                        if (w.in_gap) state = kWaits;
                     }
                 }
                 needy &= ~__ballot_sync(kFull, mine);
@@ -738,38 +726,33 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
         // ---- steps of the lanes' photons until enough lanes are idle to make
         // the exchange worth its instructions; with nothing to fill them, until
         // one more is
-        run = __ballot_sync(kFull, state == kRun);
+        // (in flight and not waiting: kFlies or kRetryNormal)
+        run = __ballot_sync(kFull, (state & 10) == 8);
         if (!run) continue;
         const int stay = supply ? 33 - a.refill : __popc(run);
         do {
-            if (state == kRun) {
+            if ((state & 10) == 8) {
                 if constexpr (kGrid) {
                     // explicit column lattice: one segment, of a photon in a column
-                    fate = w.grid_segment(a.g0);
-                    state = fate != kAlive ? kEmpty : w.in_gap ? kWait : kRun;
+                    state = w.grid_segment(a.g0);
+                    if (state == kFlies && w.in_gap) state = kWaits;
                 } else {
                     int f = kNeedsNormal;
-                    if (!xretry) {
-                        bool reflected = (tag & kReflected) != 0u;
-                        f = kMulti ? w.step(s_geom[tag & kGeomBits], a.ev_pos + event, reflected)
-                                   : w.step(a.g0, a.ev_pos + event, reflected);
-                        tag = (tag & ~kReflected) | (reflected ? kReflected : 0u);
+                    if (state == kFlies) {
+                        xtries = 0;
+                        f = kMulti ? w.step(s_geom[tag & kGeomBits], a.ev_pos + event, tag)
+                                   : w.step(a.g0, a.ev_pos + event, tag);
                     }
                     // crosstalk: one attempt at the next column's normal per
                     // step, so a rejected attempt is retried beside the other
                     // lanes' first ones
-                    if (f == kNeedsNormal) {
+                    if (f == kNeedsNormal)
                         f = kMulti ? w.crosstalk_normal(s_geom[tag & kGeomBits], xtries)
                                    : w.crosstalk_normal(a.g0, xtries);
-                        xretry = f == kRetryNormal;
-                        xtries = xretry ? xtries : 0;
-                    }
-                    const bool flies = f == kAlive || f == kRetryNormal;
-                    state = flies ? kRun : f == kNeedsFresnel ? kWait : kEmpty;
-                    fate = flies || f == kNeedsFresnel ? kAlive : f;
+                    state = f;
                 }
             }
-            run = __ballot_sync(kFull, state == kRun);
+            run = __ballot_sync(kFull, (state & 10) == 8);
         } while (__popc(run) >= stay);
     }
 
