@@ -374,15 +374,17 @@ void fit_window(fd2_ctx *c)
 // Launch shape unless the options give one, measured on a B200: one geometry
 // 256 threads x 4 CTAs per SM (32 warps at 64 registers; 20,000 config-1
 // x-rays 51.6 ms against 54.1 for 224 x 4 and 55.6 for 256 x 3, before the
-// steps below a full exchange were looped), chunks of 16 photons; several
-// geometries 256 x 3 (configuration 2, 500 x-rays: 73.0 ms against 90.6 for
-// 256 x 2; 256 x 4 the same); the column lattice 256 x 3 (10,001 config-1
-// x-rays 77.2 ms against 82.5 for 320 x 2); label mode with one geometry
-// (the surrogate's audit) as one geometry, with several 256 x 3.
+// steps below a full exchange were looped), chunks of 16 photons; the square
+// column lattice the same (10,001 config-1 x-rays 68.7 ms against 71.6 for
+// 256 x 3, 76.3 for 320 x 2); several geometries 256 x 3 (configuration 2, 500
+// x-rays: 60.5 ms against 62.5 for 256 x 4); the hexagonal lattice 256 x 3
+// (91.7 ms against 98.2 for 320 x 2), its only kernel above 256 x 2; label
+// mode with one geometry (the surrogate's audit) as one geometry, with
+// several 256 x 3.
 static void default_launch(const fd2_ctx *c, int n_geom, fd2::TransportConfig *cfg)
 {
     int block = 256, ctas = 4, chunk = 16;
-    if (c->opt.column_grid || n_geom > 1) {
+    if (c->opt.column_grid == 2 || n_geom > 1) {
         ctas = 3;
         chunk = 32;
     }

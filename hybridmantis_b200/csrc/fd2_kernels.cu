@@ -429,9 +429,10 @@ __device__ __forceinline__ void tally_ended(const TransportArgs &a, const DevGeo
 // lane for 8 others had the Fresnel part run at 9.1 lanes for a third of the
 // warps' time, its hops at 2 to 3, and steps at 25.  20,000 config-1 x-rays
 // (one B200): 59.2 ms before, 51.6 with the wall's photons parked, 46.0 with
-// ended photons tallied together and steps looped, 44.2 with the hops parked;
-// square / hexagonal lattice 109 / 151 -> 71 / 91 ms.  Per photon 1,252 -> 995
-// warp instructions, issue slots 87 % busy, 22.7 of 32 lanes.  Tallies:
+// ended photons tallied together and steps looped, 44.2 with the hops parked,
+// 42.9 with one state word per lane; 10,001 x-rays in the square / hexagonal
+// lattice 102.5 / 142.9 -> 68.7 / 91.7 ms.  Per photon 1,252 -> 959 warp
+// instructions, issue slots 87 % busy, 23 of 32 lanes.  Tallies:
 // ended photons are tallied 32 at a time (tally_ended) with L2 reductions;
 // with kAgg (tally_mode 1) the fates and the PRF core of geometry 0 are
 // tallied in shared memory first (identical tallies).  kMulti: the
@@ -923,6 +924,7 @@ cudaError_t launch_fill_chunks(cudaStream_t s, int64_t n, int chunk, const int32
     X(true, 512, 1, false, false, false) X(true, 256, 2, false, false, false)              \
     X(true, 256, 3, false, false, false) X(true, 256, 3, true, false, false)               \
     X(true, 256, 4, false, false, false) X(false, 256, 3, false, true, false)              \
+    X(false, 256, 4, false, true, false)                                                   \
     X(false, 512, 1, false, false, true) X(false, 256, 2, false, false, true)              \
     X(false, 320, 2, false, false, true) X(false, 256, 3, false, false, true)              \
     X(false, 256, 4, false, false, true) X(false, 256, 4, true, false, false)
@@ -980,7 +982,13 @@ cudaError_t launch_transport(cudaStream_t s, const TransportConfig &cfg, int sm_
     if (a.g0.grid) {
         // explicit column lattice: single geometry, 256 or 320 threads
         if (multi || a.radial) return cudaErrorInvalidConfiguration;
+        // four CTAs per SM for the square lattice only (10,001 x-rays 68.7 ms,
+        // 71.6 with three): compiled for 64 registers, the test of a hexagonal
+        // lattice's neighbour columns is contracted differently, and 9,092 of
+        // 10,001 x-rays would count other photons
         if (cfg.block == 320) transport_kernel<false, 320, 2, false, true><<<grid, cfg.block, smem, s>>>(a);
+        else if (cfg.block <= 256 && per_sm == 4 && a.g0.grid == 1)
+            transport_kernel<false, 256, 4, false, true><<<grid, cfg.block, smem, s>>>(a);
         else if (cfg.block <= 256 && per_sm >= 3) transport_kernel<false, 256, 3, false, true><<<grid, cfg.block, smem, s>>>(a);
         else if (cfg.block <= 256) transport_kernel<false, 256, 2, false, true><<<grid, cfg.block, smem, s>>>(a);
         else return cudaErrorInvalidConfiguration;

@@ -44,3 +44,24 @@ def test_tallies_do_not_depend_on_parking(require_gpu, grid, radial, geoms, even
             first = (got, counts)
         assert all(np.array_equal(a, b) for a, b in zip(first[0], got)), kw
         assert counts == first[1], kw
+
+
+@pytest.mark.parametrize("grid", [1, 2])
+@pytest.mark.parametrize("events,photons", [(1, 1), (151, 701)])
+def test_lattice_tallies_do_not_depend_on_the_kernel(require_gpu, grid, events, photons):
+    """Each register budget of the lattice kernel walks the same photons."""
+    rng = np.random.default_rng(events)
+    p = hb.default_params(num_hist=events, det_height=300.0, sensor_refl=0.25)
+    args = (rng.uniform(100, 400, events), rng.uniform(100, 400, events), rng.uniform(-149, 149, events),
+            np.full(events, 1e4), np.arange(1, events + 1), np.full(events, photons))
+    first = None
+    for kw in (dict(), dict(ctas_per_sm=4, chunk=3), dict(ctas_per_sm=3), dict(ctas_per_sm=2),
+               dict(block_size=320, ctas_per_sm=2)):
+        with hb.OpticalTransport(p, count_mode=hb.COUNT_GIVEN, seed=8, column_grid=grid, **kw) as t:
+            t.submit_events_um(*args)
+            t.run_sync()
+            c = t.counters()
+            got = (t.detected_per_primary(), t.prf(0), np.array([v for k, v in c.items() if k != "photon_distance"]))
+        assert c["generated"] == events * photons
+        first = first or got
+        assert all(np.array_equal(a, b) for a, b in zip(first, got)), kw
