@@ -375,10 +375,10 @@ void fit_window(fd2_ctx *c)
 // 256 threads x 4 CTAs per SM (32 warps at 64 registers; 20,000 config-1
 // x-rays 51.6 ms against 54.1 for 224 x 4 and 55.6 for 256 x 3, before the
 // steps below a full exchange were looped), chunks of 16 photons; the square
-// column lattice the same (10,001 config-1 x-rays 68.7 ms against 71.6 for
-// 256 x 3, 76.3 for 320 x 2); several geometries 256 x 3 (configuration 2, 500
-// x-rays: 60.5 ms against 62.5 for 256 x 4); the hexagonal lattice 256 x 3
-// (91.7 ms against 98.2 for 320 x 2), its only kernel above 256 x 2; label
+// column lattice the same (10,001 config-1 x-rays 61.7 ms against 65.1 for
+// 256 x 3, 69.4 for 320 x 2); several geometries 256 x 3 (configuration 2, 500
+// x-rays: 59.4 ms against 61.7 for 256 x 4); the hexagonal lattice 256 x 3
+// (83.0 ms against 90.4 for 320 x 2), its only kernel above 256 x 2; label
 // mode with one geometry (the surrogate's audit) as one geometry, with
 // several 256 x 3.
 static void default_launch(const fd2_ctx *c, int n_geom, fd2::TransportConfig *cfg)
@@ -638,7 +638,8 @@ fd2_status fd2_create(const fd2_params *p, const fd2_options *opt, fd2_ctx **out
     fd2::TransportConfig cfg;
     default_launch(c, 1, &cfg);
     // idle lanes that trigger a refill (20,000 config-1 x-rays: 4 / 6 / 8 / 10
-    // lanes 47.8 / 46.5 / 46.0 / 46.2 ms; the lattice 71.6 / 70.3 / 70.3 / 71.0)
+    // lanes 47.8 / 46.5 / 46.0 / 46.2 ms; the square lattice, 6 / 8 / 10 / 12:
+    // 62.0 / 61.6 / 62.2 / 63.3)
     cfg.refill = c->opt.refill > 0 ? c->opt.refill : 8;
     // photons waiting for the Fresnel part (with a lattice: in the gap) before
     // the warp runs it for them: a full warp's (16 / 24 / 32 photons: 56.7 /

@@ -430,9 +430,9 @@ __device__ __forceinline__ void tally_ended(const TransportArgs &a, const DevGeo
 // warps' time, its hops at 2 to 3, and steps at 25.  20,000 config-1 x-rays
 // (one B200): 59.2 ms before, 51.6 with the wall's photons parked, 46.0 with
 // ended photons tallied together and steps looped, 44.2 with the hops parked,
-// 42.9 with one state word per lane; 10,001 x-rays in the square / hexagonal
-// lattice 102.5 / 142.9 -> 68.7 / 91.7 ms.  Per photon 1,252 -> 959 warp
-// instructions, issue slots 87 % busy, 23 of 32 lanes.  Tallies:
+// 42.9 with one state word per lane, 41.9 with the shorter pull-back; 10,001
+// x-rays in the square / hexagonal lattice 102.5 / 142.9 -> 61.7 / 83.0 ms.
+// Per photon 1,252 -> 930 warp instructions, issue slots 87 % busy.  Tallies:
 // ended photons are tallied 32 at a time (tally_ended) with L2 reductions;
 // with kAgg (tally_mode 1) the fates and the PRF core of geometry 0 are
 // tallied in shared memory first (identical tallies).  kMulti: the
@@ -443,6 +443,8 @@ __device__ __forceinline__ void tally_ended(const TransportArgs &a, const DevGeo
 template <bool kMulti, int kMaxThreads, int kMinBlocks, bool kRadial = false, bool kGrid = false, bool kAgg = false>
 __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(const __grid_constant__ TransportArgs a)
 {
+    // of the column lattices, four CTAs per SM walk the square one only
+    constexpr bool kSquare = kGrid && kMinBlocks == 4;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int win = a.window;
@@ -619,7 +621,6 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                 w.s0 = __float_as_uint(t.x), w.s1 = __float_as_uint(t.y);
                 w.s2 = __float_as_uint(t.z), w.s3 = __float_as_uint(t.w);
                 if (flush) state = !kGrid && hop ? kHops : kWaits;
-                if (kGrid) w.in_gap = flush;
             }
             __syncwarp();
         }
@@ -627,8 +628,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
             // ---- the waiting photons' pass
             if (state == (!kGrid && hop ? kHops : kWaits)) {
                 if constexpr (kGrid) {
-                    state = w.grid_segment(a.g0);
-                    if (state == kFlies && w.in_gap) state = kWaits;
+                    state = w.grid_segment<kSquare, false>(a.g0);
                 } else {
                     state = kMulti ? w.surface_wait(s_geom[tag & kGeomBits], hop, tag) : w.surface_wait(a.g0, hop, tag);
                 }
@@ -709,8 +709,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                     w.start(s.pos.x, s.pos.y, s.pos.z, k, (uint32_t)(a.event_base + s.event), k == 0, key);
                     state = kFlies;
                     if constexpr (kGrid) {
-                        w.grid_place(a.g0);
-                        if (w.in_gap) state = kWaits;
+                        if (w.grid_place<kSquare>(a.g0)) state = kWaits;
                     }
                 }
                 needy &= ~__ballot_sync(kFull, mine);
@@ -735,8 +734,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
             if ((state & 10) == 8) {
                 if constexpr (kGrid) {
                     // explicit column lattice: one segment, of a photon in a column
-                    state = w.grid_segment(a.g0);
-                    if (state == kFlies && w.in_gap) state = kWaits;
+                    state = w.grid_segment<kSquare, true>(a.g0);
                 } else {
                     int f = kNeedsNormal;
                     if (state == kFlies) {
@@ -982,8 +980,8 @@ cudaError_t launch_transport(cudaStream_t s, const TransportConfig &cfg, int sm_
     if (a.g0.grid) {
         // explicit column lattice: single geometry, 256 or 320 threads
         if (multi || a.radial) return cudaErrorInvalidConfiguration;
-        // four CTAs per SM for the square lattice only (10,001 x-rays 68.7 ms,
-        // 71.6 with three): compiled for 64 registers, the test of a hexagonal
+        // four CTAs per SM for the square lattice only (10,001 x-rays 61.7 ms,
+        // 65.1 with three): compiled for 64 registers, the test of a hexagonal
         // lattice's neighbour columns is contracted differently, and 9,092 of
         // 10,001 x-rays would count other photons
         if (cfg.block == 320) transport_kernel<false, 320, 2, false, true><<<grid, cfg.block, smem, s>>>(a);
