@@ -98,21 +98,5 @@ __device__ __forceinline__ void decode_mix(const float *o, Mix &m)
     }
 }
 
-// Probability of radial category j (0..bins; bins = beyond r_max).
-__device__ __forceinline__ float bin_prob(const Mix &m, int j, int bins, float r_max)
-{
-    const float e_lo = radial_edge(j, bins, r_max);
-    const bool top = j >= bins;
-    const float e_hi = top ? 0.0f : radial_edge(j + 1, bins, r_max);
-    float q = 0.0f;
-#pragma unroll
-    for (int k = 0; k < kComponents; ++k) {
-        const Edge lo = edge_at(e_lo, false, m.mu[k], m.sd[k]);
-        const Edge hi = edge_at(e_hi, top, m.mu[k], m.sd[k]);
-        q += m.w[k] * ring_mass(lo, hi, m.mu[k], m.sd[k], nullptr, nullptr) / m.S[k];
-    }
-    return q;
-}
-
 }  // namespace sg
 }  // namespace fd2

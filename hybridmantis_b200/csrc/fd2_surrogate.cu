@@ -67,16 +67,27 @@ struct PointLoss {
 constexpr int kLossWarps = 4;
 constexpr int kSums = 3 * kComponents + 1;  // sums over the categories: A1, Amu, Asd of the components, and the loss
 
+// What the warp of a row shares.
+struct LossShared {
+    float v[kSums][33];         // per category of a pass: M, dM/dmu, dM/dsd of the components, log q
+    float c[32], ny[32];        // y / q and -y of the pass's categories
+    float4 mix[kComponents];    // w, mu, sd, S
+    float cross[kComponents];   // lower tail at the first edge past the ring's radius
+    float4 edge[kComponents];   // the last edge of the pass before: t, tail, pdf
+};
+
 // Loss of one point and its gradients, computed by the 32 lanes of a warp
 // together.  o: the network's outputs; y: normalised radial label over bins + 1
 // categories, used when has_rad (else the point has no radial term).  The
 // radial term is the cross-entropy -sum_j y_j log q_j of the ring mixture's
 // category probabilities q_j = sum_k w_k M_k(e_j, e_j+1) / S_k
-// (fd2_sg_mix.cuh).  A lane holds one edge of the categories, 31 categories a
-// pass, and goes through the components in order; the sums over the categories
-// run in category order, a lane per sum, from shared memory (v: kSums rows).
+// (fd2_sg_mix.cuh).  A lane holds one upper edge of the categories, 32 a pass
+// (96 bins: three passes), and goes through the components in order; the first
+// edge and the category beyond r_max, one each, are a lane per component.  The
+// sums over the categories run in category order, a lane per sum, from shared
+// memory.
 __device__ __forceinline__ PointLoss point_loss(const float *o, float t, const float *y, bool has_rad, int bins,
-                                                float r_max, float lambda, float (*v)[33], float *cj)
+                                                float r_max, float lambda, LossShared &h)
 {
     const int lane = threadIdx.x & 31, k = lane % kComponents;
     PointLoss p;
@@ -108,61 +119,96 @@ __device__ __forceinline__ PointLoss point_loss(const float *o, float t, const f
     const float t0 = -mu / sd;
     const float c0 = normcdff(-t0), p0 = norm_pdf(t0);
     const float S = fmaxf(mu * c0 + sd * p0, 1e-30f);
+    __syncwarp();  // every lane is done with the row before
+    if (lane < kComponents) {
+        // of an edge's two tails only the one away from the ring is kept, and
+        // at the first edge past the ring's radius the other one as well: the
+        // interval that holds the radius reads it (ring_mass)
+        int j = min(max((int)((float)bins * sqrtf(mu / r_max)) - 1, 1), bins);
+        while (j <= bins && radial_edge(j, bins, r_max) < mu) ++j;
+        h.cross[lane] = normcdff((radial_edge(j, bins, r_max) - mu) / sd);
+        const float te = (0.0f - mu) / sd;
+        h.edge[lane] = make_float4(te, normcdff(te >= 0.0f ? -te : te), norm_pdf(te), 0.0f);
+        h.mix[lane] = make_float4(w, mu, sd, S);
+    }
+    __syncwarp();
     // lane c of the first kSums: A1 = sum_j c_j M_j, Amu = sum_j c_j dM_j/dmu,
     // Asd = sum_j c_j dM_j/dsd of component c % 8, and the last the loss
     float sum = 0.0f;
-    for (int j0 = 0; j0 <= bins; j0 += 31) {
-        const int j = j0 + lane;
-        Edge lo;
-        lo.inf = j > bins;
-        lo.e = lo.inf ? 0.0f : radial_edge(j, bins, r_max);
+    for (int j0 = 1; j0 <= bins; j0 += 32) {
+        const int j = j0 + lane, n = min(32, bins + 1 - j0);  // of the pass's categories j - 1 and edges j
+        Edge lo, hi;
+        lo.inf = hi.inf = false;
+        lo.e = radial_edge(j - 1, bins, r_max);
+        hi.e = radial_edge(j, bins, r_max);
         float q = 0.0f;
 #pragma unroll 2
         for (int c = 0; c < kComponents; ++c) {
-            const float wc = __shfl_sync(0xffffffffu, w, c), mc = __shfl_sync(0xffffffffu, mu, c);
-            const float sc = __shfl_sync(0xffffffffu, sd, c), Sc = __shfl_sync(0xffffffffu, S, c);
-            // of an edge's two tails only those that the intervals on its two
-            // sides read (ring_mass): the lower one before the ring's radius,
-            // the upper one past it, both at the first edge past it
-            lo.t = (lo.e - mc) / sc;
-            const bool past = lo.t >= 0.0f;
-            lo.cdf = lo.ccdf = normcdff(past ? -lo.t : lo.t);
-            const bool before = __shfl_up_sync(0xffffffffu, lo.t, 1) < 0.0f;
-            if (past && before) lo.cdf = normcdff(lo.t);
-            lo.pdf = norm_pdf(lo.t);
-            if (lo.inf) {
-                lo.t = 0.0f;
-                lo.cdf = 1.0f;
-                lo.ccdf = 0.0f;
-                lo.pdf = 0.0f;
+            const float4 mix = h.mix[c];
+            const float wc = mix.x, mc = mix.y, sc = mix.z, Sc = mix.w;
+            hi.t = (hi.e - mc) / sc;
+            const bool past = hi.t >= 0.0f;
+            const float tail = normcdff(past ? -hi.t : hi.t);
+            hi.pdf = norm_pdf(hi.t);
+            lo.t = __shfl_up_sync(0xffffffffu, hi.t, 1);
+            lo.cdf = lo.ccdf = __shfl_up_sync(0xffffffffu, tail, 1);
+            lo.pdf = __shfl_up_sync(0xffffffffu, hi.pdf, 1);
+            if (lane == 0) {
+                const float4 e = h.edge[c];
+                lo.t = e.x;
+                lo.cdf = lo.ccdf = e.y;
+                lo.pdf = e.z;
             }
-            Edge hi;
-            hi.t = __shfl_down_sync(0xffffffffu, lo.t, 1);
-            hi.cdf = __shfl_down_sync(0xffffffffu, lo.cdf, 1);
-            hi.ccdf = __shfl_down_sync(0xffffffffu, lo.ccdf, 1);
-            hi.pdf = __shfl_down_sync(0xffffffffu, lo.pdf, 1);
-            hi.e = __shfl_down_sync(0xffffffffu, lo.e, 1);
-            hi.inf = j + 1 > bins;
+            hi.ccdf = tail;
+            hi.cdf = past ? h.cross[c] : tail;
             float dM_mu, dM_sd;
             const float M = ring_mass(lo, hi, mc, sc, &dM_mu, &dM_sd);
             q += wc * M / Sc;
-            v[c][lane] = M;
-            v[kComponents + c][lane] = dM_mu;
-            v[2 * kComponents + c][lane] = dM_sd;
+            h.v[c][lane] = M;
+            h.v[kComponents + c][lane] = dM_mu;
+            h.v[2 * kComponents + c][lane] = dM_sd;
+            __syncwarp();  // lane 0 has read the edge
+            if (lane == n - 1) h.edge[c] = make_float4(hi.t, tail, hi.pdf, 0.0f);
         }
-        const float yj = lane < 31 && j <= bins ? y[j] : 0.0f;
+        const float yj = lane < n ? y[j - 1] : 0.0f;
         const float qe = q + 1e-12f;
-        v[kSums - 1][lane] = yj > 0.0f ? logf(qe) : 0.0f;
-        cj[lane] = yj > 0.0f ? yj / qe : 0.0f;
-        cj[32 + lane] = -yj;
+        h.v[kSums - 1][lane] = yj > 0.0f ? logf(qe) : 0.0f;
+        h.c[lane] = yj > 0.0f ? yj / qe : 0.0f;
+        h.ny[lane] = -yj;
         __syncwarp();
         if (lane < kSums) {
-            const float *f = cj + (lane == kSums - 1 ? 32 : 0), *x = v[lane];
-            const int n = min(31, bins + 1 - j0);
+            const float *f = lane == kSums - 1 ? h.ny : h.c, *x = h.v[lane];
 #pragma unroll 4
             for (int i = 0; i < n; ++i) sum = fmaf(f[i], x[i], sum);
         }
         __syncwarp();
+    }
+    // the category beyond r_max, component k in lane k
+    {
+        const float4 e = h.edge[k];
+        Edge lo, hi;
+        lo.t = e.x;
+        lo.cdf = lo.ccdf = e.y;
+        lo.pdf = e.z;
+        lo.e = radial_edge(bins, bins, r_max);
+        lo.inf = false;
+        hi.t = 0.0f;
+        hi.cdf = 1.0f;
+        hi.ccdf = 0.0f;
+        hi.pdf = 0.0f;
+        hi.e = 0.0f;
+        hi.inf = true;
+        float dM_mu, dM_sd;
+        const float M = ring_mass(lo, hi, mu, sd, &dM_mu, &dM_sd);
+        const float part = w * M / S;
+        float q = 0.0f;
+#pragma unroll
+        for (int c = 0; c < kComponents; ++c) q += __shfl_sync(0xffffffffu, part, c);
+        const float yj = y[bins], qe = q + 1e-12f;
+        const float cj = yj > 0.0f ? yj / qe : 0.0f;
+        const float x = lane < kComponents ? M : lane < 2 * kComponents ? dM_mu : dM_sd;
+        if (lane < kSums - 1) sum = fmaf(cj, x, sum);
+        else if (lane == kSums - 1) sum = fmaf(-yj, yj > 0.0f ? logf(qe) : 0.0f, sum);
     }
     const float A1 = __shfl_sync(0xffffffffu, sum, k), Amu = __shfl_sync(0xffffffffu, sum, kComponents + k);
     const float Asd = __shfl_sync(0xffffffffu, sum, 2 * kComponents + k);
@@ -235,10 +281,12 @@ __global__ void gather_kernel(const float *__restrict__ feat, const int32_t *__r
 
 // Loss (summed into acc[0..2] = total, detection, radial) and, when dout is
 // set, dL/dout / b as BF16 [b][64].  A warp per row (point_loss); instruction
-// issue bounds it (normal tails, exponentials and divisions of 97 x 8 bin
-// masses).  A thread per row left 8,192 threads, 64 per SM, that waited for
-// their dependent instructions: 8,192 rows 588 us, eight lanes per row 136,
-// this 106.
+// issue bounds it (normal tails, exponentials and divisions of 96 x 8 bin
+// masses, issue slots 78 % busy).  8,192 rows: a thread per row left 64 threads
+// per SM that waited for their dependent instructions, 588 us; eight lanes per
+// row 136; a warp per row with 31 categories a pass (four passes for 97) and
+// both tails of each crossed edge in the pass 105 us and 88.5 M instructions,
+// this 76 us and 59.4 M.
 __global__ void __launch_bounds__(32 * kLossWarps) loss_kernel(const float *__restrict__ out, int ldo,
                                                                const float *__restrict__ target,
                                                                const float *__restrict__ ylab,
@@ -246,12 +294,13 @@ __global__ void __launch_bounds__(32 * kLossWarps) loss_kernel(const float *__re
                                                                float r_max, float lambda, int b, float scale,
                                                                __nv_bfloat16 *__restrict__ dout, double *acc)
 {
-    __shared__ float v[kLossWarps][kSums][33], cj[kLossWarps][64], s[3][kLossWarps];
+    __shared__ LossShared h[kLossWarps];
+    __shared__ float s[3][kLossWarps];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, r = blockIdx.x * kLossWarps + wid;
     PointLoss p{};
     if (r < b) {
         p = point_loss(out + (int64_t)r * ldo, target[r], ylab + (int64_t)r * (bins + 1), has_rad[r] > 0.0f, bins,
-                       r_max, lambda, v[wid], cj[wid]);
+                       r_max, lambda, h[wid]);
         if (dout) {
             __nv_bfloat16 *d = dout + (int64_t)r * kOutPad;
             if (lane < kComponents) {

@@ -31,6 +31,11 @@ def test_loss_and_gradient_at_tile_edges(require_gpu, rows, bins):
     assert np.linalg.norm(g - wg) <= 2e-3 * np.linalg.norm(wg)
 
 
+@pytest.mark.parametrize("rows,bins", [(6, 2), (7, 33), (8, 64), (9, 65), (10, 95), (11, 97)])
+def test_loss_and_gradient_around_passes_of_32_edges(require_gpu, rows, bins):
+    test_loss_and_gradient_at_tile_edges(None, rows, bins)
+
+
 @pytest.mark.parametrize("rows", [1, 127, 129, 8193, 37887, 37891, 75780])
 def test_predict_at_pass_edges(require_gpu, rows):
     f = np.random.default_rng(rows).uniform(-1, 1, (rows, 8)).astype(np.float32)
