@@ -430,10 +430,11 @@ __device__ __forceinline__ void tally_ended(const TransportArgs &a, const DevGeo
 // warps' time, its hops at 2 to 3, and steps at 25.  20,000 config-1 x-rays
 // (one B200): 59.2 ms before, 51.6 with the wall's photons parked, 46.0 with
 // ended photons tallied together and steps looped, 44.2 with the hops parked,
-// 42.9 with one state word per lane, 41.9 with the shorter pull-back; 10,001
-// x-rays in the square / hexagonal lattice 102.5 / 142.9 -> 61.7 / 83.0 ms.
-// Per photon 1,252 -> 940 warp instructions at 23 of 32 lanes, issue slots 87 %
-// busy.  Tallies:
+// 42.9 with one state word per lane, 41.9 with the shorter pull-back, 40.2 with
+// selects for branches that most lanes take and a refill's photons started
+// together; 10,001 x-rays in the square / hexagonal lattice 102.5 / 142.9 ->
+// 61.7 / 83.0 ms.  Per photon 1,252 -> 890 warp instructions at 23 of 32 lanes,
+// issue slots 87 % busy.  Tallies:
 // ended photons are tallied 32 at a time (tally_ended) with L2 reductions;
 // with kAgg (tally_mode 1) the fates and the PRF core of geometry 0 are
 // tallied in shared memory first (identical tallies).  kMulti: the
@@ -572,23 +573,16 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
             const int n_none = 32 - __popc(live);
             const int left = max(n_ready - n_held, 0), hleft = max(n_hready - n_hops, 0);
             const int taken = min(left, n_none), htaken = min(hleft, n_none - taken);
-            if (!((run >> lane) & 1u)) {
-                const unsigned same = state == kWaits ? held : !kGrid && state == kHops ? hops : ~live;
-                const int rank = __popc(same & lanemask_lt());
-                bool got;
-                if (state == kWaits) {
-                    at = n_wait + rank;
-                    got = rank < n_ready;
-                } else if (!kGrid && state == kHops) {
-                    at = kParkKind + n_hop + rank;
-                    got = rank < n_hready;
-                } else {
-                    got = rank < taken + htaken;
-                    if (got) at = rank < taken ? n_wait + n_ready - 1 - rank
-                                               : kParkKind + n_hop + n_hready - 1 - (rank - taken);
-                }
-                state = got ? kFlies : 0;
-            }
+            const bool flying = (run >> lane) & 1u;
+            const bool at_wall = state == kWaits, hopper = !kGrid && state == kHops;
+            const unsigned same = at_wall ? held : hopper ? hops : ~live;
+            const int rank = __popc(same & lanemask_lt());
+            const bool got = rank < (at_wall ? n_ready : hopper ? n_hready : taken + htaken);
+            const int own = (at_wall ? n_wait : kParkKind + n_hop) + rank;
+            const int next = (rank < taken ? n_wait + n_ready : kParkKind + n_hop + n_hready + taken) - 1 - rank;
+            at = at_wall || hopper ? own : got ? next : -1;
+            at = flying ? -1 : at;
+            state = flying ? state : got ? kFlies : 0;
             moved = n_held + n_hops + taken + htaken;
             n_wait += n_held;
             n_hop += n_hops;
@@ -639,7 +633,11 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
         // ---- hand out photons to idle lanes
         unsigned needy = __ballot_sync(kFull, state == 0);
         if (deal && needy && (__popc(needy) >= a.refill || needy == kFull)) {
+            // (which photon first; they start together below, also where the
+            // lanes' photons come from several chunks)
             int slot = m.slot, len = m.len;
+            bool fresh = false;
+            uint32_t first = 0;  // the photon's number in its event
             uint32_t used = m.used;
             while (needy) {
                 if (slot >= len) {
@@ -703,15 +701,13 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                 const bool mine = ((needy >> lane) & 1u) && rank < take;
                 if (mine) {
                     const Slot &s = m.ring[slot];
-                    const uint32_t k = s.first + used + rank;
+                    first = s.first + used + rank;
                     tag = s.geom;
                     event = s.event;
-                    if (kMulti) w.dist = 0.0f;
-                    w.start(s.pos.x, s.pos.y, s.pos.z, k, (uint32_t)(a.event_base + s.event), k == 0, key);
-                    state = kFlies;
-                    if constexpr (kGrid) {
-                        if (w.grid_place<kSquare>(a.g0)) state = kWaits;
-                    }
+                    w.px = s.pos.x;
+                    w.py = s.pos.y;
+                    w.pz = s.pos.z;
+                    fresh = true;
                 }
                 needy &= ~__ballot_sync(kFull, mine);
                 used += take;
@@ -720,6 +716,18 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) transport_kernel(cons
                 m.slot = slot;
                 m.len = len;
                 m.used = used;
+            }
+            if (fresh) {
+                if (kMulti) w.dist = 0.0f;
+                w.start(w.px, w.py, w.pz, first, (uint32_t)(a.event_base + event), first == 0, key);
+                state = kFlies;
+                if constexpr (kGrid) {
+                    if (w.grid_place<kSquare>(a.g0)) state = kWaits;
+                } else if constexpr (kMulti) {
+                    w.fill_budget(s_geom[tag & kGeomBits]);
+                } else {
+                    w.fill_budget(a.g0);
+                }
             }
             __syncwarp();
             supply = n_ready > 0 || !exhausted;
