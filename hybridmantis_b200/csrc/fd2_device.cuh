@@ -376,6 +376,10 @@ struct Walker {
     // Written as a state machine so that the kernel holds one copy of each
     // part (hop, sensor, hop after the sensor, next normal, top reflector):
     // the walk's instruction fetch grows with the kernel's code size.
+    // The parts stand in the order photons pass them, so that one round of the
+    // loop takes most photons through and the lanes meet at the next normal (a
+    // part per round: 20,000 config-1 x-rays with a reflecting sensor 44.9 ms,
+    // this 44.6).
     template <class G>
     __device__ __forceinline__ int leave_column(const G &g)
     {
@@ -421,7 +425,8 @@ struct Walker {
                 } else {
                     dist += d;
                 }
-            } else if (st == kSensor) {
+            }
+            if (st == kSensor) {
                 // sensor between columns: reflect with sensorRefl, else detect
                 if (!(g.sensor_refl > 0.0f && u() < g.sensor_refl)) {
                     return kDetect;
@@ -429,7 +434,8 @@ struct Walker {
                 dz = -dz;
                 renorm(dx, dy, dz);
                 st = kSensorHop;
-            } else if (st == kSensorHop) {
+            }
+            if (st == kSensorHop) {
                 const float sx = px, sy = py, sz = pz;
                 const float hop = fmaf(u(), g.d_span, g.d_min);
                 px = fmaf(dx, hop, sx);
@@ -449,7 +455,8 @@ struct Walker {
                     counts |= kAfterHop;
                     st = kNormal;
                 }
-            } else if (st == kNormal) {
+            }
+            if (st == kNormal) {
                 const bool after_sensor = (counts & kAfterHop) != 0u, side_hop = (counts & kSideHop) != 0u;
                 int t = after_sensor ? 0 : (int)((side_hop ? counts : counts >> 8) & 0xffu);
                 // after a sensor hop: around the hop's own reversed direction
@@ -465,7 +472,8 @@ struct Walker {
                         return kLost;
                     st = kEnd;
                 }
-            } else if (st == kAfterSensor) {
+            }
+            if (st == kAfterSensor) {
                 counts &= ~kAfterHop;
                 if (!(counts & kFromEnd)) {
                     // a sensor met during the hop: the next normal follows
@@ -481,8 +489,9 @@ struct Walker {
                     if (!at_top(g)) return kFlies;
                     st = kEnd;
                 }
-            } else {
-                // kEnd: top reflector / sensor at the end of the hop
+            }
+            if (st == kEnd) {
+                // top reflector / sensor at the end of the hop
                 if (at_top(g)) {
                     if (g.top_absfrac > 0.0f && u() < g.top_absfrac) return kAbsTop;
                     dz = -fabsf(2.0f * u() - 1.0f);

@@ -430,7 +430,7 @@ __device__ __forceinline__ void tally_ended(const TransportArgs &a, const DevGeo
 // warps' time, its hops at 2 to 3, and steps at 25.  20,000 config-1 x-rays
 // (one B200): 59.2 ms before, 51.6 with the wall's photons parked, 46.0 with
 // ended photons tallied together and steps looped, 44.2 with the hops parked,
-// 42.9 with one state word per lane, 41.9 with the shorter pull-back, 40.2 with
+// 42.9 with one state word per lane, 41.9 with the shorter pull-back, 40.0 with
 // selects for branches that most lanes take and a refill's photons started
 // together; 10,001 x-rays in the square / hexagonal lattice 102.5 / 142.9 ->
 // 61.7 / 83.0 ms.  Per photon 1,252 -> 890 warp instructions at 23 of 32 lanes,
