@@ -20,10 +20,10 @@
 //     d' = -cos(t_t) n - (sin t_t / sin t_i)(d + cos(t_i) n);
 //   * the wall quadratic uses the cancellation-free root, with the
 //     discriminant recomputed in FP64 when it nearly cancels;
-//   * the whole walk is inlined around one photon held in registers, with a
-//     single site for the column change and for the new-column normal.
-// Tallies are not touched here: a step returns the photon's fate (and
-// pixel) and the kernel aggregates them per warp.
+//   * the whole walk is inlined around one photon held in registers, and its
+//     rarer, longer parts can run later, from the photon's state alone.
+// Tallies are not touched here: a step returns the photon's fate and the
+// kernel tallies ended photons together.
 #pragma once
 
 #include <cstdint>

@@ -17,7 +17,7 @@ struct TransportConfig {
     int chunk = 32;      // photons per work-queue chunk
     int refill = 1;      // idle lanes that trigger a warp refill
     int window = 0;      // shared-memory PRF window edge (0 = off)
-    int fresnel = 8;     // parked lanes that trigger the warp's Fresnel pass
+    int fresnel = 32;    // waiting photons of a warp that start the pass for them
     bool aggregate = false;  // single geometry: warp-aggregated, shared-memory privatised tallies
 };
 
@@ -44,7 +44,7 @@ struct TransportArgs {
     int pull_shift;              // a warp's refill takes (chunks left) >> pull_shift, 1 to 32 (set by launch_transport)
     int chunk;
     int refill;
-    int fresnel_batch;           // parked lanes before the Fresnel pass runs
+    int fresnel_batch;           // waiting photons of a warp that start the pass for them
     int window;                  // window edge (0 = off), applies to geometry 0
     int win_x0, win_y0;          // window origin in pixels
     const volatile int *abort_flag;
