@@ -432,9 +432,9 @@ __device__ __forceinline__ void tally_ended(const TransportArgs &a, const DevGeo
 // ended photons tallied together and steps looped, 44.2 with the hops parked,
 // 42.9 with one state word per lane, 41.9 with the shorter pull-back, 40.0 with
 // selects for branches that most lanes take and a refill's photons started
-// together; 10,001 x-rays in the square / hexagonal lattice 102.5 / 142.9 ->
-// 61.7 / 83.0 ms.  Per photon 1,252 -> 890 warp instructions at 23 of 32 lanes,
-// issue slots 87 % busy.  Tallies:
+// together, 38.9 with a step's fate and depth tests only where they matter; 10,001 x-rays in the square / hexagonal lattice 102.5 / 142.9 ->
+// 61.1 / 83.1 ms.  Per photon 1,252 -> 863 warp instructions at 23.5 of 32 lanes
+// (5,000 x-rays), issue slots 87 % busy.  Tallies:
 // ended photons are tallied 32 at a time (tally_ended) with L2 reductions;
 // with kAgg (tally_mode 1) the fates and the PRF core of geometry 0 are
 // tallied in shared memory first (identical tallies).  kMulti: the
