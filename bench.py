@@ -276,7 +276,7 @@ def parity_vs_reference(es, nphot, nev, ref_tallies, device, seed):
 
 
 # DRAM bytes per photon of the transport kernel: dram__bytes_read.sum +
-# dram__bytes_write.sum of one ncu capture (26,715,904 B for 46,784,158
+# dram__bytes_write.sum of one ncu capture (26,714,880 B for 46,784,158
 # photons of the config-1 stream, 20,000 x-rays, steady state); the traffic is
 # one event record per chunk and grows in proportion to the photons.
 TRANSPORT_DRAM_BYTES_PER_PHOTON = 0.57
@@ -287,9 +287,9 @@ TRANSPORT_DRAM_BYTES_PER_PHOTON = 0.57
 # inst_executed), warp instructions per photon (smsp__inst_executed.sum /
 # photons) and the tallies' L2 reductions against their peak
 # (lts__t_sectors_op_red.avg.pct_of_peak_sustained_elapsed).
-TRANSPORT_NCU = {"issue_slot_utilisation": 0.882, "fp32_pipe_utilisation": 0.321,
-                 "lanes_per_instruction": 23.84, "warp_instructions_per_photon": 866.1,
-                 "l2_reduction_pct_of_peak": 0.23,
+TRANSPORT_NCU = {"issue_slot_utilisation": 0.884, "fp32_pipe_utilisation": 0.323,
+                 "lanes_per_instruction": 23.80, "warp_instructions_per_photon": 843.0,
+                 "l2_reduction_pct_of_peak": 0.24,
                  "source": "ncu --clock-control none on 20,000 config-1 x-rays "
                            "(transport_kernel<false,256,4,false,false,false>, default launch)"}
 
