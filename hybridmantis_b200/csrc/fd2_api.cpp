@@ -1118,7 +1118,7 @@ fd2_status fd2_get_timing(fd2_ctx *c, fd2_timing *out)
         FD2_CUDA(c, cudaEventElapsedTime(&out->pipeline_ms, c->ev_start, c->ev_end));
     }
     out->photons = c->last_photons;
-    out->grid = c->sm_count * (c->cfg.grid_ctas ? c->cfg.grid_ctas : c->cfg.ctas_per_sm);
+    out->grid = c->sm_count * fd2::transport_ctas(c->cfg, (int)c->geoms.size(), c->d_radial != nullptr);
     out->block = c->cfg.block;
     out->chunk = c->cfg.chunk;
     out->refill = c->cfg.refill;

@@ -93,6 +93,8 @@ cudaError_t launch_fill_chunks(cudaStream_t s, int64_t n, int chunk, const int32
                                const unsigned long long *offsets, uint2 *chunks, int64_t capacity,
                                int *status);
 cudaError_t launch_transport(cudaStream_t s, const TransportConfig &cfg, int sm_count, const TransportArgs &a);
+// The CTAs per SM that it launches.
+int transport_ctas(const TransportConfig &cfg, int n_geom, bool label);
 // Sets the kernel's shared-memory limit; call outside stream capture.
 cudaError_t prepare_transport(const TransportConfig &cfg, int n_geom);
 cudaError_t launch_bump_run_tag(cudaStream_t s, uint32_t *run_tag);

@@ -967,18 +967,25 @@ size_t transport_smem_bytes(const TransportConfig &cfg, int n_geom)
     return SmemLayout(cfg.block, n_geom, cfg.window).total;
 }
 
+// The CTAs per SM of a launch.  Label mode has one kernel for one geometry (the
+// surrogate's audit), with the production run's four CTAs per SM whatever
+// ctas_per_sm says, and one for several (training labels) with three (80
+// registers without a spill; 64 geometries x 100 points x 4,000 photons:
+// 22.9 ms, 28.5 ms with two).  A single geometry never goes to a kMulti kernel:
+// SmemLayout keeps its geometry table for several geometries only.
+int transport_ctas(const TransportConfig &cfg, int n_geom, bool label)
+{
+    if (cfg.grid_ctas) return cfg.grid_ctas;
+    if (label) return n_geom > 1 ? 3 : 4;
+    return cfg.ctas_per_sm;
+}
+
 cudaError_t launch_transport(cudaStream_t s, const TransportConfig &cfg, int sm_count, const TransportArgs &args)
 {
     TransportArgs a = args;
     const size_t smem = transport_smem_bytes(cfg, a.n_geom);
     const bool multi = a.n_geom > 1;
-    // label mode, 256 threads: one geometry (the surrogate's audit) as the
-    // production kernel, four CTAs per SM, else (training labels) three (80
-    // registers without a spill; 64 geometries x 100 points x 4,000 photons:
-    // 22.9 ms, 28.5 ms with two)
-    const int per_sm_label = !multi && cfg.ctas_per_sm >= 4 ? 4 : 3;
-    const unsigned grid = (unsigned)(sm_count * (cfg.grid_ctas ? cfg.grid_ctas
-                                                    : a.radial ? per_sm_label : cfg.ctas_per_sm));
+    const unsigned grid = (unsigned)(sm_count * transport_ctas(cfg, a.n_geom, a.radial != nullptr));
     a.refill = std::min(std::max(a.refill, 1), 32);
     a.fresnel_batch = std::min(std::max(a.fresnel_batch, 1), kPark);
     // a refill takes 1 / 2^pull_shift of the chunks left: at most half of a
@@ -1001,7 +1008,7 @@ cudaError_t launch_transport(cudaStream_t s, const TransportConfig &cfg, int sm_
         else return cudaErrorInvalidConfiguration;
     } else if (a.radial) {
         if (cfg.block > 256) return cudaErrorInvalidConfiguration;
-        if (per_sm_label == 4) transport_kernel<false, 256, 4, true><<<grid, cfg.block, smem, s>>>(a);
+        if (!multi) transport_kernel<false, 256, 4, true><<<grid, cfg.block, smem, s>>>(a);
         else transport_kernel<true, 256, 3, true><<<grid, cfg.block, smem, s>>>(a);
     } else if (!multi && cfg.aggregate) {
         // warp-aggregated, shared-memory privatised tallies (tally_mode 1)
