@@ -708,6 +708,7 @@ fd2_status fd2_set_geometries(fd2_ctx *c, const fd2_geometry *g, int32_t n)
     if (st != FD2_OK) return st;
     fd2::TransportConfig k = c->cfg;
     default_launch(c, n, &k);
+    c->tuned = false;  // the launch shape is the default again
     return set_config(c, k);
 }
 
@@ -728,9 +729,15 @@ static fd2_status submit_common(fd2_ctx *c, int64_t n, const float *xs, const fl
     if (G == 1) c->hist_per_geom[0] = c->params.num_hist;
     // A run of a few photons per lane takes as long as its longest walks, which
     // go faster beside fewer warps: two CTAs per SM below 500,000 expected
-    // photons (config 0, 25 / 100 / 400 x-rays: 0.28 / 0.41 / 0.70 ms against
-    // 0.34 / 0.48 / 0.73 with four; 936,000 photons 1.55 against 1.48)
-    const bool few = c->mu_total < 5e5 && !c->opt.ctas_per_sm && !c->tuned && G == 1 && !c->opt.column_grid;
+    // photons (two against four CTAs: config 0 0.26 / 0.38 / 0.57 ms against 0.30 /
+    // 0.46 / 0.63 at 50,000 / 199,000 / 488,000 photons, config 1 0.37 / 0.56 /
+    // 0.88 against 0.44 / 0.67 / 0.91 at 54,000 / 208,000 / 499,000, the same
+    // order with a reflecting sensor, 600 um of CsI and in label mode; config 0
+    // 1.55 against 1.48 at 936,000).  With the default block only: blocks of
+    // 128 threads already are half of those warps (config 1 at 409,000 photons
+    // 1.01 ms against 0.77), of 32 an eighth (2.81 against 1.58)
+    const bool few = c->mu_total < 5e5 && !c->opt.ctas_per_sm && !c->opt.block_size && !c->tuned && G == 1 &&
+                     !c->opt.column_grid;
     c->cfg.grid_ctas = few ? std::min(2, c->cfg.ctas_per_sm) : 0;
     if (xs) choose_window(c, xs, ys, geom, n);
     else choose_window_sums(c, sums ? sums[0] : 0.0, sums ? sums[1] : 0.0, n);
