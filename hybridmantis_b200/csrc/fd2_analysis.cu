@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <mutex>
 #include <vector>
 
@@ -207,11 +208,9 @@ __global__ void __launch_bounds__(kThreads) dft_cols_kernel(const double2 *__res
 // frequency u + shift (folded to (-wrap / 2, wrap / 2] with wrap > 0), column
 // frequency k >= 0, whose mirror (-u, -k) the map leaves out and counts as a
 // second value (`single`: the column frequency besides 0 that is its own
-// mirror, or -1).  Block b averages the values whose radius rounds to b, each
-// divided by *norm where given.
+// mirror, or -1).  Block b averages the values whose radius rounds to b.
 __global__ void __launch_bounds__(kThreads) radial_kernel(const double *__restrict__ map, int nu, int nk, int shift,
-                                                          int wrap, int single, const double *__restrict__ norm,
-                                                          double *__restrict__ out)
+                                                          int wrap, int single, double *__restrict__ out)
 {
     __shared__ double part[kThreads];
     __shared__ int count[kThreads];
@@ -243,15 +242,12 @@ __global__ void __launch_bounds__(kThreads) radial_kernel(const double *__restri
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        const double v = count[0] > 0 ? part[0] / count[0] : 0.0;
-        out[b] = norm ? v / *norm : v;
-    }
+    if (threadIdx.x == 0) out[b] = count[0] > 0 ? part[0] / count[0] : 0.0;
 }
 
-// out[k] = |h(k, 0)| / total, out[n + k] = |h(0, k)| / total, out[2 n] = total
-// from the map of |h| (row frequency 0 at row `zero`): the transforms of the
-// two line spread functions (row and column sums).  total: the image's sum.
+// out[k] = |h(k, 0)|, out[n + k] = |h(0, k)| from the map of |h| (row frequency
+// 0 at row `zero`): the transforms of the two line spread functions (row and
+// column sums); out[2 n]: the image's sum.
 __global__ void axes_kernel(const double *__restrict__ map, int nk, int zero, const double2 *__restrict__ a, int nrows,
                             double *__restrict__ out)
 {
@@ -264,12 +260,11 @@ __global__ void axes_kernel(const double *__restrict__ map, int nk, int zero, co
         if (threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
         __syncthreads();
     }
-    const double total = part[0];
     for (int k = threadIdx.x; k < nk; k += kThreads) {
-        out[k] = map[(int64_t)(zero + k) * nk] / total;
-        out[nk + k] = map[(int64_t)zero * nk + k] / total;
+        out[k] = map[(int64_t)(zero + k) * nk];
+        out[nk + k] = map[(int64_t)zero * nk + k];
     }
-    if (threadIdx.x == 0) out[2 * nk] = total;
+    if (threadIdx.x == 0) out[2 * nk] = part[0];
 }
 
 // Per-pixel mean over n images (x n stacked images of `count` values).
@@ -426,6 +421,25 @@ fd2_status to_status(cudaError_t e)
                                                                       : FD2_ERR_CUDA;
 }
 
+// The image's sum, pixel by pixel: an image has signal when it is positive and finite.
+double image_sum(const double *image, int64_t n)
+{
+    double total = 0.0;
+    for (int64_t p = 0; p < n; ++p) total += image[p];
+    return total;
+}
+
+bool any_sign_bit(const double *image, int64_t n)
+{
+    uint64_t any = 0;
+    for (int64_t p = 0; p < n; ++p) {
+        uint64_t b;
+        std::memcpy(&b, image + p, sizeof b);
+        any |= b;
+    }
+    return any >> 63;
+}
+
 unsigned tiles(int64_t n, int tile) { return (unsigned)((n + tile - 1) / tile); }
 
 unsigned blocks_for(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + kThreads - 1) / kThreads, 1 << 20)); }
@@ -441,14 +455,11 @@ fd2_status fd2_mtf(int32_t device, const double *image, int32_t xdim, int32_t yd
         return FD2_ERR_INVALID_ARGUMENT;
     const int N = std::max(xdim, ydim);
     if (n_freq > N / 2 + 1) return FD2_ERR_INVALID_ARGUMENT;
-    if (freq_per_mm)
-        for (int k = 0; k < n_freq; ++k) freq_per_mm[k] = 1000.0 * k / (N * pixel_um);
     const int64_t npx = (int64_t)xdim * ydim;
     cudaError_t e = cudaSetDevice(device);
     if (e != cudaSuccess) {
         // an image without signal is refused whatever the device
-        double total = 0.0;
-        for (int64_t p = 0; p < npx; ++p) total += image[p];
+        const double total = image_sum(image, npx);
         return !(total > 0.0) || !std::isfinite(total) ? FD2_ERR_INVALID_ARGUMENT : to_status(e);
     }
     const int K = n_freq, V = 2 * K - 1;
@@ -460,7 +471,7 @@ fd2_status fd2_mtf(int32_t device, const double *image, int32_t xdim, int32_t yd
     if ((e = d.open(device, l.bytes)) != cudaSuccess) return to_status(e);
     const cudaStream_t s = d.stream;
     double2 *tw = d.at<double2>(o_tw), *a = d.at<double2>(o_a);
-    // out: mtf_x, mtf_y, the image's sum, mtf_r
+    // out: mtf_x, mtf_y, the image's sum, mtf_r, all but the division by the sum
     double *map = d.at<double>(o_map), *out = d.at<double>(o_out);
     e = cudaMemcpyAsync(d.at<double>(o_img), image, sizeof(double) * npx, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
@@ -471,9 +482,10 @@ fd2_status fd2_mtf(int32_t device, const double *image, int32_t xdim, int32_t yd
                                                                                       0, map);
         axes_kernel<<<1, kThreads, 0, s>>>(map, K, K - 1, a, xdim, out);
         if (mtf_r)
-            radial_kernel<<<(unsigned)K, kThreads, 0, s>>>(map, V, K, 1 - K, 0, -1, out + 2 * K, out + 2 * K + 1);
+            radial_kernel<<<(unsigned)K, kThreads, 0, s>>>(map, V, K, 1 - K, 0, -1, out + 2 * K + 1);
         e = cudaGetLastError();
     }
+    const bool sign = any_sign_bit(image, npx);  // while the kernels run
     std::vector<double> r(3 * (size_t)K + 1);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(r.data(), out, sizeof(double) * (mtf_r ? r.size() : 2 * (size_t)K + 1),
@@ -481,11 +493,19 @@ fd2_status fd2_mtf(int32_t device, const double *image, int32_t xdim, int32_t yd
     const cudaError_t e2 = cudaStreamSynchronize(s);
     if (e == cudaSuccess) e = e2;
     if (e != cudaSuccess) return to_status(e);
-    const double total = r[2 * (size_t)K];
+    // The device's sum, in rows, is the image's where nothing cancels.  With
+    // negative values (or no number) the order decides a sum near zero, and with
+    // it whether the image has signal: then pixel by pixel (0.25 ms of host time
+    // at 501 x 501, which is why it is not always taken).
+    double total = r[2 * (size_t)K];
+    if (sign || !(total > 0.0) || !std::isfinite(total)) total = image_sum(image, npx);
     if (!(total > 0.0) || !std::isfinite(total)) return FD2_ERR_INVALID_ARGUMENT;
-    if (mtf_x) std::copy(r.begin(), r.begin() + K, mtf_x);
-    if (mtf_y) std::copy(r.begin() + K, r.begin() + 2 * K, mtf_y);
-    if (mtf_r) std::copy(r.begin() + 2 * K + 1, r.end(), mtf_r);
+    for (int k = 0; k < K; ++k) {
+        if (freq_per_mm) freq_per_mm[k] = 1000.0 * k / (N * pixel_um);
+        if (mtf_x) mtf_x[k] = r[(size_t)k] / total;
+        if (mtf_y) mtf_y[k] = r[(size_t)K + k] / total;
+        if (mtf_r) mtf_r[k] = r[2 * (size_t)K + 1 + k] / total;
+    }
     return FD2_OK;
 }
 
@@ -553,7 +573,7 @@ fd2_status fd2_nnps(int32_t device, const double *images, int32_t n_images, int3
         const double factor = px_mm * px_mm / ((double)R * R) * corr / ((double)n * nroi);
         power_map_kernel<<<blocks_for(per_region), kThreads, 0, s>>>(acc, planes, R, H, sums, nroi, factor, half,
                                                                      out2d, out + K);
-        radial_kernel<<<(unsigned)K, kThreads, 0, s>>>(half, R, H, 0, R, R % 2 == 0 ? R / 2 : -1, nullptr, out);
+        radial_kernel<<<(unsigned)K, kThreads, 0, s>>>(half, R, H, 0, R, R % 2 == 0 ? R / 2 : -1, out);
         e = cudaGetLastError();
     }
     std::vector<double> r((size_t)K + 1);
