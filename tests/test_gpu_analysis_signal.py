@@ -1,6 +1,8 @@
 """Which images have signal: the image's sum, added pixel by pixel, is positive
 and finite (MTF).  Images whose values cancel make the order of the additions
 visible; a refused call leaves its outputs alone."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -48,3 +50,37 @@ def test_an_image_without_signal_is_refused_untouched(require_gpu, value):
     img[4, 4] = value
     st, out = _mtf(img, 3)
     assert st == (0 if np.isfinite(value) else INVALID)
+
+
+def _region_mean(imgs, roi, across):
+    """Mean signal as fd2_nnps adds it up: pixel t of a region to one of 128
+    partial sums, those in a tree, the regions in order."""
+    mean = imgs[0] if len(imgs) == 1 else (imgs[0] + imgs[1]) / 2.0
+    total = 0.0
+    for q in range(across):
+        v = mean[:roi, q * roi:(q + 1) * roi].ravel()
+        part = np.zeros(128)
+        for i in range(0, len(v), 128):
+            part[:len(v[i:i + 128])] += v[i:i + 128]
+        w = 64
+        while w:
+            part[:w] += part[w:2 * w]
+            w //= 2
+        total += float(part[0])
+    return total / (float(across) * roi * roi)
+
+
+# of these 80 stacks 4 have means of other signs with 1,024 partial sums
+@pytest.mark.parametrize("seed", range(40))
+@pytest.mark.parametrize("n", [1, 2])
+def test_cancelling_flat_fields_are_decided_in_a_fixed_order(require_gpu, seed, n):
+    imgs = np.random.default_rng(seed).normal(0.0, 1.0, (n, 35, 70))
+    imgs -= imgs[:, :33, :66].mean()
+    want = _region_mean(imgs, 33, 2)
+    m = ctypes.c_double()
+    r = np.zeros(17)
+    st = hb.load().fd2_nnps(0, ptr(imgs), n, 35, 70, 1.0, 33, 0, 0, 1, 2, 17, None, ptr(r), None,
+                            ctypes.byref(m))
+    assert st == (0 if want > 0.0 else INVALID)
+    if st == 0:
+        assert m.value == want
