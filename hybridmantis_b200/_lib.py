@@ -187,7 +187,7 @@ EXPORTED = [
     "fd2_sg_get_hull", "fd2_sg_set_hull", "fd2_sg_save", "fd2_sg_load", "fd2_sg_loss_grad", "fd2_sg_predict",
     "fd2_sg_set_edge", "fd2_sg_get_edge",
     "fd2_sg_run",
-    "fd2_mtf", "fd2_nnps",
+    "fd2_mtf", "fd2_nnps", "fd2_analysis_release",
     "fd2_submit_events_device",
     "fd2_xray_load_material", "fd2_xray_save_material", "fd2_xray_free_material", "fd2_xray_material_get_info",
     "fd2_xray_attenuation", "fd2_xray_electron_tables", "fd2_xray_default_options", "fd2_xray_create",
@@ -281,6 +281,7 @@ def load():
         "fd2_nnps": (ctypes.c_int, [ctypes.c_int32, vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_double,
                                     ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                     ctypes.c_int32, vp, vp, vp, P(ctypes.c_double)]),
+        "fd2_analysis_release": (ctypes.c_int, [ctypes.c_int32]),
         "fd2_submit_events_device": (ctypes.c_int, [vp, vp, vp, vp, vp, vp, ctypes.c_int64]),
         "fd2_xray_load_material": (ctypes.c_int, [ctypes.c_char_p, P(vp)]),
         "fd2_xray_save_material": (ctypes.c_int, [vp, ctypes.c_char_p]),

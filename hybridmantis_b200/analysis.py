@@ -56,6 +56,11 @@ def nnps(images, pixel_um: float, roi: int, x0: int | None = None, y0: int | Non
     return {"freq": freq, "nnps_r": nr, "nnps_2d": n2, "mean_signal": m.value}
 
 
+def release(device: int = 0) -> None:
+    """Free the device memory that mtf and nnps keep between calls."""
+    check(_lib.load().fd2_analysis_release(device), "release")
+
+
 def flat_field(es, width_um: float, pixel_um: int, seed: int):
     """A pencil-beam stream (each history's depositions around the detector's
     centre, as the synthetic configurations make them) turned into a flat

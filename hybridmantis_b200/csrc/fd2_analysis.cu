@@ -14,6 +14,7 @@
 // 501 x 501 image at all frequencies; the passes below take 46 and 45 us.  All
 // regions of all images of a noise spectrum go through them together (144
 // regions of 128 x 128 pixels: 89 and 121 us; region by region 288 launches).
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -431,30 +432,51 @@ struct Layout {
     }
 };
 
+// The identity of the current CUDA context, never used twice in a process; false
+// where the driver cannot say.
+bool context_id(unsigned long long *id)
+{
+    struct Entry {
+        PFN_cuCtxGetCurrent_v4000 current = nullptr;
+        PFN_cuCtxGetId_v12000 id = nullptr;
+        Entry()
+        {
+            void *a = nullptr, *b = nullptr;
+            cudaDriverEntryPointQueryResult q{};
+            if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &a, cudaEnableDefault, &q) != cudaSuccess ||
+                q != cudaDriverEntryPointSuccess ||
+                cudaGetDriverEntryPoint("cuCtxGetId", &b, cudaEnableDefault, &q) != cudaSuccess ||
+                q != cudaDriverEntryPointSuccess)
+                return;
+            current = reinterpret_cast<PFN_cuCtxGetCurrent_v4000>(a);
+            id = reinterpret_cast<PFN_cuCtxGetId_v12000>(b);
+        }
+    };
+    static const Entry entry;
+    CUcontext c = nullptr;
+    return entry.id && entry.current(&c) == CUDA_SUCCESS && c && entry.id(c, id) == CUDA_SUCCESS;
+}
+
 // A call's device memory and stream.  One of each is kept per device between
 // calls (allocating and freeing them took 1 to 5 ms of a 501 x 501 MTF, its
-// kernels 0.12 ms): up to kKept bytes, for one call at a time.  A call that
-// needs more, or that runs beside another on the device, has its own.  The
-// kept ones are freed with the library.
+// kernels 0.12 ms): up to kKept bytes, for one call at a time, until
+// fd2_analysis_release.  A call that needs more, or that runs beside another on
+// the device, has its own.  A device reset takes the kept ones away with their
+// context, so they belong to a context's identity and are forgotten, untouched,
+// when the device's context is another one.  Nothing is freed at the process's
+// end, when the runtime may be gone.
 class Workspace {
   public:
     static constexpr size_t kKept = (size_t)128 << 20;
 
+    // with `device` current
     cudaError_t open(int device, size_t bytes)
     {
-        Kept &k = kept(device);
-        if (device < kDevices && bytes <= kKept && k.lock.try_lock()) {
+        unsigned long long id = 0;
+        if (device < kDevices && bytes <= kKept && context_id(&id) && kept(device).lock.try_lock()) {
+            Kept &k = kept(device);
             held_ = &k;
-            if (k.stream) {
-                // a device reset took them away
-                const cudaError_t q = cudaStreamQuery(k.stream);
-                if (q != cudaSuccess && q != cudaErrorNotReady) {
-                    cudaGetLastError();
-                    k.stream = nullptr;
-                    k.base = nullptr;
-                    k.bytes = 0;
-                }
-            }
+            k.belong_to(id);
             cudaError_t e = k.stream ? cudaSuccess : cudaStreamCreateWithFlags(&k.stream, cudaStreamNonBlocking);
             if (e == cudaSuccess && k.bytes < bytes) {
                 if (k.base) cudaFree(k.base);
@@ -486,25 +508,49 @@ class Workspace {
         if (stream) cudaStreamDestroy(stream);
         if (base) cudaFree(base);
     }
+    // Gives the device's kept memory and stream back, after the call that uses
+    // them; with `device` current.
+    static cudaError_t release(int device)
+    {
+        unsigned long long id = 0;
+        if (device >= kDevices || !context_id(&id)) return cudaSuccess;  // nothing is kept
+        Kept &k = kept(device);
+        std::lock_guard<std::mutex> lock(k.lock);
+        k.belong_to(id);
+        cudaError_t e = k.base ? cudaFree(k.base) : cudaSuccess;
+        if (k.stream) {
+            const cudaError_t e2 = cudaStreamDestroy(k.stream);
+            if (e == cudaSuccess) e = e2;
+        }
+        k.forget();
+        return e;
+    }
     cudaStream_t stream = nullptr;
 
   private:
     static constexpr int kDevices = 16;
     struct Kept {
         std::mutex lock;
+        unsigned long long context = 0;  // whose they are
         char *base = nullptr;
         size_t bytes = 0;
         cudaStream_t stream = nullptr;
-        ~Kept()
+        void forget()
         {
-            if (base) cudaFree(base);  // fails quietly when the runtime is gone already
-            if (stream) cudaStreamDestroy(stream);
+            base = nullptr;
+            bytes = 0;
+            stream = nullptr;
+        }
+        void belong_to(unsigned long long id)
+        {
+            if (context != id) forget();
+            context = id;
         }
     };
     static Kept &kept(int device)
     {
         static Kept k[kDevices];
-        return k[device < kDevices ? device : 0];
+        return k[device];
     }
     char *base = nullptr;
     Kept *held_ = nullptr;
@@ -704,6 +750,12 @@ fd2_status fd2_nnps(int32_t device, const double *images, int32_t n_images, int3
     if (nnps_r) std::copy(r.begin(), r.begin() + K, nnps_r);
     if (mean_signal) *mean_signal = m;
     return FD2_OK;
+}
+
+fd2_status fd2_analysis_release(int32_t device)
+{
+    const cudaError_t e = cudaSetDevice(device);
+    return to_status(e == cudaSuccess ? Workspace::release(device) : e);
 }
 
 }  // extern "C"

@@ -12,8 +12,10 @@
  *
  * Images are [xdim][ydim] row-major with the x pixel index first (the PRF
  * layout of fd2_get_prf), pixel pitch `pixel_um` micrometres, host memory.
- * Frequencies are in cycles/mm.  All functions allocate device memory on
- * `device` for the call and free it before returning.
+ * Frequencies are in cycles/mm.  All functions use device memory on `device`:
+ * up to 128 MiB of it and a stream are kept for the next call until
+ * fd2_analysis_release or the process's end, more is freed before they return.
+ * They may be called from several threads.
  */
 #ifndef FD2_ANALYSIS_H
 #define FD2_ANALYSIS_H
@@ -51,6 +53,10 @@ FD2_API fd2_status fd2_nnps(int32_t device, const double *images, int32_t n_imag
                             double pixel_um, int32_t roi, int32_t x0, int32_t y0, int32_t rois_x, int32_t rois_y,
                             int32_t n_freq, double *freq_per_mm, double *nnps_r, double *nnps_2d,
                             double *mean_signal);
+
+/* Frees the device memory and the stream that the functions above keep on
+ * `device`, after a call that is using them.  The next call allocates again. */
+FD2_API fd2_status fd2_analysis_release(int32_t device);
 
 #ifdef __cplusplus
 }
