@@ -741,10 +741,11 @@ cudaError_t launch_tc(fd2_sg *s, cudaStream_t st, const TcArgs &t0, unsigned gri
 // The backward products fit one tcgen05 pass per tile when every
 // contraction (64 outputs, H hidden, 256-row batch slices) is <= 256 and
 // every width a multiple of 16.
+bool tc_backward(const fd2_sg *s) { return s->use_tc && s->hidden % 16 == 0 && s->hidden >= 32 && s->hidden <= kTcMaxN; }
+
 bool tc_backward_ok(const fd2_sg *s, int rows)
 {
-    const int H = s->hidden;
-    return s->use_tc && s->tA && H % 16 == 0 && H >= 32 && H <= kTcMaxN && rows > 0 && rows <= s->cap_rows;
+    return tc_backward(s) && s->tA && rows > 0 && rows <= s->cap_rows;
 }
 
 // Weight gradient on tcgen05: dW [M][K] = sum over 256-row slices z of
@@ -997,18 +998,22 @@ fd2_status ensure_rows(fd2_sg *s, int rows)
 {
     if (rows <= s->cap_rows) return FD2_OK;
     const size_t H = (size_t)s->hidden, R = (size_t)rows;
-    // tcgen05 backward: transposed operands over the rows padded to 256, and
-    // one FP32 partial plane per 256-row slice
-    const size_t RP = (size_t)rows_pad(rows);
-    // (for each layer: the four weight gradients run side by side)
-    const size_t ts = std::max<size_t>(H, kOutPad) * RP;
-    SG_CUDA(s, alloc(&s->tA, 4 * ts));
-    SG_CUDA(s, alloc(&s->tB, 4 * ts));
-    s->t_stride = (int64_t)ts;
     const size_t plane = std::max<size_t>(H * H, (size_t)kOutPad * H);
-    const size_t wsf = std::max<size_t>((size_t)kMaxSplits, RP / kTcSlice) * plane;
-    SG_CUDA(s, alloc(&s->ws, 4 * wsf));
-    s->ws_floats = (int64_t)wsf;
+    if (tc_backward(s)) {
+        // transposed operands over the rows padded to 256, and one FP32 partial
+        // plane per 256-row slice, for each layer: the four weight gradients run
+        // side by side (at most 256 hidden units; 8,192 rows: 34 + 34 MB)
+        const size_t RP = (size_t)rows_pad(rows), ts = std::max<size_t>(H, kOutPad) * RP;
+        SG_CUDA(s, alloc(&s->tA, 4 * ts));
+        SG_CUDA(s, alloc(&s->tB, 4 * ts));
+        s->t_stride = (int64_t)ts;
+        s->ws_floats = (int64_t)(std::max<size_t>((size_t)kMaxSplits, RP / kTcSlice) * plane);
+        SG_CUDA(s, alloc(&s->ws, 4 * (size_t)s->ws_floats));
+    } else {
+        // the layers one after another, at most kMaxSplits partial planes
+        s->ws_floats = (int64_t)(kMaxSplits * plane);
+        SG_CUDA(s, alloc(&s->ws, (size_t)s->ws_floats));
+    }
     SG_CUDA(s, alloc(&s->x0, R * kInPad));
     SG_CUDA(s, alloc(&s->h1, R * H));
     SG_CUDA(s, alloc(&s->h2, R * H));
