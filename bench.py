@@ -137,6 +137,15 @@ def cpu_model() -> str:
     return platform.processor() or "unknown"
 
 
+def reference_missing():
+    """Why the reference's C transport cannot be run here, or None."""
+    from oracle import pyoracle as po
+    if all(po.ref_available(opt) for opt in ("O0", "O2")):
+        return None
+    return ("the reference's C transport is not built: oracle/_ref is made by `make -C oracle` from the reference's "
+            "sources, which are not here")
+
+
 class CpuReference:
     """The reference's C transport (oracle/_ref) on the host cores; one
     process per core over contiguous event slices (each event keeps its own
@@ -585,7 +594,9 @@ def run_ours(a, rank, world, local_rank):
                     "ncu": TRANSPORT_NCU}
         cpu = None
         parity = None
-        if not a.no_cpu_baseline and world == 1:
+        if not a.no_cpu_baseline and world == 1 and reference_missing():
+            cpu = {"unavailable": reference_missing()}
+        elif not a.no_cpu_baseline and world == 1:
             ref = CpuReference(es, nphot)
             rate, ph, nev, dt, tallies = ref.timed_sample(a.cpu_seconds, keep=True)
             variants = cpu_variants(ref)
@@ -663,6 +674,8 @@ def run_reference(a, rank, world):
     driver does with GSL (numpy stands in for GSL)."""
     if rank != 0:
         return None
+    if reference_missing():
+        return {"impl": "reference", "unavailable": reference_missing()}
     from oracle import pyoracle as po
     es = po.synth_events_host(a.config, a.xrays, a.seed)
     rng = np.random.default_rng(a.seed)
