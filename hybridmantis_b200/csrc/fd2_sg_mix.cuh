@@ -23,9 +23,7 @@ namespace fd2 {
 namespace sg {
 
 struct Mix {
-    float w[kComponents], mu[kComponents], dmu[kComponents], sd[kComponents], S[kComponents];
-    float dS_mu[kComponents], dS_sd[kComponents];
-    bool clamped[kComponents];
+    float w[kComponents], mu[kComponents], sd[kComponents], S[kComponents];
 };
 
 __device__ __forceinline__ float norm_pdf(float a) { return 0.3989422804014327f * expf(-0.5f * a * a); }
@@ -69,7 +67,39 @@ __device__ __forceinline__ float ring_mass(const Edge &lo, const Edge &hi, float
     return m;
 }
 
-// Decode the network's mixture outputs (o[1..24]) and each ring's normaliser.
+// A ring from its radius and width outputs, with its normaliser S and the
+// derivatives dS/dmu = c0 and dS/dsd = p0.
+struct Ring {
+    float mu, sd, c0, p0, S;
+};
+
+__device__ __forceinline__ Ring decode_ring(float om, float ls)
+{
+    Ring r;
+    r.mu = kMuScale * (fmaxf(om, 0.0f) + log1pf(expf(-fabsf(om))));  // softplus
+    r.sd = kSdScale * expf(fminf(fmaxf(ls, kLogSdMin), kLogSdMax));
+    const float t0 = -r.mu / r.sd;
+    r.c0 = normcdff(-t0);
+    r.p0 = norm_pdf(t0);
+    r.S = fmaxf(r.mu * r.c0 + r.sd * r.p0, 1e-30f);
+    return r;
+}
+
+// The softmax weight of the lane's component: `a` is the weight output of
+// component lane % kComponents, the same in all lanes of a component.
+__device__ __forceinline__ float lane_weight(float a)
+{
+    float amax = a;
+#pragma unroll
+    for (int d = kComponents / 2; d > 0; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
+    const float e = expf(a - amax);
+    float s = 0.0f;
+#pragma unroll
+    for (int c = 0; c < kComponents; ++c) s += __shfl_sync(0xffffffffu, e, c);
+    return e / s;
+}
+
+// Decode the network's mixture outputs (o[1..24]) in every lane.
 __device__ __forceinline__ void decode_mix(const float *o, Mix &m)
 {
     float amax = o[1];
@@ -84,17 +114,10 @@ __device__ __forceinline__ void decode_mix(const float *o, Mix &m)
 #pragma unroll
     for (int k = 0; k < kComponents; ++k) {
         m.w[k] /= s;
-        const float om = o[1 + kComponents + k];
-        m.mu[k] = kMuScale * (fmaxf(om, 0.0f) + log1pf(expf(-fabsf(om))));  // softplus
-        m.dmu[k] = kMuScale / (1.0f + expf(-om));                           // d mu / d output
-        const float ls = o[1 + 2 * kComponents + k];
-        m.clamped[k] = ls < kLogSdMin || ls > kLogSdMax;
-        m.sd[k] = kSdScale * expf(fminf(fmaxf(ls, kLogSdMin), kLogSdMax));
-        const float t0 = -m.mu[k] / m.sd[k];
-        const float c0 = normcdff(-t0), p0 = norm_pdf(t0);
-        m.S[k] = fmaxf(m.mu[k] * c0 + m.sd[k] * p0, 1e-30f);
-        m.dS_mu[k] = c0;
-        m.dS_sd[k] = p0;
+        const Ring r = decode_ring(o[1 + kComponents + k], o[1 + 2 * kComponents + k]);
+        m.mu[k] = r.mu;
+        m.sd[k] = r.sd;
+        m.S[k] = r.S;
     }
 }
 

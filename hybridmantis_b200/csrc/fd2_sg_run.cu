@@ -347,35 +347,24 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SampleArgs
         // the event's mixture in the warp's shared-memory table (every lane
         // draws from the same one; an indexed table in registers would go to
         // local memory): cumulative weight, mu, sd and normaliser per ring
-        // (decode_mix, a component per lane: all lanes decoding all of them was
-        // a third of the kernel's thread instructions)
+        // (a component per lane: all lanes decoding all of them was a third of the
+        // kernel's thread instructions)
         {
             const int c = lane % kComponents;
-            const float w0 = o[1 + c], om = o[1 + kComponents + c], ls = o[1 + 2 * kComponents + c];
-            float top = w0;
-#pragma unroll
-            for (int d = kComponents / 2; d > 0; d >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, d));
-            const float ew = expf(w0 - top);
-            float s = 0.0f;
-#pragma unroll
-            for (int k = 0; k < kComponents; ++k) s += __shfl_sync(0xffffffffu, ew, k);
-            const float w = ew / s;
+            const float w = lane_weight(o[1 + c]);
             float acc = 0.0f;  // the weights up to the lane's, added in order
 #pragma unroll
             for (int k = 0; k < kComponents; ++k) {
                 const float v = __shfl_sync(0xffffffffu, w, k);
                 acc = k <= c ? acc + v : acc;
             }
-            const float mu = kMuScale * (fmaxf(om, 0.0f) + log1pf(expf(-fabsf(om))));
-            const float sd = kSdScale * expf(fminf(fmaxf(ls, kLogSdMin), kLogSdMax));
-            const float t0 = -mu / sd;
-            const float S = fmaxf(mu * normcdff(-t0) + sd * norm_pdf(t0), 1e-30f);
+            const Ring ring = decode_ring(o[1 + kComponents + c], o[1 + 2 * kComponents + c]);
             __syncwarp();  // the previous event's photons are placed
             if (lane < kComponents) {
                 mix[0][c] = c == kComponents - 1 ? 2.0f : acc;
-                mix[1][c] = mu;
-                mix[2][c] = sd;
-                mix[3][c] = S;
+                mix[1][c] = ring.mu;
+                mix[2][c] = ring.sd;
+                mix[3][c] = ring.S;
             }
             __syncwarp();
         }

@@ -102,23 +102,13 @@ __device__ __forceinline__ PointLoss point_loss(const float *o, float t, const f
     p.det = p.total = ld;
     p.rad = p.ga = p.gom = p.gls = 0.0f;
     if (!has_rad) return p;
-    // component k, the same in lanes k, 8 + k, ... (decode_mix)
-    const float a = o[1 + k], om = o[1 + kComponents + k], ls = o[1 + 2 * kComponents + k];
-    float amax = a;
-#pragma unroll
-    for (int d = kComponents / 2; d > 0; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
-    const float ew = expf(a - amax);
-    float s = 0.0f;
-#pragma unroll
-    for (int c = 0; c < kComponents; ++c) s += __shfl_sync(0xffffffffu, ew, c);
-    const float w = ew / s;
-    const float mu = kMuScale * (fmaxf(om, 0.0f) + log1pf(expf(-fabsf(om))));  // softplus
-    const float dmu = kMuScale / (1.0f + expf(-om));                           // d mu / d output
+    // component k, the same in lanes k, 8 + k, ...
+    const float om = o[1 + kComponents + k], ls = o[1 + 2 * kComponents + k];
+    const float w = lane_weight(o[1 + k]);
+    const Ring ring = decode_ring(om, ls);
+    const float mu = ring.mu, sd = ring.sd, S = ring.S;
+    const float dmu = kMuScale / (1.0f + expf(-om));  // d mu / d output
     const bool clamped = ls < kLogSdMin || ls > kLogSdMax;
-    const float sd = kSdScale * expf(fminf(fmaxf(ls, kLogSdMin), kLogSdMax));
-    const float t0 = -mu / sd;
-    const float c0 = normcdff(-t0), p0 = norm_pdf(t0);
-    const float S = fmaxf(mu * c0 + sd * p0, 1e-30f);
     __syncwarp();  // every lane is done with the row before
     if (lane < kComponents) {
         // of an edge's two tails only the one away from the ring is kept, and
@@ -220,8 +210,8 @@ __device__ __forceinline__ PointLoss point_loss(const float *o, float t, const f
     for (int c = 0; c < kComponents; ++c)
         wg += __shfl_sync(0xffffffffu, w, c) * __shfl_sync(0xffffffffu, gw, c);
     const float f = w / S;
-    const float gmu = -f * (Amu - A1 * c0 / S);
-    const float gsd = -f * (Asd - A1 * p0 / S);
+    const float gmu = -f * (Amu - A1 * ring.c0 / S);
+    const float gsd = -f * (Asd - A1 * ring.p0 / S);
     p.ga = lambda * w * (gw - wg);
     p.gom = lambda * dmu * gmu;
     p.gls = clamped ? 0.0f : lambda * sd * gsd;
