@@ -953,7 +953,7 @@ struct Walker {
             const float cx = ((float)i + 0.5f) * p, cy = ((float)j + 0.5f) * p;
             const float fx = px - cx, fy = py - cy;
             const float qb = 2.0f * sum2(fx, dx, fy, dy);
-            const float qc = __fmaf_rn(-g.R, g.R, sum2(fx, fx, fy, fy));
+            const float qc = __fadd_rn(sum2(fx, fx, fy, fy), -__fmul_rn(g.R, g.R));
             if (qa > 0.0f && qb < 0.0f) {
                 const float disc = sum2(qb, qb, -(4.0f * qa), qc);
                 if (disc >= 0.0f) {
@@ -965,7 +965,7 @@ struct Walker {
                         dist += t1;
                         wx = cx;
                         wy = cy;
-                            return kToWall;
+                        return kToWall;
                     }
                 }
             }
