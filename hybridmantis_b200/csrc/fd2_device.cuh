@@ -696,6 +696,10 @@ struct Walker {
                     dy = sum2(-ct, ny, -ratio, ty);
                     dz = sum2(-ct, nz, -ratio, tz);
                     renorm(dx, dy, dz);
+                    // a direction that is no number (columns of a nanometre) has
+                    // the sign that flight takes for downwards, as a comparison
+                    // with 0 would (two more instructions in every step)
+                    if (!(dz == dz)) dz = __int_as_float(-1);
                     if (outside) break;  // entered the next column: done
                     stage = kLeave;
                 }
@@ -1029,7 +1033,7 @@ struct Walker {
             if (sensor) {
                 // sensor plane inside a column (detection)
                 if (!(g.sensor_refl > 0.0f && u() < g.sensor_refl)) return kDetect;
-                dz = -dz;  // specular reflection on the flat sensor
+                dz = dz == dz ? -dz : dz;  // specular reflection on the flat sensor
                 renorm(dx, dy, dz);
                 tag |= kReflected;
                 return kFlies;
