@@ -133,7 +133,10 @@ fd2_status alloc_tallies(fd2_ctx *c)
     }
     c->prf_total = off;
     FD2_CUDA(c, dalloc(&c->d_geoms, G));
-    FD2_CUDA(c, cudaMemcpy(c->d_geoms, c->dgeoms.data(), sizeof(DevGeom) * G, cudaMemcpyHostToDevice));
+    // uploads go through the context's stream: it does not wait for the default
+    // stream, on which a copy from pageable memory may still be under way when
+    // cudaMemcpy returns
+    FD2_CUDA(c, cudaMemcpyAsync(c->d_geoms, c->dgeoms.data(), sizeof(DevGeom) * G, cudaMemcpyHostToDevice, c->stream));
     FD2_CUDA(c, dalloc(&c->d_prf, (size_t)c->prf_total));
     FD2_CUDA(c, dalloc(&c->d_counters, G * fd2::kCounterStride));
     FD2_CUDA(c, dalloc(&c->d_distance, G));
@@ -436,7 +439,7 @@ fd2_status load_libm_table(fd2_ctx *c)
     std::fclose(f);
     if (!ok) return fail(c, FD2_ERR_PARSE, "replay table " + path + " is corrupt");
     FD2_CUDA(c, dalloc(&c->d_libm, tab.size()));
-    FD2_CUDA(c, cudaMemcpy(c->d_libm, tab.data(), 4 * tab.size(), cudaMemcpyHostToDevice));
+    FD2_CUDA(c, cudaMemcpyAsync(c->d_libm, tab.data(), 4 * tab.size(), cudaMemcpyHostToDevice, c->stream));
     c->n_acos = na;
     c->n_asin = ns;
     return FD2_OK;
@@ -624,7 +627,7 @@ fd2_status fd2_create(const fd2_params *p, const fd2_options *opt, fd2_ctx **out
     if (cudaHostAlloc((void **)&c->h_abort, sizeof(int), cudaHostAllocMapped) != cudaSuccess) return bail(FD2_ERR_CUDA);
     *c->h_abort = 0;
     if (cudaHostGetDevicePointer((void **)&c->d_abort, c->h_abort, 0) != cudaSuccess) return bail(FD2_ERR_CUDA);
-    if (dalloc(&c->d_flags, 2) != cudaSuccess || cudaMemset(c->d_flags, 0, 2 * sizeof(int)) != cudaSuccess)
+    if (dalloc(&c->d_flags, 2) != cudaSuccess || cudaMemsetAsync(c->d_flags, 0, 2 * sizeof(int), c->stream) != cudaSuccess)
         return bail(FD2_ERR_OUT_OF_MEMORY);
     c->n_prim = p->num_hist;
     if (dalloc(&c->d_per_primary, (size_t)c->n_prim) != cudaSuccess || dalloc(&c->d_prim_geom, (size_t)c->n_prim) != cudaSuccess)

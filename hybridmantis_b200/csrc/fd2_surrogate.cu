@@ -582,7 +582,7 @@ fd2_status sg_tc_check(fd2_sg *s)
     unsigned f = 0;
     SG_CUDA(s, cudaMemcpy(&f, s->d_tc_fault, sizeof f, cudaMemcpyDeviceToHost));
     if (!f) return FD2_OK;
-    SG_CUDA(s, cudaMemset(s->d_tc_fault, 0, sizeof f));
+    SG_CUDA(s, cudaMemsetAsync(s->d_tc_fault, 0, sizeof f, s->stream));
     return sg_fail(s, FD2_ERR_DEVICE_ABORT, "a tensor-core GEMM tile gave up waiting for its MMAs");
 }
 
@@ -953,19 +953,6 @@ int64_t public_count(const fd2_sg *s)
     return H * kFeatures + H + 2 * (H * H + H) + kOutputs * H + kOutputs;
 }
 
-fd2_status upload_params(fd2_sg *s, const std::vector<float> &master)
-{
-    SG_CUDA(s, cudaSetDevice(s->device));
-    SG_CUDA(s, cudaMemcpy(s->p, master.data(), sizeof(float) * master.size(), cudaMemcpyHostToDevice));
-    to_bf16_kernel<<<grid_for(s->n_params, 256), 256>>>(s->p, s->pb, s->n_params);
-    SG_CUDA(s, cudaGetLastError());
-    SG_CUDA(s, cudaMemset(s->m, 0, sizeof(float) * s->n_params));
-    SG_CUDA(s, cudaMemset(s->v, 0, sizeof(float) * s->n_params));
-    SG_CUDA(s, cudaMemset(s->d_step, 0, sizeof(unsigned long long)));
-    SG_CUDA(s, cudaDeviceSynchronize());
-    return FD2_OK;
-}
-
 void set_norm(fd2_sg *s)
 {
     for (int i = 0; i < kFeatures; ++i) {
@@ -975,12 +962,33 @@ void set_norm(fd2_sg *s)
     }
 }
 
+// Uploads go through the surrogate's stream.  It does not wait for the default
+// stream, on which a copy from pageable memory may still be under way when
+// cudaMemcpy returns: a kernel of the stream could read what was there before.
+cudaError_t upload(fd2_sg *s, void *dst, const void *src, size_t bytes)
+{
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s->stream);
+}
+
 template <class T>
 cudaError_t alloc(T **p, size_t n)
 {
     if (*p) cudaFree(*p);
     *p = nullptr;
     return cudaMalloc((void **)p, sizeof(T) * std::max<size_t>(n, 1));
+}
+
+fd2_status upload_params(fd2_sg *s, const std::vector<float> &master)
+{
+    SG_CUDA(s, cudaSetDevice(s->device));
+    SG_CUDA(s, upload(s, s->p, master.data(), sizeof(float) * master.size()));
+    to_bf16_kernel<<<grid_for(s->n_params, 256), 256, 0, s->stream>>>(s->p, s->pb, s->n_params);
+    SG_CUDA(s, cudaGetLastError());
+    SG_CUDA(s, cudaMemsetAsync(s->m, 0, sizeof(float) * s->n_params, s->stream));
+    SG_CUDA(s, cudaMemsetAsync(s->v, 0, sizeof(float) * s->n_params, s->stream));
+    SG_CUDA(s, cudaMemsetAsync(s->d_step, 0, sizeof(unsigned long long), s->stream));
+    SG_CUDA(s, cudaStreamSynchronize(s->stream));
+    return FD2_OK;
 }
 
 // Activation buffers for `rows` rows.
@@ -1099,8 +1107,8 @@ fd2_status fd2_sg_create(const fd2_sg_config *cfg, fd2_sg **out)
         alloc(&s->d_live, P) || alloc(&s->d_step, 1) || alloc(&s->d_acc, 4) || alloc(&s->d_lr, 1) ||
         alloc(&s->pbT, 2 * (size_t)s->hidden * s->hidden + (size_t)s->hidden * kOutPad))
         return bail(FD2_ERR_OUT_OF_MEMORY);
-    if (cudaMemcpy(s->d_lr, &s->lr, sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) return bail(FD2_ERR_CUDA);
-    if (alloc(&s->d_tc_fault, 1) || cudaMemset(s->d_tc_fault, 0, sizeof(unsigned)) != cudaSuccess)
+    if (upload(s, s->d_lr, &s->lr, sizeof(float)) != cudaSuccess) return bail(FD2_ERR_CUDA);
+    if (alloc(&s->d_tc_fault, 1) || cudaMemsetAsync(s->d_tc_fault, 0, sizeof(unsigned), s->stream) != cudaSuccess)
         return bail(FD2_ERR_OUT_OF_MEMORY);
     {
         int sms = 0;
@@ -1135,8 +1143,8 @@ fd2_status fd2_sg_create(const fd2_sg_config *cfg, fd2_sg **out)
             return bail(FD2_ERR_CUDA);
     }
     const std::vector<uint8_t> live = live_mask(s);
-    if (cudaMemcpy(s->d_live, live.data(), P, cudaMemcpyHostToDevice) != cudaSuccess) return bail(FD2_ERR_CUDA);
-    if (cudaMemset(s->g, 0, sizeof(float) * P) != cudaSuccess) return bail(FD2_ERR_CUDA);
+    if (upload(s, s->d_live, live.data(), P) != cudaSuccess) return bail(FD2_ERR_CUDA);
+    if (cudaMemsetAsync(s->g, 0, sizeof(float) * P, s->stream) != cudaSuccess) return bail(FD2_ERR_CUDA);
     // He-normal weights (Box-Muller on a splitmix64 stream), small last
     // layer, zero biases; mixture biases spread the components in radius
     // and width.
@@ -1204,7 +1212,8 @@ fd2_status fd2_sg_set_lr(fd2_sg *s, float lr)
     SG_CUDA(s, cudaSetDevice(s->device));
     SG_CUDA(s, cudaStreamSynchronize(s->stream));
     s->lr = lr;
-    SG_CUDA(s, cudaMemcpy(s->d_lr, &s->lr, sizeof(float), cudaMemcpyHostToDevice));
+    SG_CUDA(s, upload(s, s->d_lr, &s->lr, sizeof(float)));
+    SG_CUDA(s, cudaStreamSynchronize(s->stream));
     return FD2_OK;
 }
 
@@ -1302,10 +1311,11 @@ fd2_status fd2_sg_set_data(fd2_sg *s, const float *features, const int32_t *phot
     SG_CUDA(s, alloc(&s->d_photons, N));
     SG_CUDA(s, alloc(&s->d_detected, N));
     SG_CUDA(s, alloc(&s->d_radial, N * nb));
-    SG_CUDA(s, cudaMemcpy(s->d_feat, features, sizeof(float) * N * kFeatures, cudaMemcpyHostToDevice));
-    SG_CUDA(s, cudaMemcpy(s->d_photons, photons, sizeof(int32_t) * N, cudaMemcpyHostToDevice));
-    SG_CUDA(s, cudaMemcpy(s->d_detected, detected, sizeof(int32_t) * N, cudaMemcpyHostToDevice));
-    SG_CUDA(s, cudaMemcpy(s->d_radial, radial, sizeof(uint32_t) * N * nb, cudaMemcpyHostToDevice));
+    SG_CUDA(s, upload(s, s->d_feat, features, sizeof(float) * N * kFeatures));
+    SG_CUDA(s, upload(s, s->d_photons, photons, sizeof(int32_t) * N));
+    SG_CUDA(s, upload(s, s->d_detected, detected, sizeof(int32_t) * N));
+    SG_CUDA(s, upload(s, s->d_radial, radial, sizeof(uint32_t) * N * nb));
+    SG_CUDA(s, cudaStreamSynchronize(s->stream));  // the arrays are the caller's
     s->n_points = n;
     s->n_train = n_train;
     s->n_val = n_val;
@@ -1397,10 +1407,10 @@ fd2_status fd2_sg_loss_grad(fd2_sg *s, const float *features, const int32_t *pho
     if (e == cudaSuccess) e = cudaMalloc(&dp, sizeof(int32_t) * b);
     if (e == cudaSuccess) e = cudaMalloc(&dd, sizeof(int32_t) * b);
     if (e == cudaSuccess) e = cudaMalloc(&dr, sizeof(uint32_t) * b * nb);
-    if (e == cudaSuccess) e = cudaMemcpy(df, features, sizeof(float) * b * kFeatures, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(dp, photons, sizeof(int32_t) * b, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(dd, detected, sizeof(int32_t) * b, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(dr, radial, sizeof(uint32_t) * b * nb, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload(s, df, features, sizeof(float) * b * kFeatures);
+    if (e == cudaSuccess) e = upload(s, dp, photons, sizeof(int32_t) * b);
+    if (e == cudaSuccess) e = upload(s, dd, detected, sizeof(int32_t) * b);
+    if (e == cudaSuccess) e = upload(s, dr, radial, sizeof(uint32_t) * b * nb);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->d_acc, 0, sizeof(double) * 4, s->stream);
     if (e == cudaSuccess) {
         gather_kernel<<<warps_for(b), 256, 0, s->stream>>>(df, dp, dd, dr, s->bins, b, 0, b, true, s->seed,

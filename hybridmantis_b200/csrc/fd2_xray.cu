@@ -799,14 +799,16 @@ fd2_status xfail(fd2_xray *x, fd2_status s, const std::string &m)
         if (e_ != cudaSuccess) return xfail(x, FD2_ERR_CUDA, cudaGetErrorString(e_)); \
     } while (0)
 
+// On the front end's stream, which does not wait for the default stream: a
+// copy from pageable memory may still be under way when cudaMemcpy returns.
 template <class T>
-cudaError_t upload(T **d, const std::vector<T> &h)
+cudaError_t upload(cudaStream_t s, T **d, const std::vector<T> &h)
 {
     if (*d) cudaFree(*d);
     *d = nullptr;
     cudaError_t e = cudaMalloc((void **)d, sizeof(T) * std::max<size_t>(h.size(), 1));
     if (e != cudaSuccess) return e;
-    return h.empty() ? cudaSuccess : cudaMemcpy(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice);
+    return h.empty() ? cudaSuccess : cudaMemcpyAsync(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, s);
 }
 
 double lnz(double v) { return std::log(std::max(v, 1e-300)); }
@@ -854,17 +856,17 @@ fd2_status upload_tables(fd2_xray *x)
         }
         toff[k * (kDesignators + 1) + kDesignators] = (int)ts.size();
     }
-    XCUDA(x, upload(&x->d_e, m.e));
-    XCUDA(x, upload(&x->d_lnv, lnv));
-    XCUDA(x, upload(&x->d_ee, m.ee));
-    XCUDA(x, upload(&x->d_lnee, lnee));
-    XCUDA(x, upload(&x->d_lnr, lnr));
-    XCUDA(x, upload(&x->d_lnl1, lnl1));
-    XCUDA(x, upload(&x->d_bind, bind));
-    XCUDA(x, upload(&x->d_toff, toff));
-    XCUDA(x, upload(&x->d_ts, ts));
-    XCUDA(x, upload(&x->d_tcum, tcum));
-    XCUDA(x, upload(&x->d_te, te));
+    XCUDA(x, upload(x->stream, &x->d_e, m.e));
+    XCUDA(x, upload(x->stream, &x->d_lnv, lnv));
+    XCUDA(x, upload(x->stream, &x->d_ee, m.ee));
+    XCUDA(x, upload(x->stream, &x->d_lnee, lnee));
+    XCUDA(x, upload(x->stream, &x->d_lnr, lnr));
+    XCUDA(x, upload(x->stream, &x->d_lnl1, lnl1));
+    XCUDA(x, upload(x->stream, &x->d_bind, bind));
+    XCUDA(x, upload(x->stream, &x->d_toff, toff));
+    XCUDA(x, upload(x->stream, &x->d_ts, ts));
+    XCUDA(x, upload(x->stream, &x->d_tcum, tcum));
+    XCUDA(x, upload(x->stream, &x->d_te, te));
     XDev &g = x->dev;
     g.n_nodes = (int)n;
     g.n_el = nel;
@@ -998,7 +1000,7 @@ fd2_status make_source(fd2_xray *x, const fd2_xray_source *s, XSource &o)
         XCUDA(x, cudaMalloc(&x->d_spec, sizeof(double) * buf.size()));
         x->spec_cap = (int)buf.size();
     }
-    XCUDA(x, cudaMemcpy(x->d_spec, buf.data(), sizeof(double) * buf.size(), cudaMemcpyHostToDevice));
+    XCUDA(x, cudaMemcpyAsync(x->d_spec, buf.data(), sizeof(double) * buf.size(), cudaMemcpyHostToDevice, x->stream));
     o.espc = x->d_spec;
     o.pcum = x->d_spec + n;
     o.despc = x->d_spec + 2 * n;
@@ -1151,7 +1153,9 @@ FD2_API fd2_status fd2_xray_create(const fd2_xray_material *m, const fd2_xray_op
     // [0] a batch's EDE total, [1] the history kernel's counter
     if (st == FD2_OK && cudaMalloc(&x->d_total, 2 * sizeof(unsigned long long)) != cudaSuccess)
         st = FD2_ERR_OUT_OF_MEMORY;
-    if (st == FD2_OK && cudaMemset(x->d_tot, 0, sizeof(Totals)) != cudaSuccess) st = FD2_ERR_CUDA;
+    if (st == FD2_OK && (cudaMemsetAsync(x->d_tot, 0, sizeof(Totals), x->stream) != cudaSuccess ||
+                         cudaStreamSynchronize(x->stream) != cudaSuccess))
+        st = FD2_ERR_CUDA;
     if (st != FD2_OK) {
         fd2_xray_destroy(x);
         return st;
@@ -1309,7 +1313,8 @@ FD2_API fd2_status fd2_xray_clear_stats(fd2_xray *x)
 {
     if (!x) return FD2_ERR_INVALID_ARGUMENT;
     XCUDA(x, cudaSetDevice(x->device));
-    XCUDA(x, cudaMemset(x->d_tot, 0, sizeof(Totals)));
+    XCUDA(x, cudaMemsetAsync(x->d_tot, 0, sizeof(Totals), x->stream));
+    XCUDA(x, cudaStreamSynchronize(x->stream));
     x->stats = fd2_xray_stats{};
     return FD2_OK;
 }
