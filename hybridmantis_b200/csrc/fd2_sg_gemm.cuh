@@ -10,9 +10,10 @@
 // same kernel without transposing anything in memory.
 //
 // Tiles: 64 x 64 x 32 per CTA, four warps of 32 x 32, mma.sync m16n8k16.
-// M and N may be ragged (zero-filled loads, guarded stores); K must be a
-// multiple of 32 and every row stride a multiple of 8 elements (16-byte
-// loads).  An optional device pointer caps M at run time (rows beyond it
+// M and N may be ragged (zero-filled loads, guarded stores), and K where both
+// operands have the output index contiguous (a batch of any number of rows);
+// otherwise K must be a multiple of 32.  Every row stride is a multiple of 8
+// elements (16-byte loads).  An optional device pointer caps M at run time (rows beyond it
 // are skipped), for batches whose size is known only on the device.
 #pragma once
 
@@ -125,7 +126,9 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_kernel(const GemmArgs g)
                 const int r = v >> 3, c = (v & 7) * 8;
                 const int m = m0 + c;
                 uint4 val = zero;
-                if (m + 8 <= M) {
+                if (k0 + r >= k_end) {
+                    // past the contraction: whatever lies there counts as zero
+                } else if (m + 8 <= M) {
                     val = *reinterpret_cast<const uint4 *>(g.A + (long long)(k0 + r) * g.lda + m);
                 } else if (m < M) {
                     __align__(16) __nv_bfloat16 tmp[8];
@@ -149,7 +152,8 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_kernel(const GemmArgs g)
                 const int r = v >> 3, c = (v & 7) * 8;
                 const int n = n0 + c;
                 uint4 val = zero;
-                if (n + 8 <= N) {
+                if (k0 + r >= k_end) {
+                } else if (n + 8 <= N) {
                     val = *reinterpret_cast<const uint4 *>(g.B + (long long)(k0 + r) * g.ldb + n);
                 } else if (n < N) {
                     __align__(16) __nv_bfloat16 tmp[8];
