@@ -11,7 +11,8 @@
 // twiddles of a warp are the same for its lanes (broadcast reads), and the
 // next chunk of a tile is loaded while one is summed.  One thread per output
 // with a table read of its own per multiply-add took 164 us and 323 us for a
-// 501 x 501 image at all frequencies; the passes below take 46 and 45 us.  All
+// 501 x 501 image at all frequencies; the passes below take 46 and 45 us.  The
+// axes alone (MTF without mtf_r) come from the two line spread functions.  All
 // regions of all images of a noise spectrum go through them together (144
 // regions of 128 x 128 pixels: 89 and 121 us; region by region 288 launches).
 #include <cudaTypedefs.h>

@@ -376,14 +376,15 @@ void fit_window(fd2_ctx *c)
 
 // Launch shape unless the options give one, measured on a B200: one geometry
 // 256 threads x 4 CTAs per SM (32 warps at 64 registers; 20,000 config-1
-// x-rays 51.6 ms against 54.1 for 224 x 4 and 55.6 for 256 x 3, before the
-// steps below a full exchange were looped), chunks of 16 photons; the square
-// column lattice the same (10,001 config-1 x-rays 61.7 ms against 65.1 for
-// 256 x 3, 69.4 for 320 x 2); several geometries 256 x 3 (configuration 2, 500
-// x-rays: 59.4 ms against 61.7 for 256 x 4); the hexagonal lattice 256 x 3
-// (83.0 ms against 90.4 for 320 x 2), its only kernel above 256 x 2; label
-// mode with one geometry (the surrogate's audit) as one geometry, with
-// several 256 x 3.
+// x-rays 38.7 ms against 39.4 for 224 x 4, 39.9 for 256 x 3, 42.6 for 320 x 2);
+// the square column lattice the same (10,001 config-1 x-rays 60.9 ms against
+// 64.5 for 256 x 3, 68.6 for 320 x 2); several geometries 256 x 3
+// (configuration 2, 500 x-rays: 57.9 ms against 59.5 for 256 x 4, 62.5 for 320 x
+// 2); the hexagonal lattice 256 x 3 (83.0 ms against 87.6 for 320 x 2), its only
+// kernel above 256 x 2; label mode: transport_ctas.  Chunks of 16 photons, 32
+// where warps are fewer: small runs spread better over the warps (300 / 20,000 /
+// 100,000 config-1 x-rays: 1.10 / 38.74 / 191.7 ms with 16, 1.12 / 38.65 / 191.1
+// with 64, 1.19 / 38.72 / 191.1 with 128).
 static void default_launch(const fd2_ctx *c, int n_geom, fd2::TransportConfig *cfg)
 {
     int block = 256, ctas = 4, chunk = 16;
@@ -640,13 +641,13 @@ fd2_status fd2_create(const fd2_params *p, const fd2_options *opt, fd2_ctx **out
     if ((st = alloc_tallies(c)) != FD2_OK) return bail(st);
     fd2::TransportConfig cfg;
     default_launch(c, 1, &cfg);
-    // idle lanes that trigger a refill (20,000 config-1 x-rays: 4 / 6 / 8 / 10
-    // lanes 47.8 / 46.5 / 46.0 / 46.2 ms; the square lattice, 6 / 8 / 10 / 12:
-    // 62.0 / 61.6 / 62.2 / 63.3)
+    // idle lanes that trigger a refill (20,000 config-1 x-rays: 4 / 6 / 8 / 10 / 12
+    // lanes 40.9 / 39.3 / 38.8 / 38.6 / 39.3 ms; 10,001 in the square lattice, 6 /
+    // 8 / 10 / 12: 61.2 / 60.9 / 61.5 / 62.5)
     cfg.refill = c->opt.refill > 0 ? c->opt.refill : 8;
     // photons waiting for the Fresnel part (with a lattice: in the gap) before
-    // the warp runs it for them: a full warp's (16 / 24 / 32 photons: 56.7 /
-    // 53.3 / 51.9 ms, hexagonal lattice 114 ms at 24, 104 at 32)
+    // the warp runs it for them: a full warp's (8 / 16 / 24 / 32 photons: 48.4 /
+    // 42.6 / 39.6 / 38.7 ms; hexagonal lattice, 16 / 24 / 32: 104.8 / 89.3 / 82.9)
     cfg.fresnel = c->opt.fresnel_batch > 0 ? c->opt.fresnel_batch : 32;
     if ((st = set_config(c, cfg)) != FD2_OK) return bail(st);
     *out = c;

@@ -65,8 +65,8 @@ __device__ __forceinline__ uint4 philox4x32_10_rk(uint4 c, const uint32_t *rk)
 __device__ __forceinline__ float u01(uint32_t r)
 {
     // 0x3F800000 + (r >> 9) as one multiply-add, which runs beside the integer
-    // pipe that the generator fills (a funnel shift of 0x7F and r: 64
-    // geometries x 500 x-rays 56.1 ms, this 55.4; one geometry the same)
+    // pipe that the generator fills (a funnel shift of 0x7F and r: 1 % slower
+    // with several geometries, the same with one)
     uint32_t b;
     asm("mad.hi.u32 %0, %1, 0x800000, 0x3f800000;" : "=r"(b) : "r"(r));
     return __uint_as_float(b) - 0.99999994039535522461f;
@@ -98,7 +98,11 @@ struct RngKey {
 // the compiler fuses depends on the code around it: the transport's kernel
 // variants must round a walk alike (a column billiard turns a last-bit
 // difference into another history), so that label runs, geometry scans and
-// single-geometry runs of the same photons keep giving the same tallies.
+// single-geometry runs of the same photons keep giving the same tallies.  Not
+// written out is the neighbour test of the hexagonal lattice (fx, fy, disc in
+// grid_flight), whose fusing no explicit form tried reproduces: its kernels are
+// those that the compiler rounds alike, and a compiler that fuses it otherwise
+// changes their histories.
 __device__ __forceinline__ float sum2(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }
 __device__ __forceinline__ float sum3(float a, float b, float c, float d, float e, float f)
 {
@@ -288,10 +292,8 @@ struct Walker {
     // (dist_to_surface), then bulk absorption (isotropic).  Selects instead of
     // early exits and of branches that most lanes take (a branch is three
     // instructions for the warp): the pull-back's first step and the absorption
-    // run for all lanes.  20,000 config-1 x-rays: the pull-back one loop with
-    // two counters 42.9 ms, its first step before the loop 42.3, by selects
-    // 41.9; absorption by selects 41.4.  `ended`: the photon's walk is over,
-    // with the fate that is returned.
+    // run for all lanes (20,000 config-1 x-rays 41.4 ms, by branches 42.9).
+    // `ended`: the photon's walk is over, with the fate that is returned.
     template <class G>
     __device__ __forceinline__ int flight(const G &g, bool &ended)
     {
@@ -383,8 +385,7 @@ struct Walker {
     // the walk's instruction fetch grows with the kernel's code size.
     // The parts stand in the order photons pass them, so that one round of the
     // loop takes most photons through and the lanes meet at the next normal (a
-    // part per round: 20,000 config-1 x-rays with a reflecting sensor 44.9 ms,
-    // this 44.6).
+    // part per round 1 % slower).
     template <class G>
     __device__ __forceinline__ int leave_column(const G &g)
     {
@@ -574,8 +575,9 @@ struct Walker {
     }
 
     // The photon's tag: its geometry in bits 0-7, bit 8 just reflected by the
-    // sensor, above it the retry counts of a wall interaction while it waits: tries at an incidence angle and at a next normal (at
-    // most 100 each), perturbations (3) and smooth attempts (25).
+    // sensor, above it the retry counts of a wall interaction while it waits:
+    // tries at an incidence angle and at a next normal (at most 100 each),
+    // perturbations (3) and smooth attempts (25).
     static constexpr uint32_t kGeomBits = 0xffu, kReflected = 1u << 8;
     static constexpr int kTheta = 9, kPerturb = 16, kSmooth = 18, kNormalTry = 23;
     static constexpr uint32_t kCounts = (0x7fu << kTheta) | (3u << kPerturb) | (0x1fu << kSmooth) | (0x7fu << kNormalTry);
@@ -584,7 +586,8 @@ struct Walker {
     // / refraction on the rough wall (boundary_analysis, second part).  A
     // photon that refracts out of its column waits again, for its hop
     // (kHops); with `hop` it continues there, until it is back inside a
-    // column or meets the next column's wall from outside and hops again.  One
+    // column or meets the next column's wall from outside and hops again.  Hops
+    // count as boundary interactions, which bounds them.  One
     // in five wall interactions leaves the column: run to their end beside the
     // others, the hops took half of the pass at 2 to 3 lanes.  `counts` keeps
     // the retry counts between the two.
@@ -592,7 +595,7 @@ struct Walker {
     __device__ __forceinline__ int surface_wait(const G &g, bool hop, uint32_t &counts)
     {
         if (!hop && at_top(g)) return top_reflector(g);
-        if (hop && ++rebound > kMaxBoundaryCalls) return kCapped;  // bounds the passes of one interaction
+        if (hop && ++rebound > kMaxBoundaryCalls) return kCapped;
         bool outside = hop;
         int tries_theta = (counts >> kTheta) & 0x7f, tries_normal = (counts >> kNormalTry) & 0x7f;
         int reperturbs = (counts >> kPerturb) & 3, smooth = (counts >> kSmooth) & 0x1f;
@@ -656,7 +659,7 @@ struct Walker {
                 }
                 const float si = sqrtf(fmaxf(0.0f, 1.0f - c1 * c1));
                 // selects: total reflection and the rest, inside and out, in
-                // one piece of code (20,000 config-1 x-rays 40.75 -> 40.55 ms)
+                // one piece of code (by branches 0.5 % slower)
                 const bool stale = outside && g.stale_out;
                 const float eta = outside ? g.eta_out : g.eta_in;
                 const float nst = eta * si, nct = sqrtf(fmaxf(0.0f, 1.0f - nst * nst)), npr = fresnel(c1, nct, eta);
@@ -1024,7 +1027,7 @@ struct Walker {
         bool ended;
         const int f = flight(g, ended);
         // one branch for all that few lanes do, at a plane, ended or trapped (four
-        // in turn 41.2 ms for 20,000 config-1 x-rays, this 40.8)
+        // in turn 1 % slower)
         const bool trapped = fabsf(dz) < kEps;
         if (ended || fabsf(fabsf(pz) - g.half) < kEps || trapped || rebound >= (uint32_t)kMaxBoundaryCalls) {
             if (ended) return f;

@@ -425,16 +425,13 @@ __device__ __forceinline__ void tally_ended(const TransportArgs &a, const DevGeo
 // their lane for the warp's shared memory (up to 32 of either kind, 64 bytes
 // each) and the lane goes on with another photon; once `fresnel_batch` wait,
 // they are exchanged into the lanes and that part runs for all of them, the
-// photons they displaced waiting as ready ones.  Photons that waited in their
-// lane for 8 others had the Fresnel part run at 9.1 lanes for a third of the
-// warps' time, its hops at 2 to 3, and steps at 25.  20,000 config-1 x-rays
-// (one B200): 59.2 ms before, 51.6 with the wall's photons parked, 46.0 with
-// ended photons tallied together and steps looped, 44.2 with the hops parked,
-// 42.9 with one state word per lane, 41.9 with the shorter pull-back, 40.0 with
-// selects for branches that most lanes take and a refill's photons started
-// together, 38.9 with a step's fate and depth tests only where they matter; 10,001 x-rays in the square / hexagonal lattice 102.5 / 142.9 ->
-// 61.1 / 83.1 ms.  Per photon 1,252 -> 863 warp instructions at 23.5 of 32 lanes
-// (5,000 x-rays), issue slots 87 % busy.  Tallies:
+// photons they displaced waiting as ready ones.  Run in the lane they wait in,
+// beside 8 others, those parts had 9 lanes (the hops 2 to 3) and a third of the
+// warps' time: 20,000 config-1 x-rays 59.1 ms that way, 38.7 this way; 10,001
+// x-rays in the square / hexagonal lattice 102.5 / 142.9 and 60.9 / 83.0.  Per
+// photon 843 warp instructions at 23.8 of 32 lanes, issue slots 88 % busy; in
+// the square / hexagonal lattice 2,731 at 19.6, 91 % / 3,442 at 18.0, 84 %.
+// Tallies:
 // ended photons are tallied 32 at a time (tally_ended) with L2 reductions;
 // with kAgg (tally_mode 1) the fates and the PRF core of geometry 0 are
 // tallied in shared memory first (identical tallies).  kMulti: the
@@ -970,8 +967,10 @@ size_t transport_smem_bytes(const TransportConfig &cfg, int n_geom)
 // The CTAs per SM of a launch.  Label mode has one kernel for one geometry (the
 // surrogate's audit), with the production run's four CTAs per SM whatever
 // ctas_per_sm says, and one for several (training labels) with three (80
-// registers without a spill; 64 geometries x 100 points x 4,000 photons:
-// 22.9 ms, 28.5 ms with two).  A single geometry never goes to a kMulti kernel:
+// registers without a spill; 25,600 points x 4,000 photons in 64 geometries: 66.8
+// ms, 82 with two).  From 182 geometries on the table beside the parked photons
+// leaves room for two CTAs on an SM, and the third of each runs when the queue is
+// empty (182 / 256 geometries: 82.8 / 83.4 ms).  A single geometry never goes to a kMulti kernel:
 // SmemLayout keeps its geometry table for several geometries only.
 int transport_ctas(const TransportConfig &cfg, int n_geom, bool label)
 {
@@ -996,8 +995,8 @@ cudaError_t launch_transport(cudaStream_t s, const TransportConfig &cfg, int sm_
     if (a.g0.grid) {
         // explicit column lattice: single geometry, 256 or 320 threads
         if (multi || a.radial) return cudaErrorInvalidConfiguration;
-        // four CTAs per SM for the square lattice only (10,001 x-rays 61.7 ms,
-        // 65.1 with three): compiled for 64 registers, the test of a hexagonal
+        // four CTAs per SM for the square lattice only (10,001 x-rays 60.9 ms,
+        // 64.5 with three): compiled for 64 registers, the test of a hexagonal
         // lattice's neighbour columns is contracted differently, and 9,092 of
         // 10,001 x-rays would count other photons
         if (cfg.block == 320) transport_kernel<false, 320, 2, false, true><<<grid, cfg.block, smem, s>>>(a);

@@ -117,7 +117,9 @@ typedef struct fd2_options {
     int32_t chunk;                 /* photons per work-queue chunk; 0 = default  */
     int32_t refill;                /* idle lanes before a warp refills; 0 = def. */
     int32_t prf_window;            /* shared-memory PRF window edge; 0 = off, -1 = auto */
-    int32_t use_graph;             /* replay the pipeline as one CUDA graph      */
+    int32_t use_graph;             /* replay the pipeline as CUDA graphs, from a
+                                      submission's second run on (its first is
+                                      launched directly)                         */
     double wait_timeout_s;         /* fd2_wait deadline; <= 0 = none             */
     const char *tune_cache;        /* autotuner cache file (JSON), may be NULL   */
     int64_t event_base;            /* global index of the first submitted event: a
@@ -147,17 +149,17 @@ typedef struct fd2_options {
                                       counterpart in the reference; single
                                       geometry, production transport only)  */
     double grid_gap_um;            /* lattice: gap between neighbouring columns */
-    int32_t tally_mode;            /* 0 (default): each ended photon adds to the
-                                      global tallies with one L2 reduction of its
-                                      lane; 1 (single-geometry runs of the
-                                      reference's column model): fates and
-                                      per-history counts are aggregated across the
-                                      warp (__match_any_sync) and privatised in
-                                      shared memory, the PRF core in a
-                                      shared-memory window (prf_window).  The
-                                      tallies are identical; 0 is faster on a B200
-                                      (the tally rate is far below the L2's atomic
-                                      throughput, so aggregation only costs issue) */
+    int32_t tally_mode;            /* A warp tallies 32 ended photons together,
+                                      fates and per-history counts aggregated
+                                      across the warp (__match_any_sync).
+                                      0 (default): straight to the global tallies
+                                      by L2 reductions; 1 (single-geometry runs of
+                                      the reference's column model): fates
+                                      privatised in shared memory, the PRF core in
+                                      a shared-memory window (prf_window).  The
+                                      tallies are identical, and so is the time on
+                                      a B200 (the tally rate is far below the L2's
+                                      atomic throughput)                         */
 } fd2_options;
 
 typedef struct fd2_counters {
