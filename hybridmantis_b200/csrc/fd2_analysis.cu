@@ -688,7 +688,9 @@ fd2_status fd2_nnps(int32_t device, const double *images, int32_t n_images, int3
     const int64_t all = (int64_t)n * nroi, per_region = (int64_t)R * H;
     const int batch = (int)std::max<int64_t>(1, std::min<int64_t>({all, 65535, (128ll << 20) / (16 * per_region)}));
     const unsigned tiles2 = tiles(H, kColTile) * tiles(R, kFreqs);
-    const int planes = (int)std::max<int64_t>(1, std::min<int64_t>(batch, 1184 / tiles2));
+    int sms = 0;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return to_status(e);
+    const int planes = (int)std::max<int64_t>(1, std::min<int64_t>(batch, 8 * (unsigned)sms / tiles2));
     Layout l;
     Workspace d;
     // only the regions' pixels are copied

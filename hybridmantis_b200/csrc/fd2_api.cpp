@@ -841,7 +841,7 @@ fd2_status fd2_submit_events_device(fd2_ctx *c, const double *x_cm, const double
     if (n > 0) {
         if (!c->d_sums) FD2_CUDA(c, dalloc(&c->d_sums, 3));
         FD2_CUDA(c, cudaMemsetAsync(c->d_sums, 0, 3 * sizeof(double), c->stream));
-        FD2_CUDA(c, fd2::launch_event_sums(c->stream, n, x_cm, y_cm, de_ev, c->d_sums));
+        FD2_CUDA(c, fd2::launch_event_sums(c->stream, c->sm_count, n, x_cm, y_cm, de_ev, c->d_sums));
         FD2_CUDA(c, cudaMemcpyAsync(sums, c->d_sums, sizeof sums, cudaMemcpyDeviceToHost, c->stream));
         FD2_CUDA(c, cudaStreamSynchronize(c->stream));
     }

@@ -19,7 +19,6 @@ constexpr int kComponents = FD2_SG_COMPONENTS;
 constexpr int kInPad = 32;   // input width seen by the first GEMM (K multiple of 32)
 constexpr int kOutPad = 64;  // output width of the last GEMM
 constexpr int kMaxSplits = 16;
-constexpr int kPredictRows = 2 * 148 * 128;  // rows of one prediction pass at 256 hidden units
 constexpr float kMuScale = 50.0f;  // ring radius = kMuScale * softplus(output), um (>= 0)
 constexpr float kSdScale = 10.0f;  // um
 constexpr float kLateralUnitUm = 50.0f;  // unit of feature 2, the deposition's distance from the detector centre

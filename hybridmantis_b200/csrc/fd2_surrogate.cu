@@ -1445,12 +1445,12 @@ fd2_status fd2_sg_predict(fd2_sg *s, const float *features, int64_t n, float *ou
     if (!s || !features || !out || n < 0) return FD2_ERR_INVALID_ARGUMENT;
     if (n == 0) return FD2_OK;
     SG_CUDA(s, cudaSetDevice(s->device));
-    // up to kPredictRows rows a pass (fewer with wider layers): two tiles for
-    // every SM, where the training batch's 8,192 rows are 64 tiles in all.  The
-    // outputs leave the device packed, straight into the caller's array (50,001
-    // rows: seven batches of padded rows, each waited for and unpadded on the
-    // host, 2.5 ms; two passes 0.9)
-    const int64_t most = std::min<int64_t>(kPredictRows, ((int64_t)kPredictRows * 256) / s->hidden);
+    // two tiles of 128 rows for every SM a pass (fewer with wider layers), where
+    // the training batch's 8,192 rows are 64 tiles in all.  The outputs leave the
+    // device packed, straight into the caller's array (50,001 rows: seven batches
+    // of padded rows, each waited for and unpadded on the host, 2.5 ms; two passes
+    // 0.9)
+    const int64_t rows = 2 * 128 * (int64_t)s->sm_count, most = std::min(rows, rows * 256 / s->hidden);
     const int64_t cap = std::min(n, most);
     if (cap > s->predict_cap) {
         // one allocation: outputs, packed outputs and features in FP32, then

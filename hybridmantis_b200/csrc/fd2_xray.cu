@@ -739,11 +739,11 @@ __global__ void __launch_bounds__(256) event_sums_kernel(int64_t n, const double
     }
 }
 
-cudaError_t launch_event_sums(cudaStream_t s, int64_t n, const double *x_cm, const double *y_cm, const double *de,
-                              double *out)
+cudaError_t launch_event_sums(cudaStream_t s, int sm_count, int64_t n, const double *x_cm, const double *y_cm,
+                              const double *de, double *out)
 {
     if (n <= 0) return cudaSuccess;
-    const int blocks = (int)std::min<int64_t>((n + 255) / 256, 592);
+    const int blocks = (int)std::min<int64_t>((n + 255) / 256, 4 * sm_count);
     event_sums_kernel<<<blocks, 256, 0, s>>>(n, x_cm, y_cm, de, out);
     return cudaGetLastError();
 }
